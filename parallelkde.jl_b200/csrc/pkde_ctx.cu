@@ -76,6 +76,8 @@ int pkde_destroy(pkde_ctx *ctx) {
   pkde::stop_server(ctx);  // finishes the queued requests first
   cudaDeviceSynchronize();
   for (auto &b : ctx->buf) b.release();
+  for (auto &t : ctx->twiddles) t.second.release();
+  for (auto &t : ctx->stage_tw) t.second.release();
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
   if (ctx->engine_flags) cudaFreeHost(ctx->engine_flags);
   delete ctx;

@@ -559,7 +559,9 @@ struct Plan {
   double2 *spectra;
   ConvState cs;
   double *tables;    // fz tables then fw tables, S x tot each
-  double *per_step;  // 1-D: f (S x G), mu (S x G), cw, vscale, dlogt (S each)
+  double *per_step;  // 1-D: f (S x G), mu (S x G)
+  double2 *state1d;
+  const double *d_scal;  // 1-D: cw, vscale, dlogt (S each)
   char *bin_scratch;
   int *misc;         // 256-byte block for the binning's flags and max count
   DiracJob job;
@@ -761,16 +763,26 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   const size_t off_tables = arena;
   arena += tables_bytes;
   size_t times_doubles = 0;
-  for (int e = 0; e < count; ++e) times_doubles += (size_t)plans[e].L.S * plans[e].N;
+  size_t n1d = 0;
+  for (int e = 0; e < count; ++e) {
+    times_doubles += (size_t)plans[e].L.S * plans[e].N;
+    if (plans[e].path == StepPath::Steps1D) {
+      ++n1d;
+      times_doubles += 3 * (size_t)plans[e].L.S;
+    }
+  }
   const size_t tjob_bytes = al256(sizeof(TableJob) * count) + al256(sizeof(double) * times_doubles);
   const size_t off_tjobs = arena;
   arena += tjob_bytes;
+  const size_t off_rjobs = arena;
+  arena += al256(steps1d_job_bytes() * n1d);
   for (int e = 0; e < count; ++e) {
     Plan &P = plans[e];
     off[e] = arena;
     arena += al256(sizeof(double2) * (2 * P.npairs + 1) * P.G);
     arena += state_bytes(P.G);
-    if (P.path == StepPath::Steps1D) arena += al256(sizeof(double) * (2 * P.L.S * P.G + 3 * P.L.S));
+    if (P.path == StepPath::Steps1D)
+      arena += al256(sizeof(double) * 2 * P.L.S * P.G) + al256(steps1d_state_bytes((int)P.G, (int)P.npairs, P.L.S));
     arena += dirac_job_scratch(P.g, ests[e].n, P.B);
     if (P.path == StepPath::Generic) {
       generic_wel = std::max(generic_wel, sizeof(double) * 2 * (size_t)P.G);
@@ -801,7 +813,9 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     P.per_step = nullptr;
     if (P.path == StepPath::Steps1D) {
       P.per_step = (double *)q;
-      q += al256(sizeof(double) * (2 * S * P.G + 3 * S));
+      q += al256(sizeof(double) * 2 * S * P.G);
+      P.state1d = (double2 *)q;
+      q += al256(steps1d_state_bytes((int)P.G, (int)P.npairs, S));
     }
     P.bin_scratch = q;
     P.job.g = P.g;
@@ -817,7 +831,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   for (int e = 0; e < count; ++e) dirac_job_phase_a(ctx, plans[e].job, st);
   // ---- propagation factor tables, on the device: the ladders' times and the job
   // descriptors go up in one copy from page-locked memory, one kernel fills every table
-  char *hp = (char *)pinned_staging(ctx, al256(tjob_bytes) + 256 * (size_t)count);
+  char *hp = (char *)pinned_staging(ctx, al256(tjob_bytes) + 256 * (size_t)count + al256(steps1d_job_bytes() * n1d));
   if (tables_bytes) {
     TableJob *hj = (TableJob *)hp;
     double *ht = (double *)(hp + al256(sizeof(TableJob) * count));
@@ -825,7 +839,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     const double two_pi = 6.283185307179586;
     int64_t tpos = 0, maxtotal = 1;
     for (int e = 0; e < count; ++e) {
-      const Plan &P = plans[e];
+      Plan &P = plans[e];
       TableJob &J = hj[e];
       J.fz = P.tables;
       J.S = P.L.S;
@@ -839,6 +853,13 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
       std::memcpy(ht + tpos, P.L.times.data(), sizeof(double) * P.L.S * P.N);
       J.times = dt + tpos;
       tpos += P.L.S * P.N;
+      if (P.path == StepPath::Steps1D) {
+        P.d_scal = dt + tpos;
+        for (const std::vector<double> *v : {&P.L.cw, &P.L.vscale, &P.L.dlogt}) {
+          std::memcpy(ht + tpos, v->data(), sizeof(double) * P.L.S);
+          tpos += P.L.S;
+        }
+      }
       maxtotal = std::max<int64_t>(maxtotal, P.L.S * P.tot);
     }
     PKDE_CUDA_TRY(cudaMemcpyAsync(base + off_tjobs, hp, tjob_bytes, cudaMemcpyHostToDevice, st));
@@ -863,22 +884,30 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
            PKDE_PHASE_FORWARD_FFT);
   // ---- bandwidth steps
   std::vector<EngineArgs> eng;
+  std::vector<Steps1dArgs> line;
   for (int e = 0; e < count; ++e) {
     Plan &P = plans[e];
     const Ladder &L = P.L;
     const int64_t S = L.S;
     const double *dfz = P.tables, *dfw = P.tables + S * P.tot;
     if (P.path == StepPath::Steps1D) {
-      // 1-D: every bandwidth step in parallel (one CTA each), then the convergence
-      // state machine over the stored per-step f_s and means.
-      double *f_all = P.per_step, *mu_all = P.per_step + S * P.G;
-      double *d_cw = mu_all + S * P.G, *d_vs = d_cw + S, *d_dl = d_vs + S;
-      PKDE_CUDA_TRY(cudaMemcpyAsync(d_cw, L.cw.data(), sizeof(double) * S, cudaMemcpyHostToDevice, st));
-      PKDE_CUDA_TRY(cudaMemcpyAsync(d_vs, L.vscale.data(), sizeof(double) * S, cudaMemcpyHostToDevice, st));
-      PKDE_CUDA_TRY(cudaMemcpyAsync(d_dl, L.dlogt.data(), sizeof(double) * S, cudaMemcpyHostToDevice, st));
-      steps1d(ctx, (int)P.g->dims[0], P.spectra, (int)P.npairs, (int)P.B, (int)S, dfz, dfw, P.tot, d_cw,
-              1.0 / (double)P.G, 1.0 / (double)ests[e].n, d_vs, f_all, mu_all, st);
-      converge_steps(ctx, P.G, (int)S, f_all, mu_all, d_dl, L.eps, L.steps_low, L.steps_over, P.cs, st);
+      Steps1dArgs A{};
+      A.n1 = (int)P.G;
+      A.npairs = (int)P.npairs;
+      A.nboot = (int)P.B;
+      A.S = (int)S;
+      A.fused = P.G >= 256 && (P.G & (P.G - 1)) == 0;
+      A.n = ests[e].n;
+      A.spectra = P.spectra;
+      A.fz = dfz;
+      A.fw = dfw;
+      A.tab_stride = P.tot;
+      A.cw = P.d_scal;
+      A.vscale = P.d_scal + S;
+      A.f_out = P.per_step;
+      A.mu_out = P.per_step + S * P.G;
+      A.state = P.state1d;
+      line.push_back(A);
       continue;
     }
     auto init_state = [&] {
@@ -915,6 +944,16 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     autotune_engine(ctx, A, st);  // trial runs (if any) overwrite the state: initialise after
     init_state();
     eng.push_back(A);
+  }
+  // 1-D estimations: every bandwidth step of all of them in one launch, then the
+  // convergence state machine over the stored per-step f_s and means
+  steps1d(ctx, line.data(), (int)line.size(), hp + al256(tjob_bytes) + 256 * (size_t)count, base + off_rjobs, st);
+  for (int e = 0; e < count; ++e) {
+    Plan &P = plans[e];
+    if (P.path != StepPath::Steps1D) continue;
+    const int64_t S = P.L.S;
+    converge_steps(ctx, P.G, (int)S, P.per_step, P.per_step + S * P.G, P.d_scal + 2 * S, P.L.eps, P.L.steps_low,
+                   P.L.steps_over, P.cs, st);
   }
   // two persistent launches: estimations whose axes all take the register power-of-two
   // tiles run in the lean kernel instantiation, the others in the one with the

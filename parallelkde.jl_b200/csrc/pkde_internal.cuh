@@ -104,6 +104,7 @@ struct pkde_ctx {
   int device = 0;
   pkde::DevBuf buf[pkde::BUF_COUNT_];
   std::map<int, pkde::DevBuf> twiddles;  // per line length
+  std::map<std::array<int, 3>, pkde::DevBuf> stage_tw;  // per (length, radix, product of the earlier radices)
   int sm_count = 0;
   size_t smem_optin = 0;
   // tracing (pkde_set_profiling / pkde_get_stats)

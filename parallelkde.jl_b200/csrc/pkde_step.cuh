@@ -21,13 +21,17 @@ struct StabilityResult {
   uint8_t flag;
 };
 
-// find_stability (DirectSpace.jl:975-1031) with first/second_difference (:1092-1100),
-// in FP64.  Explicit-rounding intrinsics keep the operation order of the reference.
-__device__ __forceinline__ StabilityResult find_stability(double f, double f1, double f2, double dlogt, double eps,
-                                                          int64_t steps_low, int64_t steps_over, double minimum,
-                                                          uint16_t c_low, uint16_t c_over, uint8_t flag) {
-  const double d1 = log(fabs(__ddiv_rn(__dsub_rn(f, f1), __dmul_rn(2.0, dlogt))));
-  const double d2 = log(fabs(__ddiv_rn(__dadd_rn(__dsub_rn(f, __dmul_rn(2.0, f1)), f2), __dmul_rn(dlogt, dlogt))));
+// The logarithms of the first and second differences of f (DirectSpace.jl:1092-1100), in
+// FP64.  Explicit-rounding intrinsics keep the operation order of the reference.
+__device__ __forceinline__ void log_differences(double f, double f1, double f2, double dlogt, double &d1, double &d2) {
+  d1 = log(fabs(__ddiv_rn(__dsub_rn(f, f1), __dmul_rn(2.0, dlogt))));
+  d2 = log(fabs(__ddiv_rn(__dadd_rn(__dsub_rn(f, __dmul_rn(2.0, f1)), f2), __dmul_rn(dlogt, dlogt))));
+}
+
+// find_stability (DirectSpace.jl:975-1031) from those logarithms.
+__device__ __forceinline__ StabilityResult decide_stability(double d1, double d2, double eps, int64_t steps_low,
+                                                            int64_t steps_over, double minimum, uint16_t c_low,
+                                                            uint16_t c_over, uint8_t flag) {
   StabilityResult r{false, nan(""), c_low, c_over, flag};
   if (!flag) {
     if (d2 < eps) {
@@ -53,6 +57,14 @@ __device__ __forceinline__ StabilityResult find_stability(double f, double f1, d
   }
   if (isnan(r.new_min)) r.new_min = minimum;
   return r;
+}
+
+__device__ __forceinline__ StabilityResult find_stability(double f, double f1, double f2, double dlogt, double eps,
+                                                          int64_t steps_low, int64_t steps_over, double minimum,
+                                                          uint16_t c_low, uint16_t c_over, uint8_t flag) {
+  double d1, d2;
+  log_differences(f, f1, f2, dlogt, d1, d2);
+  return decide_stability(d1, d2, eps, steps_low, steps_over, minimum, c_low, c_over, flag);
 }
 
 // One step of update_state! (GradeProEstimator.jl:638-669) at grid point i:
@@ -85,44 +97,6 @@ __device__ __forceinline__ void step_update(const StepState &cs, int64_t i, doub
   cs.f2[i] = f1;
   cs.f1[i] = f;
   cs.mu_last[i] = mu;
-}
-
-// The convergence state machine of one grid point over all steps, from the stored
-// per-step log variances f[s*G + i] and means mu[s*G + i]; state kept in registers.
-__device__ __forceinline__ void converge_point_all_steps(const StepState &cs, int64_t i, int64_t G, int S,
-                                                        const double *f_all, const double *mu_all,
-                                                        const double *dlogt, double eps, int64_t steps_low,
-                                                        int64_t steps_over) {
-  double f1 = nan(""), f2 = nan(""), minimum = nan(""), density = nan(""), mu = nan("");
-  uint16_t c_low = 0, c_over = 0;
-  uint8_t flag = 0;
-  int32_t selected = -1;
-  for (int s = 0; s < S; ++s) {
-    const double f = f_all[(int64_t)s * G + i];
-    mu = mu_all[(int64_t)s * G + i];
-    StabilityResult r = find_stability(f, f1, f2, dlogt[s], eps, steps_low, steps_over, minimum, c_low, c_over, flag);
-    c_low = r.c_low;
-    c_over = r.c_over;
-    flag = r.flag;
-    minimum = r.new_min;
-    if (r.more_stable) {
-      density = mu;
-      selected = s;
-    }
-    f2 = f1;
-    f1 = f;
-  }
-  // replace_nans! (GradeProEstimator.jl:1053-1072)
-  if (isnan(density)) density = mu;
-  cs.density[i] = density;
-  cs.selected[i] = selected < 0 ? S : selected;
-  cs.mu_last[i] = mu;
-  cs.f1[i] = f1;
-  cs.f2[i] = f2;
-  cs.minima[i] = minimum;
-  cs.c_low[i] = c_low;
-  cs.c_over[i] = c_over;
-  cs.flags[i] = flag;
 }
 
 // persistent step engine (pkde_engine.cu)
@@ -159,13 +133,29 @@ constexpr int kNarrowSlotMB = 64;
 // Several estimations in one persistent launch (their EngineArgs are independent).
 void run_engine_batch(pkde_ctx *ctx, const EngineArgs *args, int count, cudaStream_t st);
 
-// power-of-two path (pkde_step.cu)
+// Bandwidth steps of 1-D estimations (pkde_steps1d.cu).  f_out and mu_out: S x n1, each
+// step's log scaled variance and means; cw and vscale: device arrays of S values.
+struct Steps1dArgs {
+  int n1, npairs, nboot, S;
+  int fused;  // 1: the step engine's power-of-two arithmetic, 0: every VMR operation rounded by itself
+  int64_t n;
+  const double2 *spectra;
+  const double *fz, *fw;
+  int64_t tab_stride;
+  const double *cw, *vscale;
+  double *f_out, *mu_out;
+  double2 *state;  // steps1d_state_bytes
+};
 bool steps1d_ok(const pkde_grid *g);
-void steps1d(pkde_ctx *ctx, int n1, const double2 *spectra, int npairs, int nboot, int S, const double *fz_all,
-             const double *fw_all, int64_t tab_stride, const double *cw, double invG, double inv_n,
-             const double *vscale, double *f_out, double *mu_out, cudaStream_t st);
+size_t steps1d_job_bytes();
+size_t steps1d_state_bytes(int n1, int npairs, int64_t S);
+// host_jobs (page-locked) and dev_jobs: count x steps1d_job_bytes() each.
+void steps1d(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs, void *dev_jobs, cudaStream_t st);
+// The convergence state machine over all steps (density and selected step of every point).
 void converge_steps(pkde_ctx *ctx, int64_t G, int S, const double *f_all, const double *mu_all, const double *dlogt,
                     double eps, int64_t steps_low, int64_t steps_over, const StepState &cs, cudaStream_t st);
+
+// power-of-two path (pkde_step.cu)
 bool pow2_path_ok(const pkde_grid *g);
 void axis_pass_pow2(pkde_ctx *ctx, const LineSet &ls, const double2 *in, double2 *out, const double *const *factors,
                     const double *scal, int nfac, cudaStream_t st);
