@@ -1024,7 +1024,7 @@ static size_t mix_tile_elems(int R, int lm) {
 }
 
 // Combine twiddles of N = R * M: (cos, sin)(2 pi n1 k2 / N), n1 = 1..R-1, k2 < M.
-static const double2 *combine_twiddles_device(pkde_ctx *ctx, int R, int M) {
+const double2 *combine_twiddles_device(pkde_ctx *ctx, int R, int M) {
   const int N = R * M;
   const int key = -(1000000 + 10 * N + R);
   auto it = ctx->twiddles.find(key);
@@ -1078,6 +1078,13 @@ static AxisShape axis_shape(const pkde_grid *g, int j) {
   return AxisShape{true, 1, tl};
 }
 
+static int mix_radix(int64_t n) { return n % 3 == 0 && ilog2_pow2(n / 3) >= 3 ? 3 : 5; }
+
+EngineAxis engine_axis(const pkde_grid *g, int j) {
+  const AxisShape sh = axis_shape(g, j);
+  return EngineAxis{sh.ok, sh.ok && sh.gen == 0, sh.gen == 2 ? mix_radix(g->dims[j]) : 1};
+}
+
 bool engine_ok(const pkde_grid *g) {
   if (g->ndim < 2) return false;
   for (int j = 0; j < g->ndim; ++j)
@@ -1108,7 +1115,7 @@ EngineEst describe(const EngineArgs &A) {
     E.tl[j] = sh.tl;
     E.mixr[j] = 0;
     if (sh.gen == 2) {
-      E.mixr[j] = g->dims[j] % 3 == 0 && ilog2_pow2(g->dims[j] / 3) >= 3 ? 3 : 5;
+      E.mixr[j] = mix_radix(g->dims[j]);
       E.logn[j] = ilog2_pow2(g->dims[j] / E.mixr[j]);
     } else {
       E.logn[j] = sh.gen ? -1 : ilog2_pow2(g->dims[j]);

@@ -543,7 +543,7 @@ struct Estimation {
   int32_t *d_selected;  // may be null
 };
 
-enum class StepPath { Steps1D, Engine, Generic };
+enum class StepPath { Steps1D, Chunk, Engine, Generic };
 
 // Everything the device work of one estimation needs.
 struct Plan {
@@ -561,7 +561,8 @@ struct Plan {
   double *tables;    // fz tables then fw tables, S x tot each
   double *per_step;  // 1-D: f (S x G), mu (S x G)
   double2 *state1d;
-  const double *d_scal;  // 1-D: cw, vscale, dlogt (S each)
+  bool final_state = false;  // density and selected step need no replace_nans
+  const double *d_scal;  // 1-D, chunks: cw, vscale, dlogt (S each)
   char *bin_scratch;
   int *misc;         // 256-byte block for the binning's flags and max count
   DiracJob job;
@@ -741,7 +742,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   // ---- ladders, factor tables, paths
   size_t arena = al256(256 * (size_t)count);  // misc blocks first (one read-back)
   size_t tables_bytes = 0;
-  size_t generic_wel = 0, generic_scr = 0;
+  size_t generic_wel = 0, generic_scr = 0, chunk_scr = 0;
   std::vector<size_t> off(count);
   for (int e = 0, k = 0; e < count; ++e) {
     Plan &P = plans[e];
@@ -754,7 +755,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     P.L = make_ladder(ests[e].p, bw, ests[e].n);
     axis_offsets(P.g, P.aoff);
     P.tot = P.aoff[P.N];
-    P.path = steps1d_ok(P.g) ? StepPath::Steps1D : (engine_ok(P.g) ? StepPath::Engine : StepPath::Generic);
+    P.path = steps1d_ok(P.g) ? StepPath::Steps1D : chunk_ok(P.g) ? StepPath::Chunk : (engine_ok(P.g) ? StepPath::Engine : StepPath::Generic);
     if (ctx->step_path == PKDE_STEPS_PER_STEP_LAUNCH) P.path = StepPath::Generic;
     tables_bytes += al256(sizeof(double) * 2 * P.L.S * P.tot);
   }
@@ -766,10 +767,8 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   size_t n1d = 0;
   for (int e = 0; e < count; ++e) {
     times_doubles += (size_t)plans[e].L.S * plans[e].N;
-    if (plans[e].path == StepPath::Steps1D) {
-      ++n1d;
-      times_doubles += 3 * (size_t)plans[e].L.S;
-    }
+    if (plans[e].path == StepPath::Steps1D) ++n1d;
+    if (plans[e].path == StepPath::Steps1D || plans[e].path == StepPath::Chunk) times_doubles += 3 * (size_t)plans[e].L.S;
   }
   const size_t tjob_bytes = al256(sizeof(TableJob) * count) + al256(sizeof(double) * times_doubles);
   const size_t off_tjobs = arena;
@@ -784,6 +783,8 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     if (P.path == StepPath::Steps1D)
       arena += al256(sizeof(double) * 2 * P.L.S * P.G) + al256(steps1d_state_bytes((int)P.G, (int)P.npairs, P.L.S));
     arena += dirac_job_scratch(P.g, ests[e].n, P.B);
+    if (P.path == StepPath::Chunk)
+      chunk_scr = std::max(chunk_scr, chunk_scratch_bytes(P.g, (int)P.npairs, (int)P.B, (int)P.L.S));
     if (P.path == StepPath::Generic) {
       generic_wel = std::max(generic_wel, sizeof(double) * 2 * (size_t)P.G);
       const int64_t pair_bytes = (int64_t)sizeof(double2) * 2 * P.G;
@@ -792,8 +793,8 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     }
   }
   char *base = (char *)ensure(ctx, BUF_BATCH, arena);
-  if (generic_scr) {  // sized once, so that no buffer grows while kernels are queued
-    ensure(ctx, BUF_SCRATCH, generic_scr);
+  if (generic_scr || chunk_scr) {  // sized once, so that no buffer grows while kernels are queued
+    ensure(ctx, BUF_SCRATCH, std::max(generic_scr, chunk_scr));
     ensure(ctx, BUF_WELFORD, generic_wel);
   }
   std::vector<size_t> toffs(count);
@@ -853,7 +854,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
       std::memcpy(ht + tpos, P.L.times.data(), sizeof(double) * P.L.S * P.N);
       J.times = dt + tpos;
       tpos += P.L.S * P.N;
-      if (P.path == StepPath::Steps1D) {
+      if (P.path == StepPath::Steps1D || P.path == StepPath::Chunk) {
         P.d_scal = dt + tpos;
         for (const std::vector<double> *v : {&P.L.cw, &P.L.vscale, &P.L.dlogt}) {
           std::memcpy(ht + tpos, v->data(), sizeof(double) * P.L.S);
@@ -917,6 +918,30 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
       }
       PKDE_CHECK_LAUNCH();
     };
+    if (P.path == StepPath::Chunk) {
+      ChunkArgs A{};
+      A.grid = P.g;
+      A.npairs = (int)P.npairs;
+      A.nboot = (int)P.B;
+      A.S = (int)S;
+      A.spectra = P.spectra;
+      A.fz = dfz;
+      A.fw = dfw;
+      A.tab_stride = P.tot;
+      for (int j = 0; j < P.N; ++j) A.aoff[j] = P.aoff[j];
+      A.cw = P.d_scal;
+      A.vscale = P.d_scal + S;
+      A.dlogt = P.d_scal + 2 * S;
+      A.inv_n = 1.0 / (double)ests[e].n;
+      A.eps = L.eps;
+      A.steps_low = L.steps_low;
+      A.steps_over = L.steps_over;
+      A.cs = P.cs;
+      P.final_state = chunk_keeps_all(P.g, A.npairs, A.S);
+      if (!P.final_state) init_state();
+      run_chunk(ctx, A, (char *)ctx->buf[BUF_SCRATCH].ptr, st);
+      continue;
+    }
     if (P.path == StepPath::Generic) {
       init_state();
       run_generic(ctx, P, st);
@@ -995,7 +1020,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   // ---- replace_nans! and outputs
   for (int e = 0; e < count; ++e) {
     Plan &P = plans[e];
-    if (P.path != StepPath::Steps1D) {
+    if (P.path != StepPath::Steps1D && !P.final_state) {
       ::pkde::Trace _tr(ctx, PKDE_PHASE_OTHER, st);
       replace_nans_kernel<<<blocks_for(ctx, P.G), kThreads, 0, st>>>(P.G, P.cs, (int)P.L.S);
     }

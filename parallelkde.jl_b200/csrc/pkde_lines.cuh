@@ -1,0 +1,180 @@
+// Stockham FFT stages over tiles of lines of any length, several lines a tile (element k
+// of line l at unit k P + l: lanes run over lines, then butterflies, so that accesses are
+// contiguous and the lines of a butterfly share one twiddle load).  The arithmetic is that
+// of smem_fft (pkde_internal.cuh), operation for operation.
+#pragma once
+
+#include "pkde_internal.cuh"
+
+namespace pkde {
+
+constexpr int kStages1 = 8;  // enough for every n <= 4096 (3^7 has seven)
+
+// Stockham stage of radix R: nb = n / R butterflies a line, Ns the product of the earlier
+// radices.  tw: twiddles W^(r k) as [k][r - 1] (radix 2, 3, 4, 5, 8), the plain table
+// (cos, sin)(2 pi m / n) for other radices.
+struct Stage1 {
+  int R, nb, Ns, tstep;
+  FastDiv dns;
+  const double2 *tw;
+};
+
+// The transforms' complex product with its fusions written out: the decisions at
+// rounding-decided grid points follow the last bit, so a product must not depend on how
+// the compiler contracts it in one place or another.
+__device__ __forceinline__ double2 cmul1(double2 a, double2 b) {
+  return make_double2(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)), __fma_rn(a.y, b.x, __dmul_rn(a.x, b.y)));
+}
+
+// First level of a radix-8 butterfly on inputs scaled by s: the scaling of one operand of
+// each sum is fused into it, as in the register tiles, where the scaled values feed the
+// sums directly.
+__device__ __forceinline__ void dft4_scaled(double2 *v, const double *s) {
+  auto add = [](double a, double sa, double b, double sb) { return __fma_rn(a, sa, __dmul_rn(b, sb)); };
+  auto sub = [](double a, double sa, double b, double sb) { return __fma_rn(a, sa, -__dmul_rn(b, sb)); };
+  const double2 t0 = make_double2(add(v[0].x, s[0], v[2].x, s[2]), add(v[0].y, s[0], v[2].y, s[2]));
+  const double2 t1 = make_double2(sub(v[0].x, s[0], v[2].x, s[2]), sub(v[0].y, s[0], v[2].y, s[2]));
+  const double2 t2 = make_double2(add(v[1].x, s[1], v[3].x, s[3]), add(v[1].y, s[1], v[3].y, s[3]));
+  const double2 d3 = make_double2(sub(v[1].x, s[1], v[3].x, s[3]), sub(v[1].y, s[1], v[3].y, s[3]));
+  const double2 t3 = cmul_si(d3, 1);
+  v[0] = cadd(t0, t2);
+  v[2] = csub(t0, t2);
+  v[1] = cadd(t1, t3);
+  v[3] = csub(t1, t3);
+}
+// Second level of the radix-8 butterfly from its even and odd halves.
+__device__ __forceinline__ void dft8_join(double2 *v, const double2 *e, const double2 *o) {
+  const double h = 0.70710678118654752440;  // sqrt(1/2)
+  auto join = [h](double2 e, double ax, double ay, double2 &p, double2 &m) {
+    p = make_double2(__fma_rn(h, ax, e.x), __fma_rn(h, ay, e.y));
+    m = make_double2(__fma_rn(-h, ax, e.x), __fma_rn(-h, ay, e.y));
+  };
+  v[0] = cadd(e[0], o[0]);
+  v[4] = csub(e[0], o[0]);
+  join(e[1], o[1].x - o[1].y, o[1].y + o[1].x, v[1], v[5]);
+  const double2 o2 = cmul_si(o[2], 1);
+  v[2] = cadd(e[2], o2);
+  v[6] = csub(e[2], o2);
+  join(e[3], -o[3].x - o[3].y, o[3].x - o[3].y, v[3], v[7]);
+}
+__device__ __forceinline__ void dft8_scaled(double2 *v, const double *s) {
+  double2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+  const double se[4] = {s[0], s[2], s[4], s[6]}, so[4] = {s[1], s[3], s[5], s[7]};
+  dft4_scaled(e, se);
+  dft4_scaled(o, so);
+  dft8_join(v, e, o);
+}
+__device__ __forceinline__ void dft3_fused(double2 *v) {
+  const double s3 = 0.86602540378443864676;  // sin(2 pi / 3)
+  const double2 t = cadd(v[1], v[2]), d = csub(v[1], v[2]);
+  const double2 m = make_double2(__fma_rn(-0.5, t.x, v[0].x), __fma_rn(-0.5, t.y, v[0].y));
+  v[0] = cadd(v[0], t);
+  v[1] = make_double2(__fma_rn(-s3, d.y, m.x), __fma_rn(s3, d.x, m.y));
+  v[2] = make_double2(__fma_rn(s3, d.y, m.x), __fma_rn(-s3, d.x, m.y));
+}
+__device__ __forceinline__ void dft5_fused(double2 *v) {
+  const double c1 = 0.30901699437494742410, c2 = -0.80901699437494742410;  // cos(2 pi / 5), cos(4 pi / 5)
+  const double s1 = 0.95105651629515357212, s2 = 0.58778525229247312917;   // sin(2 pi / 5), sin(4 pi / 5)
+  const double2 a1 = cadd(v[1], v[4]), b1 = csub(v[1], v[4]);
+  const double2 a2 = cadd(v[2], v[3]), b2 = csub(v[2], v[3]);
+  const double2 x0 = v[0];
+  auto even = [](double x, double p, double a, double q, double b) { return __fma_rn(q, b, __fma_rn(p, a, x)); };
+  auto odd = [](double p, double a, double q, double b) { return __fma_rn(p, a, __dmul_rn(q, b)); };
+  const double2 p1 = make_double2(even(x0.x, c1, a1.x, c2, a2.x), even(x0.y, c1, a1.y, c2, a2.y));
+  const double2 p2 = make_double2(even(x0.x, c2, a1.x, c1, a2.x), even(x0.y, c2, a1.y, c1, a2.y));
+  const double2 q1 = cmul_si(make_double2(odd(s1, b1.x, s2, b2.x), odd(s1, b1.y, s2, b2.y)), 1);
+  const double2 q2 = cmul_si(make_double2(odd(s2, b1.x, -s1, b2.x), odd(s2, b1.y, -s1, b2.y)), 1);
+  v[0] = cadd(x0, cadd(a1, a2));
+  v[1] = cadd(p1, q1);
+  v[4] = csub(p1, q1);
+  v[2] = cadd(p2, q2);
+  v[3] = csub(p2, q2);
+}
+template <int R>
+__device__ __forceinline__ void dft_r(double2 *v) {
+  if constexpr (R == 2) dft2<1>(v);
+  if constexpr (R == 3) dft3_fused(v);
+  if constexpr (R == 4) dft4<1>(v);
+  if constexpr (R == 5) dft5_fused(v);
+  if constexpr (R == 8) {
+    double2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+    dft4<1>(e);
+    dft4<1>(o);
+    dft8_join(v, e, o);
+  }
+}
+
+// One stage of radix R over L lines in T threads.  ld(j, l, v): the R inputs of butterfly j
+// of line l (elements j + r nb); returns true when it has applied the butterfly itself (a
+// first stage that scales its inputs).  st(l, pos, v): element pos + q Ns of line l is v[q].
+template <int T, int R, class Ld, class St>
+__device__ __forceinline__ void line_stage(const Stage1 &s, int L, FastDiv dL, bool first, Ld ld, St st) {
+  const int items = s.nb * L, Ns = s.Ns;
+  const double2 *tw = s.tw;
+  const FastDiv dns = s.dns;
+  for (int e = threadIdx.x; e < items; e += T) {
+    const int j = (int)fdiv((uint32_t)e, dL), l = e - j * L;
+    double2 v[R];
+    if (!ld(j, l, v)) {
+      int jq = j;
+      if (!first) {
+        jq = (int)fdiv((uint32_t)j, dns);
+        const int k = j - jq * Ns;
+        if (k > 0) {
+          const double2 *w = tw + k * (R - 1) - 1;
+#pragma unroll
+          for (int r = 1; r < R; ++r) v[r] = cmul1(v[r], __ldg(w + r));
+        }
+      }
+      dft_r<R>(v);
+      st(l, j + jq * Ns * (R - 1), v);
+    } else {
+      st(l, j * R, v);
+    }
+  }
+}
+
+// Any other radix: an item is QB outputs of one butterfly, every input is read once an
+// item.  src: the tile (pitch P); st(l, pos, v): output pos of line l.
+template <int T, class St>
+__device__ __forceinline__ void line_stage_generic(const Stage1 &s, int n, int L, FastDiv dL, const double2 *src, int P,
+                                                   St st) {
+  constexpr int QB = 4;
+  const int R = s.R, nb = s.nb, Ns = s.Ns;
+  const int nblk = (R + QB - 1) / QB, per = nb * L;
+  for (int i = threadIdx.x; i < nblk * per; i += T) {
+    const int qb = i / per, e = i - qb * per;
+    const int j = (int)fdiv((uint32_t)e, dL), l = e - j * L;
+    const int jq = (int)fdiv((uint32_t)j, s.dns), k = j - jq * Ns;
+    const int q0 = qb * QB, nq = min(QB, R - q0);
+    double2 v[QB];
+    int m[QB], inc[QB];
+#pragma unroll
+    for (int q = 0; q < QB; ++q) {
+      m[q] = 0;
+      inc[q] = q < nq ? k * s.tstep + (q0 + q) * nb : 0;
+      v[q] = make_double2(0.0, 0.0);
+    }
+    const double2 *p = src + j * P + l;
+    for (int r = 0; r < R; ++r, p += nb * P) {
+      const double2 x = *p;
+#pragma unroll
+      for (int q = 0; q < QB; ++q) {
+        v[q] = cadd(v[q], cmul1(x, __ldg(s.tw + m[q])));
+        m[q] += inc[q];
+        if (m[q] >= n) m[q] -= n;
+      }
+    }
+    const int o = j + jq * Ns * (R - 1) + q0 * Ns;
+#pragma unroll
+    for (int q = 0; q < QB; ++q)
+      if (q < nq) st(l, o + q * Ns, v[q]);
+  }
+}
+
+// Host: the stages of an n-point line (radix sequence of make_plan, tables on the device);
+// returns their number.
+bool stages_ok(int n);
+int make_stages(pkde_ctx *ctx, int n, Stage1 *st);
+
+}  // namespace pkde

@@ -73,7 +73,7 @@ size_t footprint(const pkde_gradepro_params *p, int64_t n, bool has_idx) {
   b += 4 * n + 8 * N * n + 32 * nc * n + 4 * (B + 1) * G;                                 // binning
   b += sizeof(double2) * (2 * P + 1) * G;  // low parts of the fixed-point sums
   b += 4 * B * n + 8 * n + 8 * (size_t)G;  // draws per sample, cell order, cell starts
-  if (N == 1) b += sizeof(double) * 2 * S * G;                                            // 1-D steps
+  if (N == 1) b += sizeof(double) * 4 * S * G;                                            // 1-D steps
   const size_t slot = std::max<size_t>(32u << 20, sizeof(double2) * 2 * (size_t)G);
   b += 8 * slot + 32 * (size_t)G + sizeof(int) * (size_t)S * (P + 1) * (N + G / 16 + 1);  // engine
   return b + (4u << 20);

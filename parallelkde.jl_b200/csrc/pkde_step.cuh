@@ -133,6 +133,36 @@ constexpr int kNarrowSlotMB = 64;
 // Several estimations in one persistent launch (their EngineArgs are independent).
 void run_engine_batch(pkde_ctx *ctx, const EngineArgs *args, int count, cudaStream_t st);
 
+// How the step engine transforms an axis (its arithmetic): register power-of-two tiles, N = R M
+// mixed-radix tiles (R = 3 or 5), or plain Stockham stages (R = 1, pow2 false).
+struct EngineAxis {
+  bool ok, pow2;
+  int R;
+};
+EngineAxis engine_axis(const pkde_grid *g, int j);
+// Combine twiddles of N = R M: (cos, sin)(2 pi n1 k2 / N) as [n1 - 1][k2].
+const double2 *combine_twiddles_device(pkde_ctx *ctx, int R, int M);
+
+// Bandwidth steps of N-D estimations in chunks of steps (pkde_chunk.cu).
+struct ChunkArgs {
+  const pkde_grid *grid;
+  int npairs, nboot, S;
+  const double2 *spectra;
+  const double *fz, *fw;
+  int64_t tab_stride;
+  int64_t aoff[4];
+  const double *cw, *vscale, *dlogt;  // device arrays of S values
+  double inv_n, eps;
+  int64_t steps_low, steps_over;
+  StepState cs;
+};
+bool chunk_ok(const pkde_grid *g);
+size_t chunk_scratch_bytes(const pkde_grid *g, int npairs, int nboot, int S);
+// Whether density and selected step come out final (else the caller initialises the state
+// before and fills the points without a selected step after).
+bool chunk_keeps_all(const pkde_grid *g, int npairs, int S);
+void run_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch, cudaStream_t st);
+
 // Bandwidth steps of 1-D estimations (pkde_steps1d.cu).  f_out and mu_out: S x n1, each
 // step's log scaled variance and means; cw and vscale: device arrays of S values.
 struct Steps1dArgs {

@@ -10,22 +10,12 @@
 // step's log scaled variance f_s and means mu_s, and converge_steps_kernel walks them.
 #include <algorithm>
 
+#include "pkde_lines.cuh"
 #include "pkde_regfft.cuh"
 #include "pkde_step.cuh"
 
 namespace pkde {
 namespace {
-
-constexpr int kStages1 = 8;  // enough for every n <= 4096 (3^7 has seven)
-
-// Stockham stage of radix R: nb = n / R butterflies a line, Ns the product of the earlier
-// radices.  tw: twiddles W^(r k) as [k][r - 1] (radix 2, 3, 4, 5, 8), the plain table
-// (cos, sin)(2 pi m / n) for other radices.
-struct Stage1 {
-  int R, nb, Ns, tstep;
-  FastDiv dns;
-  const double2 *tw;
-};
 
 // One estimation (device-resident descriptor).  A tile holds the L = 2 a arrays (z, w) of
 // a bootstrap pairs; index 0 / 1 / 2: full tile, last tile, means (L = 1).
@@ -42,65 +32,6 @@ struct Job1 {
   double2 *state;  // S x n running (mean, m2), lines too long for shared memory
   Stage1 st[kStages1];
 };
-
-// The transforms' complex product with its fusions written out: the decisions at
-// rounding-decided grid points follow the last bit, so a product must not depend on how
-// the compiler contracts it in one place or another.
-__device__ __forceinline__ double2 cmul1(double2 a, double2 b) {
-  return make_double2(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)), __fma_rn(a.y, b.x, __dmul_rn(a.x, b.y)));
-}
-
-// First level of a radix-8 butterfly on inputs scaled by s: the scaling of one operand of
-// each sum is fused into it, as in the register tiles, where the scaled values feed the
-// sums directly.
-__device__ __forceinline__ void dft4_scaled(double2 *v, const double *s) {
-  auto add = [](double a, double sa, double b, double sb) { return __fma_rn(a, sa, __dmul_rn(b, sb)); };
-  auto sub = [](double a, double sa, double b, double sb) { return __fma_rn(a, sa, -__dmul_rn(b, sb)); };
-  const double2 t0 = make_double2(add(v[0].x, s[0], v[2].x, s[2]), add(v[0].y, s[0], v[2].y, s[2]));
-  const double2 t1 = make_double2(sub(v[0].x, s[0], v[2].x, s[2]), sub(v[0].y, s[0], v[2].y, s[2]));
-  const double2 t2 = make_double2(add(v[1].x, s[1], v[3].x, s[3]), add(v[1].y, s[1], v[3].y, s[3]));
-  const double2 d3 = make_double2(sub(v[1].x, s[1], v[3].x, s[3]), sub(v[1].y, s[1], v[3].y, s[3]));
-  const double2 t3 = cmul_si(d3, 1);
-  v[0] = cadd(t0, t2);
-  v[2] = csub(t0, t2);
-  v[1] = cadd(t1, t3);
-  v[3] = csub(t1, t3);
-}
-// Second level of the radix-8 butterfly from its even and odd halves.
-__device__ __forceinline__ void dft8_join(double2 *v, const double2 *e, const double2 *o) {
-  const double h = 0.70710678118654752440;  // sqrt(1/2)
-  auto join = [h](double2 e, double ax, double ay, double2 &p, double2 &m) {
-    p = make_double2(__fma_rn(h, ax, e.x), __fma_rn(h, ay, e.y));
-    m = make_double2(__fma_rn(-h, ax, e.x), __fma_rn(-h, ay, e.y));
-  };
-  v[0] = cadd(e[0], o[0]);
-  v[4] = csub(e[0], o[0]);
-  join(e[1], o[1].x - o[1].y, o[1].y + o[1].x, v[1], v[5]);
-  const double2 o2 = cmul_si(o[2], 1);
-  v[2] = cadd(e[2], o2);
-  v[6] = csub(e[2], o2);
-  join(e[3], -o[3].x - o[3].y, o[3].x - o[3].y, v[3], v[7]);
-}
-__device__ __forceinline__ void dft8_scaled(double2 *v, const double *s) {
-  double2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-  const double se[4] = {s[0], s[2], s[4], s[6]}, so[4] = {s[1], s[3], s[5], s[7]};
-  dft4_scaled(e, se);
-  dft4_scaled(o, so);
-  dft8_join(v, e, o);
-}
-template <int R>
-__device__ __forceinline__ void dft_r(double2 *v) {
-  if constexpr (R == 2) dft2<1>(v);
-  if constexpr (R == 3) dft3<1>(v);
-  if constexpr (R == 4) dft4<1>(v);
-  if constexpr (R == 5) dft5<1>(v);
-  if constexpr (R == 8) {
-    double2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-    dft4<1>(e);
-    dft4<1>(o);
-    dft8_join(v, e, o);
-  }
-}
 
 extern __shared__ double2 sm1[];
 
@@ -465,22 +396,6 @@ Shape1 shape1(int n, int npairs) {
   return r;
 }
 
-// Twiddles of a radix-2/3/4/5/8 stage, [k][r - 1].
-const double2 *stage1_twiddles(pkde_ctx *ctx, int n, int R, int Ns) {
-  const std::array<int, 3> k3{n, R, Ns};
-  auto it = ctx->stage_tw.find(k3);
-  if (it != ctx->stage_tw.end()) return it->second.as<double2>();
-  const std::vector<double2> w = make_twiddles(n);
-  std::vector<double2> tw;
-  const int tstep = n / (Ns * R);
-  for (int k = 0; k < Ns; ++k)
-    for (int r = 1; r < R; ++r) tw.push_back(w[(size_t)r * k * tstep]);
-  DevBuf &b = ctx->stage_tw[k3];
-  b.ensure(sizeof(double2) * tw.size());
-  PKDE_CUDA_TRY(cudaMemcpy(b.ptr, tw.data(), sizeof(double2) * tw.size(), cudaMemcpyHostToDevice));
-  return b.as<double2>();
-}
-
 // d1 and d2 of find_stability are functions of three consecutive f alone, so the logarithms
 // of a block's points are computed for kConvSteps steps by all threads, then one thread per
 // point walks the steps: the walk alone is a serial chain of S steps, the logarithms were
@@ -537,8 +452,38 @@ __global__ void __launch_bounds__(kConvThreads) converge_steps_kernel(
 
 }  // namespace
 
+// Twiddles of a radix-2/3/4/5/8 stage, [k][r - 1].
+static const double2 *stage1_twiddles(pkde_ctx *ctx, int n, int R, int Ns) {
+  const std::array<int, 3> k3{n, R, Ns};
+  auto it = ctx->stage_tw.find(k3);
+  if (it != ctx->stage_tw.end()) return it->second.as<double2>();
+  const std::vector<double2> w = make_twiddles(n);
+  std::vector<double2> tw;
+  const int tstep = n / (Ns * R);
+  for (int k = 0; k < Ns; ++k)
+    for (int r = 1; r < R; ++r) tw.push_back(w[(size_t)r * k * tstep]);
+  DevBuf &b = ctx->stage_tw[k3];
+  b.ensure(sizeof(double2) * tw.size());
+  PKDE_CUDA_TRY(cudaMemcpy(b.ptr, tw.data(), sizeof(double2) * tw.size(), cudaMemcpyHostToDevice));
+  return b.as<double2>();
+}
+
+bool stages_ok(int n) { return make_plan(n).nstages <= kStages1; }
+
+int make_stages(pkde_ctx *ctx, int n, Stage1 *st) {
+  const FftPlan p = make_plan(n);
+  int ns = 1;
+  for (int q = 0; q < p.nstages; ++q) {
+    const int R = p.radix[q];
+    st[q] = Stage1{R, n / R, ns, n / (ns * R), p.div_ns[q],
+                   R <= 5 || R == 8 ? stage1_twiddles(ctx, n, R, ns) : twiddles_device(ctx, n)};
+    ns *= R;
+  }
+  return p.nstages;
+}
+
 bool steps1d_ok(const pkde_grid *g) {
-  return g->ndim == 1 && g->dims[0] <= 4096 && make_plan((int)g->dims[0]).nstages <= kStages1;
+  return g->ndim == 1 && g->dims[0] <= 4096 && stages_ok((int)g->dims[0]);
 }
 
 const double2 *stage_twiddles_device(pkde_ctx *ctx, int logn);
@@ -590,15 +535,7 @@ void steps1d(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs,
       J.inv_ns = 1.0 / (double)A.n;
       J.f_out = A.f_out;
       J.mu_out = A.mu_out;
-      const FftPlan p = make_plan(A.n1);
-      J.nst = p.nstages;
-      int ns = 1;
-      for (int q = 0; q < p.nstages; ++q) {
-        const int R = p.radix[q];
-        J.st[q] = Stage1{R, A.n1 / R, ns, A.n1 / (ns * R), p.div_ns[q],
-                         R <= 5 || R == 8 ? stage1_twiddles(ctx, A.n1, R, ns) : twiddles_device(ctx, A.n1)};
-        ns *= R;
-      }
+      J.nst = make_stages(ctx, A.n1, J.st);
       hj[k++] = J;
     }
     first[c + 1] = k;
