@@ -16,6 +16,7 @@
 // points, as many lines as fit, lines of different arrays and steps side by side).
 // The persistent engine (pkde_engine.cu) keeps the shapes whose tiles it fills itself.
 #include <algorithm>
+#include <cstring>
 
 #include "pkde_lines.cuh"
 #include "pkde_step.cuh"
@@ -23,8 +24,9 @@
 namespace pkde {
 namespace {
 
-constexpr int kCT = 256;       // threads
-constexpr int kTilePts = 2048; // points per tile
+constexpr int kCT = 256;           // threads
+constexpr int kTilePts = 8 * kCT;  // points per tile
+constexpr int kCtas = 768 / kCT;   // CTAs per SM (80 registers a thread)
 
 // One grid axis.  Lines of n = R M points: R = 1, plain Stockham stages; R = 3 or 5 (M a power
 // of two from 8), the R interleaved sub-lines x[R n2 + n1] through the stages of M, then
@@ -61,11 +63,59 @@ __host__ __device__ __forceinline__ int axis_tiles_held(const ChunkAxis &ax) {
 
 extern __shared__ double2 smc[];
 
+// A launch covers one or several estimations: blocks [block0, next job's block0) are the job's.
+struct AxisJob {
+  ChunkAxis ax;
+  ChunkTile t;
+  ChunkRun run;
+  const double2 *in;
+  double2 *out;
+};
+struct RowsJob {
+  ChunkAxis ax;
+  ChunkTile t;
+  int G, A, arr0, rt, pairs, np, b0, nboot, tiles, parts;  // blocks: tiles x parts x steps
+  double inv_n;
+  const double2 *in;
+  double *out;
+};
+struct VarJob {
+  int64_t G;
+  int nboot, blocks;  // blocks: per step
+  const double *x, *vscale;
+  double *f;
+};
+
+// The job of this block: of several (job array and first blocks in device memory) copied into
+// shared memory, of one the kernel's own parameter.
+template <class J>
+__device__ __forceinline__ void find_job(const J *jobs, const unsigned *block0, int count, J &sj, unsigned &first) {
+  __shared__ int s_job;
+  if (threadIdx.x < 32) {
+    int job = 0;
+    for (;;) {  // block0 increases: the lanes at or below this block form a prefix
+      const int k = job + 1 + (int)threadIdx.x;
+      const bool le = k < count && __ldg(block0 + k) <= blockIdx.x;
+      const int c = __popc(__ballot_sync(0xffffffffu, le));
+      job += c;
+      if (c < 32) break;
+    }
+    if (threadIdx.x == 0) s_job = job;
+  }
+  __syncthreads();
+  const int job = s_job;
+  const int *src = reinterpret_cast<const int *>(jobs + job);
+  int *dst = reinterpret_cast<int *>(&sj);
+  for (int i = threadIdx.x; i < (int)(sizeof(J) / sizeof(int)); i += blockDim.x) dst[i] = __ldg(src + i);
+  first = __ldg(block0 + job);
+  __syncthreads();
+}
+
 // Lines through every stage: input element k of line l at src(l) + k ss (loaded by ld, scaled by
 // scale(l) and f[k] where `scaled`), tiles a and b in turn, output position p of line l through
 // st(l, p, value).  Every thread calls; the caller synchronises before the tiles are reused.
 template <class Src, class Ld, class Fac, class St>
-__device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const ChunkTile &t, double2 *a, double2 *b,
+__device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const ChunkTile &t, int a, int b,
                                                 int64_t ss, Src src, Ld ld, bool scaled, Fac fac, St st) {
   const int R = ax.R, L = t.L, Lr = t.Lr, P = t.P;
   const int total = ax.nst + (R > 1 ? 1 : 0);
@@ -74,7 +124,7 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
     return l - n1 * L;
   };
   int s0 = 0;
-  double2 *in = b, *out = a;
+  int in = b, out = a;  // tiles, as units of smc (pointers would lose the address space)
   const int64_t rs = ss * R;
   if (ax.generic_first) {  // its inputs pass through the tile (R = 1)
     for (int e = threadIdx.x; e < ax.n * L; e += kCT) {
@@ -86,7 +136,7 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
         const double sc = __ldg(f + k) * c;
         v = make_double2(__dmul_rn(v.x, sc), __dmul_rn(v.y, sc));
       }
-      out[k * P + l] = v;
+      smc[out + k * P + l] = v;
     }
     __syncthreads();
     in = a;
@@ -126,7 +176,7 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
         });
       } else {
         line_stage<kCT, Q>(s, Lr, t.dLr, true, load, [&](int l, int pos, double2(&v)[Q]) {
-          double2 *o = out + pos * P + l;
+          double2 *o = smc + out + pos * P + l;
 #pragma unroll
           for (int q = 0; q < Q; ++q) o[q * P] = v[q];
         });
@@ -150,7 +200,7 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
     auto stage = [&](auto rc) {
       constexpr int Q = decltype(rc)::value;
       auto load = [&](int j, int l, double2(&v)[Q]) {
-        const double2 *p = in + j * P + l;
+        const double2 *p = smc + in + j * P + l;
         const int step = s.nb * P;
 #pragma unroll
         for (int r = 0; r < Q; ++r) v[r] = p[r * step];
@@ -163,7 +213,7 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
         });
       } else {
         line_stage<kCT, Q>(s, Lr, t.dLr, false, load, [&](int l, int pos, double2(&v)[Q]) {
-          double2 *o = out + pos * P + l;
+          double2 *o = smc + out + pos * P + l;
           const int step = s.Ns * P;
 #pragma unroll
           for (int q = 0; q < Q; ++q) o[q * step] = v[q];
@@ -177,12 +227,12 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
       case 3: stage(std::integral_constant<int, 3>{}); break;
       case 5: stage(std::integral_constant<int, 5>{}); break;
       default:
-        if (last) line_stage_generic<kCT>(s, ax.n, Lr, t.dLr, in, P, st);
-        else line_stage_generic<kCT>(s, ax.n, Lr, t.dLr, in, P, [&](int l, int pos, double2 v) { out[pos * P + l] = v; });
+        if (last) line_stage_generic<kCT>(s, ax.n, Lr, t.dLr, smc + in, P, st);
+        else line_stage_generic<kCT>(s, ax.n, Lr, t.dLr, smc + in, P, [&](int l, int pos, double2 v) { smc[out + pos * P + l] = v; });
         break;
     }
     if (!last) __syncthreads();
-    double2 *x = in;
+    const int x = in;
     in = out;
     out = x;
   }
@@ -195,7 +245,7 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
         double2 y[Q];
 #pragma unroll
         for (int n1 = 0; n1 < Q; ++n1) {
-          y[n1] = in[k2 * P + n1 * L + l];
+          y[n1] = smc[in + k2 * P + n1 * L + l];
           if (n1 > 0) {  // the engine's combine fuses the other product of the imaginary part
             const double2 v = y[n1], w = __ldg(ax.twc + (n1 - 1) * M + k2);
             y[n1] = make_double2(__fma_rn(v.x, w.x, -__dmul_rn(v.y, w.y)), __fma_rn(v.x, w.y, __dmul_rn(v.y, w.x)));
@@ -215,10 +265,12 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
 // of the flattened (step, array, line) index.  SPECTRA: the first pass, from the spectra,
 // with the factors of every axis and the array's scalar; else in place.
 template <bool SPECTRA>
-__global__ void __launch_bounds__(kCT, 3)
-    chunk_axis_kernel(const __grid_constant__ ChunkAxis ax, const __grid_constant__ ChunkTile t,
-                      const __grid_constant__ ChunkRun run, const double2 *in, double2 *out) {
-  double2 *a = smc, *b = a + t.size;
+__device__ __forceinline__ void axis_body(const AxisJob &job, unsigned block) {
+  const ChunkAxis &ax = job.ax;
+  const ChunkTile &t = job.t;
+  const ChunkRun &run = job.run;
+  const double2 *in = job.in;
+  double2 *out = job.out;
   int64_t *so = reinterpret_cast<int64_t *>(smc + axis_tiles_held(ax) * t.size);
   int64_t *si = so + t.L;
   const double **sf = reinterpret_cast<const double **>(si + t.L);
@@ -227,7 +279,7 @@ __global__ void __launch_bounds__(kCT, 3)
   {
     const unsigned per = (unsigned)run.A * ax.lines, total = (unsigned)run.C * per;
     for (int l = threadIdx.x; l < t.L; l += kCT) {
-      unsigned w = blockIdx.x * (unsigned)t.L + l;
+      unsigned w = block * (unsigned)t.L + l;
       const bool valid = w < total;
       if (!valid) w = 0;
       const unsigned c = w / per, r = w - c * per, arr = r / ax.lines;
@@ -253,7 +305,7 @@ __global__ void __launch_bounds__(kCT, 3)
   }
   __syncthreads();
   chunk_transform(
-      ax, t, a, b, ax.inner, [&](int l) { return in + si[l]; },
+      ax, t, 0, t.size, ax.inner, [&](int l) { return in + si[l]; },
       [](const double2 *p) { return SPECTRA ? __ldg(p) : __ldcg(p); }, SPECTRA,
       [&](int l, double &c) {
         c = sc[l];
@@ -263,6 +315,19 @@ __global__ void __launch_bounds__(kCT, 3)
         const int64_t o = so[l];
         if (o >= 0) __stcg(out + o + (int64_t)pos * ax.inner, v);
       });
+}
+
+template <bool SPECTRA>
+__global__ void __launch_bounds__(kCT, kCtas) chunk_axis_kernel(const __grid_constant__ AxisJob job) {
+  axis_body<SPECTRA>(job, blockIdx.x);
+}
+template <bool SPECTRA>
+__global__ void __launch_bounds__(kCT, kCtas)
+    chunk_axis_many_kernel(const AxisJob *jobs, const unsigned *block0, int count) {
+  __shared__ AxisJob job;
+  unsigned first;
+  find_job(jobs, block0, count, job, first);
+  axis_body<SPECTRA>(job, blockIdx.x - first);
 }
 
 __device__ __forceinline__ double chunk_vmr(double Mv, double Vv, double inv_n) {
@@ -281,14 +346,18 @@ __device__ __forceinline__ void cp_async16(double2 *dst, const double2 *src) {
 // of the next pair come in by cp.async while the VMR of this one is computed.  Else
 // the rows of the means' array, mu[step G + point] = their magnitudes.
 template <bool VMR>
-__global__ void __launch_bounds__(kCT, 3)
-    chunk_rows_kernel(const __grid_constant__ ChunkAxis ax, const __grid_constant__ ChunkTile t, int G, int A, int arr0,
-                      int rt, int pairs, int np, int b0, int nboot, double inv_n, const double2 *in, double *out) {
-  const int n = ax.n, PN = t.PN, row0 = blockIdx.x * rt, nrow = min(rt, ax.lines - row0);
-  const int p0 = VMR ? blockIdx.y * np : 0, p1 = VMR ? min(p0 + np, pairs) : 1;
-  const double2 *base = in + ((int64_t)blockIdx.z * A + arr0) * G + (int64_t)row0 * n;
-  double2 *buf[2] = {smc, smc + t.size};
-  auto load = [&](int p, double2 *dst) {
+__device__ __forceinline__ void rows_body(const RowsJob &job, unsigned block) {
+  const ChunkAxis &ax = job.ax;
+  const ChunkTile &t = job.t;
+  const int G = job.G, rt = job.rt, nboot = job.nboot;
+  const double inv_n = job.inv_n;
+  const unsigned q = block / (unsigned)job.tiles, bx = block - q * job.tiles;
+  const unsigned bz = q / (unsigned)job.parts, by = q - bz * job.parts;
+  const int n = ax.n, PN = t.PN, row0 = bx * rt, nrow = min(rt, ax.lines - row0);
+  const int p0 = VMR ? by * job.np : 0, p1 = VMR ? min(p0 + job.np, job.pairs) : 1;
+  const double2 *base = job.in + ((int64_t)bz * job.A + job.arr0) * G + (int64_t)row0 * n;
+  auto load = [&](int p, int tile) {
+    double2 *dst = smc + tile;
     const double2 *z = base + (VMR ? (int64_t)(2 * p) * G : 0);
     const int count = nrow * n;
     int l = threadIdx.x / n, k = threadIdx.x - l * n;
@@ -302,34 +371,34 @@ __global__ void __launch_bounds__(kCT, 3)
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  int cur = 0;
-  load(p0, buf[0]);
+  int cur = 0;  // the tile (of two) that holds the inputs
+  load(p0, 0);
   for (int p = p0; p < p1; ++p) {
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     // stage i reads one buffer and writes the other; the results lie in the buffer the last one wrote
     const int total = ax.nst + (ax.R > 1 ? 1 : 0);
     const int res = ((total + ax.generic_first) & 1) ? 1 - cur : cur;
-    double2 *dst = buf[res], *src = buf[cur];
+    const int dst = res * t.size, src = cur * t.size;
     chunk_transform(
-        ax, t, buf[1 - cur], buf[cur], PN, [&](int l) { return (const double2 *)src + l; },
+        ax, t, t.size - src, src, PN, [&](int l) { return (const double2 *)smc + src + l; },
         [](const double2 *q) { return *q; }, false,
         [&](int, double &c) {
           c = 1.0;
           return (const double *)nullptr;
         },
-        [&](int l, int pos, double2 v) { dst[pos * PN + l] = v; });
+        [&](int l, int pos, double2 v) { smc[dst + pos * PN + l] = v; });
     __syncthreads();
     cur = 1 - res;
-    if (p + 1 < p1) load(p + 1, buf[cur]);
+    if (p + 1 < p1) load(p + 1, cur * t.size);
     const int count = nrow * n;
     int l = threadIdx.x / n, k = threadIdx.x - l * n;
     const int dl = kCT / n, dk = kCT - dl * n;
     if constexpr (VMR) {
-      const int b = b0 + 2 * p;
-      double *xa = out + ((int64_t)blockIdx.z * nboot + b) * G + (int64_t)row0 * n;
+      const int b = job.b0 + 2 * p;
+      double *xa = job.out + ((int64_t)bz * nboot + b) * G + (int64_t)row0 * n;
       for (int e = threadIdx.x; e < count; e += kCT) {
-        const double2 z = dst[k * PN + l], w = dst[k * PN + rt + l];
+        const double2 z = smc[dst + k * PN + l], w = smc[dst + k * PN + rt + l];
         __stcg(xa + e, chunk_vmr(z.x, w.x, inv_n));
         if (b + 1 < nboot) __stcg(xa + G + e, chunk_vmr(z.y, w.y, inv_n));
         l += dl;
@@ -338,8 +407,8 @@ __global__ void __launch_bounds__(kCT, 3)
       }
     } else {
       for (int e = threadIdx.x; e < count; e += kCT) {
-        const double2 z = dst[k * PN + l];
-        out[(int64_t)blockIdx.z * G + (int64_t)row0 * n + e] = sqrt(__fma_rn(z.x, z.x, __dmul_rn(z.y, z.y)));
+        const double2 z = smc[dst + k * PN + l];
+        job.out[(int64_t)bz * G + (int64_t)row0 * n + e] = sqrt(__fma_rn(z.x, z.x, __dmul_rn(z.y, z.y)));
         l += dl;
         k += dk;
         if (k >= n) k -= n, ++l;
@@ -348,20 +417,39 @@ __global__ void __launch_bounds__(kCT, 3)
   }
 }
 
-// Welford over the bootstraps in order, then f = log(scaled variance), of every point of C steps.
-__global__ void __launch_bounds__(kCT) chunk_var_kernel(int64_t G, int nboot, const double *__restrict__ x,
-                                                        const double *__restrict__ vscale, double *__restrict__ f) {
+template <bool VMR>
+__global__ void __launch_bounds__(kCT, kCtas) chunk_rows_kernel(const __grid_constant__ RowsJob job) {
+  rows_body<VMR>(job, blockIdx.x);
+}
+template <bool VMR>
+__global__ void __launch_bounds__(kCT, kCtas)
+    chunk_rows_many_kernel(const RowsJob *jobs, const unsigned *block0, int count) {
+  __shared__ RowsJob job;
+  unsigned first;
+  find_job(jobs, block0, count, job, first);
+  rows_body<VMR>(job, blockIdx.x - first);
+}
+
+// Welford over the bootstraps in order, then f = log(scaled variance), of every point of the
+// job's steps.
+constexpr int kVT = 128;
+__global__ void __launch_bounds__(kVT) chunk_var_kernel(const VarJob *jobs, const unsigned *block0, int count) {
+  __shared__ VarJob J;
   __shared__ double recip[1024];  // 1 / i, IEEE
-  const int64_t i = blockIdx.x * (int64_t)kCT + threadIdx.x;
-  const double *p = x + (int64_t)blockIdx.y * nboot * G + i;
+  unsigned first;
+  find_job(jobs, block0, count, J, first);
+  const int64_t G = J.G;
+  const unsigned step = (blockIdx.x - first) / (unsigned)J.blocks;
+  const int64_t i = (blockIdx.x - first - step * J.blocks) * (int64_t)kVT + threadIdx.x;
+  const double *p = J.x + (int64_t)step * J.nboot * G + i;
   double mean = 0.0, m2 = 0.0;
-  for (int b0 = 0; b0 < nboot; b0 += 1024) {
-    const int nb = min(1024, nboot - b0);
+  for (int b0 = 0; b0 < J.nboot; b0 += 1024) {
+    const int nb = min(1024, J.nboot - b0);
     __syncthreads();
-    for (int b = threadIdx.x; b < nb; b += kCT) recip[b] = 1.0 / (double)(b0 + b + 1);
+    for (int b = threadIdx.x; b < nb; b += kVT) recip[b] = 1.0 / (double)(b0 + b + 1);
     __syncthreads();
     if (i < G) {
-#pragma unroll 8
+#pragma unroll 16
       for (int b = 0; b < nb; ++b) {
         const double v = __ldcg(p + (int64_t)(b0 + b) * G);
         const double delta = __dsub_rn(v, mean);
@@ -371,8 +459,8 @@ __global__ void __launch_bounds__(kCT) chunk_var_kernel(int64_t G, int nboot, co
     }
   }
   if (i < G) {
-    const double v = __ddiv_rn(__dmul_rn(vscale[blockIdx.y], m2), (double)(nboot - 1));
-    f[(int64_t)blockIdx.y * G + i] = isfinite(v) ? log(v) : nan("");
+    const double v = __ddiv_rn(__dmul_rn(J.vscale[step], m2), (double)(J.nboot - 1));
+    J.f[(int64_t)step * G + i] = isfinite(v) ? log(v) : nan("");
   }
 }
 
@@ -430,9 +518,9 @@ struct ChunkShape {
   bool all_steps; // f and the means of every step are kept, the convergence walk runs once
 };
 
-// Chunks hold about 48 MB of intermediates (half of the L2 beside the spectra and the x
+// Chunks hold up to 64 MB of intermediates (half of the L2 beside the spectra and the x
 // values being written); f and means of all steps are kept up to 512 MB.
-constexpr int64_t kChunkBytes = int64_t(48) << 20, kKeepBytes = int64_t(512) << 20;
+constexpr int64_t kChunkBytes = int64_t(64) << 20, kKeepBytes = int64_t(512) << 20;
 ChunkShape chunk_shape(int64_t G, int npairs, int S) {
   ChunkShape c;
   const int64_t step = (int64_t)sizeof(double2) * (2 * npairs + 1) * G;
@@ -451,6 +539,12 @@ ChunkShape chunk_shape(int64_t G, int npairs, int S) {
 
 }  // namespace
 
+// Grids with an axis that is neither a power of two nor 3 or 5 times one: the engine's
+// shared-memory tiles hold few lines there (100 x 100, 100 bootstraps, 250 steps: 66 ms
+// against 8.1 ms here; 50 x 41 x 36, 32 bootstraps, 100 steps: 148 against 16.6 ms).  Small grids of
+// any lengths: a step has too few tiles for the engine's order of items (64 x 64, 33 bootstraps,
+// 40 steps: 2.0 against 0.4 ms; 64^3: 7 against 11 ms).
+constexpr int64_t kSmallGrid = 65536;
 bool chunk_ok(const pkde_grid *g) {
   if (g->ndim < 2) return false;
   const int64_t G = grid_size(g);
@@ -464,13 +558,13 @@ bool chunk_ok(const pkde_grid *g) {
       if (!stages_ok((int)g->dims[j])) return false;
     }
   }
-  return any || getenv("PKDE_PROBE_CHUNK");
+  return any || G < kSmallGrid;
 }
 
-// Scratch: [intermediates][x][f][means].
+// Scratch of one estimation: [intermediates][x][f][means].
 static void chunk_scratch(int64_t G, int npairs, int nboot, int S, const ChunkShape &c, size_t off[5]) {
   auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-  const int64_t arrays = std::max<int64_t>(c.g == npairs ? 2 * npairs + 1 : 2 * c.g, 1);
+  const int64_t arrays = c.g == npairs ? 2 * npairs + 1 : 2 * c.g;
   const int64_t keep = c.all_steps ? S : c.C;
   off[0] = 0;
   off[1] = off[0] + al(sizeof(double2) * (size_t)(c.C * arrays * G));
@@ -488,21 +582,52 @@ size_t chunk_scratch_bytes(const pkde_grid *g, int npairs, int nboot, int S) {
 
 bool chunk_keeps_all(const pkde_grid *g, int npairs, int S) { return chunk_shape(grid_size(g), npairs, S).all_steps; }
 
-void run_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch, cudaStream_t st) {
-  const pkde_grid *g = A.grid;
-  const int N = g->ndim, S = A.S, nboot = A.nboot, npairs = A.npairs;
-  const int G = (int)grid_size(g);
-  const ChunkShape c = chunk_shape(G, npairs, S);
-  size_t off[5];
-  chunk_scratch(G, npairs, nboot, S, c, off);
-  double2 *mid = (double2 *)(scratch + off[0]);
-  double *x = (double *)(scratch + off[1]), *f = (double *)(scratch + off[2]), *mu = (double *)(scratch + off[3]);
+namespace {
+
+// One launch of a pass over the jobs of several estimations.
+template <class J>
+struct Launch {
+  std::vector<J> jobs;
+  std::vector<unsigned> block0;
+  unsigned blocks = 0;
+  size_t smem = 0;
+  void add(const J &j, unsigned n, size_t bytes) {
+    jobs.push_back(j);
+    block0.push_back(blocks);
+    blocks += n;
+    smem = std::max(smem, bytes);
+  }
+};
+// The launches of chunk k: axis passes (first the one that reads the spectra), rows, variances.
+struct ChunkLaunches {
+  Launch<AxisJob> axis[3];
+  Launch<RowsJob> vmr, means;
+  Launch<VarJob> var;
+};
+
+struct ChunkPlan {
   ChunkAxis ax[4];
+  ChunkRun run;
+  ChunkShape c;
+  double2 *mid;
+  double *x, *f, *mu;
+};
+
+ChunkPlan plan_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch) {
+  ChunkPlan P{};
+  const pkde_grid *g = A.grid;
+  const int N = g->ndim, G = (int)grid_size(g);
+  P.c = chunk_shape(G, A.npairs, A.S);
+  size_t off[5];
+  chunk_scratch(G, A.npairs, A.nboot, A.S, P.c, off);
+  P.mid = (double2 *)(scratch + off[0]);
+  P.x = (double *)(scratch + off[1]);
+  P.f = (double *)(scratch + off[2]);
+  P.mu = (double *)(scratch + off[3]);
   int inner = 1;
   for (int j = 0; j < N; ++j) {
     const EngineAxis k = engine_axis(g, j);
-    ChunkAxis &a = ax[j];
-    a = ChunkAxis{};
+    ChunkAxis &a = P.ax[j];
     a.n = (int)g->dims[j];
     a.R = k.R;
     a.M = a.n / a.R;
@@ -514,10 +639,10 @@ void run_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch, cudaStream_t st
     a.generic_first = a.st[0].R > 5 && a.st[0].R != 8;
     inner *= a.n;
   }
-  ChunkRun run{};
+  ChunkRun &run = P.run;
   run.N = N;
   run.G = G;
-  run.mean = 2 * npairs;
+  run.mean = 2 * A.npairs;
   run.tab_stride = A.tab_stride;
   run.fz = A.fz;
   run.fw = A.fw;
@@ -527,81 +652,198 @@ void run_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch, cudaStream_t st
     run.dims[j] = (int)g->dims[j];
     run.aoff[j] = A.aoff[j];
   }
-  // the passes over axes N..2 of `arrays` arrays from a0 in C steps from s0
-  auto axes = [&](int64_t s0, int C, int a0, int arrays) {
-    run.s0 = s0;
-    run.C = C;
-    run.a0 = a0;
-    run.A = arrays;
-    for (int j = N - 1; j >= 1; --j) {
-      const ChunkAxis &a = ax[j];
-      const int64_t lines = (int64_t)C * arrays * a.lines;
-      const int most = kTilePts / a.n;
-      ChunkTile t = make_tile(a.n, a.R, std::min<int64_t>(lines, most), most, false);
-      const size_t smem = sizeof(double2) * (size_t)axis_tiles_held(a) * t.size + 32 * (size_t)t.L;
-      const unsigned blocks = (unsigned)((lines + t.L - 1) / t.L);
-      Trace tr(ctx, PKDE_PHASE_STEP_FFT, st);
-      if (j == N - 1) {
-        allow_dynamic_smem(ctx, chunk_axis_kernel<true>, smem);
-        chunk_axis_kernel<true><<<blocks, kCT, smem, st>>>(a, t, run, A.spectra, mid);
+  return P;
+}
+
+// Passes over axes N..2 of `arrays` arrays from a0 in C steps from s0.
+void add_axes(ChunkLaunches &L, const ChunkArgs &A, const ChunkPlan &P, int64_t s0, int C, int a0, int arrays) {
+  const int N = P.run.N;
+  for (int j = N - 1; j >= 1; --j) {
+    AxisJob J{};
+    J.ax = P.ax[j];
+    J.run = P.run;
+    J.run.s0 = s0;
+    J.run.C = C;
+    J.run.a0 = a0;
+    J.run.A = arrays;
+    const int64_t lines = (int64_t)C * arrays * J.ax.lines;
+    const int most = kTilePts / J.ax.n;
+    J.t = make_tile(J.ax.n, J.ax.R, std::min<int64_t>(lines, most), most, false);
+    J.in = j == N - 1 ? A.spectra : P.mid;
+    J.out = P.mid;
+    const size_t smem = sizeof(double2) * (size_t)axis_tiles_held(J.ax) * J.t.size + 32 * (size_t)J.t.L;
+    L.axis[N - 1 - j].add(J, (unsigned)((lines + J.t.L - 1) / J.t.L), smem);
+  }
+}
+
+void add_rows(pkde_ctx *ctx, Launch<RowsJob> &L, const ChunkArgs &A, const ChunkPlan &P, int C, int arrays, int arr0,
+              bool vmr, int pairs, int b0, double *out) {
+  RowsJob J{};
+  J.ax = P.ax[0];
+  const int per = vmr ? 2 : 1, most = std::max(1, kTilePts / (per * J.ax.n));
+  J.rt = make_tile(J.ax.n, 1, J.ax.lines, most, false).L;
+  J.t = make_tile(J.ax.n, J.ax.R, per * J.rt, per * J.rt, true);
+  J.G = P.run.G;
+  J.A = arrays;
+  J.arr0 = arr0;
+  J.pairs = pairs;
+  J.b0 = b0;
+  J.nboot = A.nboot;
+  J.inv_n = A.inv_n;
+  J.in = P.mid;
+  J.out = out;
+  J.tiles = (J.ax.lines + J.rt - 1) / J.rt;
+  // pairs per CTA: enough CTAs for a few waves, at most 8 pairs (the rows of the next pair are
+  // fetched while this one's ratios are computed)
+  J.np = 1;
+  J.parts = 1;
+  if (vmr) {
+    J.np = (int)std::max<int64_t>(
+        1, std::min<int64_t>(8, (int64_t)J.tiles * C * pairs / (6 * kCtas * (int64_t)ctx->sm_count)));
+    J.parts = (pairs + J.np - 1) / J.np;
+    J.np = (pairs + J.parts - 1) / J.parts;
+  }
+  L.add(J, (unsigned)J.tiles * J.parts * C, sizeof(double2) * 2 * (size_t)J.t.size);
+}
+
+size_t al256c(size_t x) { return (x + 255) & ~size_t(255); }
+
+}  // namespace
+
+// The bandwidth steps of `count` estimations, scratch[e] for each: chunk k of every
+// estimation shares its launches.
+void run_chunk(pkde_ctx *ctx, const ChunkArgs *args, int count, char *const *scratch, cudaStream_t st) {
+  std::vector<ChunkPlan> plan;
+  int chunks = 0;
+  for (int e = 0; e < count; ++e) {
+    plan.push_back(plan_chunk(ctx, args[e], scratch[e]));
+    chunks = std::max(chunks, (args[e].S + plan[e].c.C - 1) / plan[e].c.C);
+  }
+  // every launch of the call; estimations whose steps are split by pair groups add launches of their own
+  std::vector<ChunkLaunches> all;
+  std::vector<std::vector<std::array<int, 2>>> converge;  // per launch group: (estimation, first step)
+  for (int k = 0; k < chunks; ++k) {
+    const size_t g0 = all.size();
+    all.emplace_back();
+    converge.emplace_back();
+    for (int e = 0; e < count; ++e) {
+      const ChunkArgs &A = args[e];
+      const ChunkPlan &P = plan[e];
+      const int64_t G = P.run.G, s0 = (int64_t)k * P.c.C;
+      if (s0 >= A.S) continue;
+      const int C = (int)std::min<int64_t>(P.c.C, A.S - s0);
+      double *fs = P.f + (P.c.all_steps ? s0 * G : 0), *ms = P.mu + (P.c.all_steps ? s0 * G : 0);
+      size_t at = g0;
+      auto group = [&](size_t i) -> ChunkLaunches & {
+        while (all.size() <= i) {
+          all.emplace_back();
+          converge.emplace_back();
+        }
+        return all[i];
+      };
+      if (P.c.g == A.npairs) {
+        ChunkLaunches &L = group(at);
+        add_axes(L, A, P, s0, C, 0, 2 * A.npairs + 1);
+        add_rows(ctx, L.vmr, A, P, C, 2 * A.npairs + 1, 0, true, A.npairs, 0, P.x);
+        add_rows(ctx, L.means, A, P, C, 2 * A.npairs + 1, 2 * A.npairs, false, 0, 0, ms);
       } else {
-        allow_dynamic_smem(ctx, chunk_axis_kernel<false>, smem);
-        chunk_axis_kernel<false><<<blocks, kCT, smem, st>>>(a, t, run, mid, mid);
+        for (int p0 = 0; p0 < A.npairs; p0 += P.c.g, ++at) {
+          const int np = std::min(P.c.g, A.npairs - p0);
+          ChunkLaunches &L = group(at);
+          add_axes(L, A, P, s0, C, 2 * p0, 2 * np);
+          add_rows(ctx, L.vmr, A, P, C, 2 * np, 0, true, np, 2 * p0, P.x);
+        }
+        ChunkLaunches &L = group(at);
+        add_axes(L, A, P, s0, C, 2 * A.npairs, 1);
+        add_rows(ctx, L.means, A, P, C, 1, 0, false, 0, 0, ms);
       }
-      PKDE_CHECK_LAUNCH();
+      VarJob V{};
+      V.G = G;
+      V.nboot = A.nboot;
+      V.blocks = (int)((G + kVT - 1) / kVT);
+      V.x = P.x;
+      V.vscale = A.vscale + s0;
+      V.f = fs;
+      group(at).var.add(V, (unsigned)(V.blocks * C), 0);
+      if (!P.c.all_steps) converge[at].push_back({e, (int)s0});
     }
+  }
+  // job arrays to the device in one copy
+  size_t bytes = 0;
+  auto place = [&](auto &L, bool always) {
+    const size_t at = bytes;
+    if (L.jobs.size() < 2 && !always) return at;  // one job: a kernel parameter
+    bytes += al256c(L.jobs.size() * sizeof(L.jobs[0])) + al256c(L.jobs.size() * sizeof(unsigned));
+    return at;
   };
-  const ChunkAxis &a1 = ax[0];
-  auto rows = [&](auto kern, int C, int arrays, int arr0, bool vmr, int pairs, int b0, double *out) {
-    const int per = vmr ? 2 : 1;
-    const int most = std::max(1, kTilePts / (per * a1.n));
-    const ChunkTile rt = make_tile(a1.n, 1, a1.lines, most, false);
-    ChunkTile t = make_tile(a1.n, a1.R, per * rt.L, per * rt.L, true);
-    const size_t smem = sizeof(double2) * 2 * (size_t)t.size;
-    const unsigned tiles = (unsigned)((a1.lines + rt.L - 1) / rt.L);
-    // pairs per CTA: enough CTAs for a few waves, at most 8 pairs (the rows of the next pair are
-    // fetched while this one's ratios are computed)
-    int np = 1;
-    if (vmr) {
-      np = (int)std::max<int64_t>(1, std::min<int64_t>(8, (int64_t)tiles * C * pairs / (6 * 3 * ctx->sm_count)));
-      const int parts = (pairs + np - 1) / np;
-      np = (pairs + parts - 1) / parts;
-    }
-    allow_dynamic_smem(ctx, kern, smem);
-    Trace tr(ctx, vmr ? PKDE_PHASE_STEP_VMR : PKDE_PHASE_STEP_MEANS, st);
-    kern<<<dim3(tiles, vmr ? (unsigned)((pairs + np - 1) / np) : 1u, (unsigned)C), kCT, smem, st>>>(
-        a1, t, G, arrays, arr0, rt.L, pairs, np, b0, nboot, A.inv_n, mid, out);
-    PKDE_CHECK_LAUNCH();
+  std::vector<std::array<size_t, 6>> at(all.size());
+  for (size_t i = 0; i < all.size(); ++i) {
+    for (int j = 0; j < 3; ++j) at[i][j] = place(all[i].axis[j], false);
+    at[i][3] = place(all[i].vmr, false);
+    at[i][4] = place(all[i].means, false);
+    at[i][5] = place(all[i].var, true);
+  }
+  char *dev = (char *)ensure(ctx, BUF_CHUNK, bytes);
+  std::vector<char> host(bytes);
+  auto store = [&](auto &L, size_t o, bool always) {
+    if (L.jobs.empty() || (L.jobs.size() < 2 && !always)) return;
+    std::memcpy(host.data() + o, L.jobs.data(), L.jobs.size() * sizeof(L.jobs[0]));
+    std::memcpy(host.data() + o + al256c(L.jobs.size() * sizeof(L.jobs[0])), L.block0.data(),
+                L.block0.size() * sizeof(unsigned));
   };
-  for (int64_t s0 = 0; s0 < S; s0 += c.C) {
-    const int C = (int)std::min<int64_t>(c.C, S - s0);
-    double *fs = f + (c.all_steps ? s0 * G : 0), *ms = mu + (c.all_steps ? s0 * G : 0);
-    if (c.g == npairs) {
-      axes(s0, C, 0, 2 * npairs + 1);
-      rows(chunk_rows_kernel<true>, C, 2 * npairs + 1, 0, true, npairs, 0, x);
-      rows(chunk_rows_kernel<false>, C, 2 * npairs + 1, 2 * npairs, false, 0, 0, ms);
-    } else {
-      for (int p0 = 0; p0 < npairs; p0 += c.g) {
-        const int np = std::min(c.g, npairs - p0);
-        axes(s0, C, 2 * p0, 2 * np);
-        rows(chunk_rows_kernel<true>, C, 2 * np, 0, true, np, 2 * p0, x);
-      }
-      axes(s0, C, 2 * npairs, 1);
-      rows(chunk_rows_kernel<false>, C, 1, 0, false, 0, 0, ms);
-    }
+  for (size_t i = 0; i < all.size(); ++i) {
+    for (int j = 0; j < 3; ++j) store(all[i].axis[j], at[i][j], false);
+    store(all[i].vmr, at[i][3], false);
+    store(all[i].means, at[i][4], false);
+    store(all[i].var, at[i][5], true);
+  }
+  PKDE_CUDA_TRY(cudaMemcpyAsync(dev, host.data(), bytes, cudaMemcpyHostToDevice, st));
+  auto launch = [&](auto &L, size_t o, int phase, auto one, auto many) {
+    if (L.jobs.empty()) return;
+    using J = std::decay_t<decltype(L.jobs[0])>;
+    const J *jobs = reinterpret_cast<const J *>(dev + o);
+    const unsigned *block0 = reinterpret_cast<const unsigned *>(dev + o + al256c(L.jobs.size() * sizeof(J)));
     {
-      Trace tr(ctx, PKDE_PHASE_STEP_VMR, st);
-      chunk_var_kernel<<<dim3((unsigned)((G + kCT - 1) / kCT), (unsigned)C), kCT, 0, st>>>(G, nboot, x, A.vscale + s0, fs);
+      Trace tr(ctx, phase, st);
+      if (L.jobs.size() == 1) {
+        allow_dynamic_smem(ctx, one, L.smem);
+        one<<<L.blocks, kCT, L.smem, st>>>(L.jobs[0]);
+      } else {
+        allow_dynamic_smem(ctx, many, L.smem);
+        many<<<L.blocks, kCT, L.smem, st>>>(jobs, block0, (int)L.jobs.size());
+      }
     }
     PKDE_CHECK_LAUNCH();
-    if (!c.all_steps) {
+  };
+  for (size_t i = 0; i < all.size(); ++i) {
+    ChunkLaunches &L = all[i];
+    launch(L.axis[0], at[i][0], PKDE_PHASE_STEP_FFT, chunk_axis_kernel<true>, chunk_axis_many_kernel<true>);
+    for (int j = 1; j < 3; ++j)
+      launch(L.axis[j], at[i][j], PKDE_PHASE_STEP_FFT, chunk_axis_kernel<false>, chunk_axis_many_kernel<false>);
+    launch(L.vmr, at[i][3], PKDE_PHASE_STEP_VMR, chunk_rows_kernel<true>, chunk_rows_many_kernel<true>);
+    launch(L.means, at[i][4], PKDE_PHASE_STEP_MEANS, chunk_rows_kernel<false>, chunk_rows_many_kernel<false>);
+    if (!L.var.jobs.empty()) {
+      const char *o = dev + at[i][5];
       Trace tr(ctx, PKDE_PHASE_STEP_MEANS, st);
-      chunk_converge_kernel<<<(unsigned)((G + kCT - 1) / kCT), kCT, 0, st>>>(
-          G, C, (int)s0, fs, ms, A.dlogt, A.eps, A.steps_low, A.steps_over, A.cs);
+      chunk_var_kernel<<<L.var.blocks, kVT, 0, st>>>(
+          reinterpret_cast<const VarJob *>(o),
+          reinterpret_cast<const unsigned *>(o + al256c(L.var.jobs.size() * sizeof(VarJob))), (int)L.var.jobs.size());
+    }
+    PKDE_CHECK_LAUNCH();
+    for (const auto &c : converge[i]) {
+      const ChunkArgs &A = args[c[0]];
+      const ChunkPlan &P = plan[c[0]];
+      Trace tr(ctx, PKDE_PHASE_STEP_MEANS, st);
+      chunk_converge_kernel<<<(unsigned)((P.run.G + kCT - 1) / kCT), kCT, 0, st>>>(
+          P.run.G, std::min(P.c.C, A.S - c[1]), c[1], P.f, P.mu, A.dlogt, A.eps, A.steps_low, A.steps_over, A.cs);
     }
     PKDE_CHECK_LAUNCH();
   }
-  if (c.all_steps) converge_steps(ctx, G, S, f, mu, A.dlogt, A.eps, A.steps_low, A.steps_over, A.cs, st);
+  for (int e = 0; e < count; ++e) {
+    const ChunkArgs &A = args[e];
+    if (plan[e].c.all_steps)
+      converge_steps(ctx, plan[e].run.G, A.S, plan[e].f, plan[e].mu, A.dlogt, A.eps, A.steps_low, A.steps_over, A.cs, st);
+  }
 }
 
 }  // namespace pkde

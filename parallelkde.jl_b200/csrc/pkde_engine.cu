@@ -1371,10 +1371,10 @@ size_t engine_ring_bytes(const EngineArgs &A) {
 // ---------------------------------------------------------------- autotuning
 // Key of a shape: grid dimensions and pairs of bootstraps (the schedule depends on
 // nothing else).
-static std::string tune_key(const EngineArgs &A) {
-  std::string k = std::to_string(A.grid->ndim);
-  for (int j = 0; j < A.grid->ndim; ++j) k += "x" + std::to_string(A.grid->dims[j]);
-  return k + ":p" + std::to_string(A.npairs);
+static std::string tune_key(const pkde_grid *g, int npairs) {
+  std::string k = std::to_string(g->ndim);
+  for (int j = 0; j < g->ndim; ++j) k += "x" + std::to_string(g->dims[j]);
+  return k + ":p" + std::to_string(npairs);
 }
 
 static void load_tune_file(pkde_ctx *ctx) {
@@ -1399,9 +1399,23 @@ static void save_tune(pkde_ctx *ctx, const std::string &key, const std::array<in
   fclose(f);
 }
 
+// A shape's schedule may also be "in chunks of steps" (0 0 0), which the rule of chunk_ok
+// chooses without trials.  An engine schedule in the file for such a shape is kept.
+bool chunk_schedule(pkde_ctx *ctx, const pkde_grid *g, int npairs) {
+  load_tune_file(ctx);
+  const std::string key = tune_key(g, npairs);
+  auto it = ctx->tune.find(key);
+  if (it != ctx->tune.end()) return it->second[0] == 0 || !engine_ok(g);
+  if (ctx->autotune) {
+    ctx->tune[key] = {0, 0, 0};
+    save_tune(ctx, key, {0, 0, 0});
+  }
+  return true;
+}
+
 void autotune_engine(pkde_ctx *ctx, EngineArgs &A, cudaStream_t st) {
   load_tune_file(ctx);
-  const std::string key = tune_key(A);
+  const std::string key = tune_key(A.grid, A.npairs);
   auto it = ctx->tune.find(key);
   if (it == ctx->tune.end()) {
     if (!ctx->autotune) return;

@@ -520,6 +520,17 @@ static void check_binning_flags(pkde_ctx *ctx) {
   }
 }
 
+// Scratch that the estimations of a batch call may hold together in buffer `id`: half of the
+// free memory, capped by PKDE_RING_BUDGET_MB (tests use it to force one launch per estimation).
+static size_t shared_budget(pkde_ctx *ctx, BufId id) {
+  size_t freeb = 0, totalb = 0;
+  PKDE_CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
+  size_t budget = (freeb + ctx->buf[id].bytes) / 2;
+  if (const char *cap = getenv("PKDE_RING_BUDGET_MB"); cap && *cap)
+    budget = std::min(budget, (size_t)std::max(0LL, atoll(cap)) << 20);
+  return budget;
+}
+
 // Page-locked staging buffer of the context (grow-only), for asynchronous uploads.
 static void *pinned_staging(pkde_ctx *ctx, size_t bytes) {
   if (bytes > ctx->pinned_bytes) {
@@ -743,6 +754,8 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   size_t arena = al256(256 * (size_t)count);  // misc blocks first (one read-back)
   size_t tables_bytes = 0;
   size_t generic_wel = 0, generic_scr = 0, chunk_scr = 0;
+  std::vector<int> chunk_e;           // estimations that run in chunks of steps, their scratch
+  std::vector<size_t> chunk_bytes;
   std::vector<size_t> off(count);
   for (int e = 0, k = 0; e < count; ++e) {
     Plan &P = plans[e];
@@ -755,7 +768,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     P.L = make_ladder(ests[e].p, bw, ests[e].n);
     axis_offsets(P.g, P.aoff);
     P.tot = P.aoff[P.N];
-    P.path = steps1d_ok(P.g) ? StepPath::Steps1D : chunk_ok(P.g) ? StepPath::Chunk : (engine_ok(P.g) ? StepPath::Engine : StepPath::Generic);
+    P.path = steps1d_ok(P.g) ? StepPath::Steps1D : (chunk_ok(P.g) && chunk_schedule(ctx, P.g, (int)P.npairs)) ? StepPath::Chunk : (engine_ok(P.g) ? StepPath::Engine : StepPath::Generic);
     if (ctx->step_path == PKDE_STEPS_PER_STEP_LAUNCH) P.path = StepPath::Generic;
     tables_bytes += al256(sizeof(double) * 2 * P.L.S * P.tot);
   }
@@ -783,8 +796,10 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     if (P.path == StepPath::Steps1D)
       arena += al256(sizeof(double) * 2 * P.L.S * P.G) + al256(steps1d_state_bytes((int)P.G, (int)P.npairs, P.L.S));
     arena += dirac_job_scratch(P.g, ests[e].n, P.B);
-    if (P.path == StepPath::Chunk)
-      chunk_scr = std::max(chunk_scr, chunk_scratch_bytes(P.g, (int)P.npairs, (int)P.B, (int)P.L.S));
+    if (P.path == StepPath::Chunk) {
+      chunk_e.push_back(e);
+      chunk_bytes.push_back(chunk_scratch_bytes(P.g, (int)P.npairs, (int)P.B, (int)P.L.S));
+    }
     if (P.path == StepPath::Generic) {
       generic_wel = std::max(generic_wel, sizeof(double) * 2 * (size_t)P.G);
       const int64_t pair_bytes = (int64_t)sizeof(double2) * 2 * P.G;
@@ -793,6 +808,22 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     }
   }
   char *base = (char *)ensure(ctx, BUF_BATCH, arena);
+  // estimations in chunks of steps share launches as far as their scratch together fits the
+  // memory budget: chunk_group[i] = first of the i-th set
+  std::vector<size_t> chunk_group{0};
+  {
+    const size_t budget = chunk_e.size() > 1 ? shared_budget(ctx, BUF_SCRATCH) : 0;
+    size_t need = 0;
+    for (size_t i = 0; i < chunk_e.size(); ++i) {
+      if (i > chunk_group.back() && need + chunk_bytes[i] > budget) {
+        chunk_group.push_back(i);
+        need = 0;
+      }
+      need += chunk_bytes[i];
+      chunk_scr = std::max(chunk_scr, need);
+    }
+    chunk_group.push_back(chunk_e.size());
+  }
   if (generic_scr || chunk_scr) {  // sized once, so that no buffer grows while kernels are queued
     ensure(ctx, BUF_SCRATCH, std::max(generic_scr, chunk_scr));
     ensure(ctx, BUF_WELFORD, generic_wel);
@@ -886,6 +917,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   // ---- bandwidth steps
   std::vector<EngineArgs> eng;
   std::vector<Steps1dArgs> line;
+  std::vector<ChunkArgs> chunk;
   for (int e = 0; e < count; ++e) {
     Plan &P = plans[e];
     const Ladder &L = P.L;
@@ -939,7 +971,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
       A.cs = P.cs;
       P.final_state = chunk_keeps_all(P.g, A.npairs, A.S);
       if (!P.final_state) init_state();
-      run_chunk(ctx, A, (char *)ctx->buf[BUF_SCRATCH].ptr, st);
+      chunk.push_back(A);
       continue;
     }
     if (P.path == StepPath::Generic) {
@@ -970,6 +1002,15 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     init_state();
     eng.push_back(A);
   }
+  for (size_t q = 0; q + 1 < chunk_group.size(); ++q) {
+    std::vector<char *> scr;
+    char *p = (char *)ctx->buf[BUF_SCRATCH].ptr;
+    for (size_t i = chunk_group[q]; i < chunk_group[q + 1]; ++i) {
+      scr.push_back(p);
+      p += chunk_bytes[i];
+    }
+    if (!scr.empty()) run_chunk(ctx, chunk.data() + chunk_group[q], (int)scr.size(), scr.data(), st);
+  }
   // 1-D estimations: every bandwidth step of all of them in one launch, then the
   // convergence state machine over the stored per-step f_s and means
   steps1d(ctx, line.data(), (int)line.size(), hp + al256(tjob_bytes) + 256 * (size_t)count, base + off_rjobs, st);
@@ -995,12 +1036,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     // launch boundaries do (it ran slower than the same estimations one call each).
     auto launch_fitting = [&](std::vector<EngineArgs> &v) {
       if (v.empty()) return;
-      size_t freeb = 0, totalb = 0;
-      PKDE_CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
-      size_t budget = (freeb + ctx->buf[BUF_ENGINE].bytes) / 2;
-      // PKDE_RING_BUDGET_MB caps the budget (tests use it to force one launch per estimation)
-      if (const char *cap = getenv("PKDE_RING_BUDGET_MB"); cap && *cap)
-        budget = std::min(budget, (size_t)std::max(0LL, atoll(cap)) << 20);
+      const size_t budget = shared_budget(ctx, BUF_ENGINE);
       size_t i = 0;
       while (i < v.size()) {
         size_t need = 0, j = i;

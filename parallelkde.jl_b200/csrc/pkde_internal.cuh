@@ -95,6 +95,7 @@ enum BufId {
   BUF_MISC,         // reductions
   BUF_ENGINE,       // step engine: descriptors, schedule, ring slots, counters
   BUF_BATCH,        // per-estimation buffers of a batch
+  BUF_CHUNK,        // job arrays of the chunked bandwidth steps
   BUF_COUNT_
 };
 

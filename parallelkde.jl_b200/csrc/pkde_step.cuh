@@ -157,11 +157,13 @@ struct ChunkArgs {
   StepState cs;
 };
 bool chunk_ok(const pkde_grid *g);
+// Whether an estimation that chunk_ok takes runs in chunks (a schedule file may say otherwise).
+bool chunk_schedule(pkde_ctx *ctx, const pkde_grid *g, int npairs);
 size_t chunk_scratch_bytes(const pkde_grid *g, int npairs, int nboot, int S);
 // Whether density and selected step come out final (else the caller initialises the state
 // before and fills the points without a selected step after).
 bool chunk_keeps_all(const pkde_grid *g, int npairs, int S);
-void run_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch, cudaStream_t st);
+void run_chunk(pkde_ctx *ctx, const ChunkArgs *args, int count, char *const *scratch, cudaStream_t st);
 
 // Bandwidth steps of 1-D estimations (pkde_steps1d.cu).  f_out and mu_out: S x n1, each
 // step's log scaled variance and means; cw and vscale: device arrays of S values.
