@@ -1,13 +1,11 @@
 // Bandwidth steps of N-D estimations (N >= 2) several steps at a time: one launch per pass
-// for a chunk of steps and bootstrap pairs whose intermediates stay in the L2.
+// for a chunk of steps.
 //
 //   chunk_axis_kernel   inverse FFT along axes N..2, the propagation factors applied on
 //                       the first load (FourierSpace.jl:215-262, :445-524);
-//   chunk_rows_kernel   inverse FFT along axis 1 of the z and w rows of a few pairs, the
-//                       variance-to-mean ratio of each bootstrap (DirectSpace.jl:550-552),
-//                       or of the means' rows (:747-764);
-//   chunk_var_kernel    the running variance over the bootstraps in order and the log
-//                       scaled variance of every point (:544-581);
+//   chunk_rows_kernel   inverse FFT along axis 1 of the z and w rows of the pairs in turn, the
+//                       variance-to-mean ratio of each bootstrap and its running variance
+//                       (DirectSpace.jl:544-581), or of the means' rows (:747-764);
 //   then the convergence walk (:829-1031), over all steps at the end where f and the
 //   means of every step fit in memory, else chunk by chunk.
 //
@@ -27,6 +25,11 @@ namespace {
 constexpr int kCT = 256;           // threads
 constexpr int kTilePts = 8 * kCT;  // points per tile
 constexpr int kCtas = 768 / kCT;   // CTAs per SM (80 registers a thread)
+// Row kernel: tiles of 4 points a thread (and their z and w), 128 threads where a row fits, else
+// 256 (384 x 384, 33 bootstraps, 40 steps: 5.2 ms with 128 threads, 5.8 with 256).
+constexpr int kRowPts = 4;
+constexpr int row_threads(int n) { return n <= 128 * kRowPts ? 128 : 256; }
+constexpr int row_ctas(int T) { return 640 / T; }  // CTAs per SM (96 or 128 registers a thread)
 
 // One grid axis.  Lines of n = R M points: R = 1, plain Stockham stages; R = 3 or 5 (M a power
 // of two from 8), the R interleaved sub-lines x[R n2 + n1] through the stages of M, then
@@ -63,6 +66,17 @@ __host__ __device__ __forceinline__ int axis_tiles_held(const ChunkAxis &ax) {
 
 extern __shared__ double2 smc[];
 
+// Shared memory by byte address: strided accesses then cost one 32-bit addition each.
+__device__ __forceinline__ unsigned smem_of(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ double2 lds(unsigned a) {
+  double2 v;
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts(unsigned a, double2 v) {
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
+}
+
 // A launch covers one or several estimations: blocks [block0, next job's block0) are the job's.
 struct AxisJob {
   ChunkAxis ax;
@@ -74,17 +88,19 @@ struct AxisJob {
 struct RowsJob {
   ChunkAxis ax;
   ChunkTile t;
-  int G, A, arr0, rt, pairs, np, b0, nboot, tiles, parts;  // blocks: tiles x parts x steps
+  int G, A, arr0, rt, pairs, b0, nboot, tiles;  // blocks: tiles x steps
   double inv_n;
+  const double *vscale;
   const double2 *in;
+  double2 *state;
   double *out;
 };
-struct VarJob {
-  int64_t G;
-  int nboot, blocks;  // blocks: per step
-  const double *x, *vscale;
-  double *f;
-};
+
+// 1 / i for the running variance over bootstraps, i < kChunkRecip: the IEEE quotients, filled once
+// per device; read with an index that is the same for the block.
+constexpr int kChunkRecip = 2048;
+__constant__ double c_chunk_recip[kChunkRecip];
+__device__ __forceinline__ double recip_of(int i) { return i < kChunkRecip ? c_chunk_recip[i] : 1.0 / (double)i; }
 
 // The job of this block: of several (job array and first blocks in device memory) copied into
 // shared memory, of one the kernel's own parameter.
@@ -111,75 +127,83 @@ __device__ __forceinline__ void find_job(const J *jobs, const unsigned *block0, 
   __syncthreads();
 }
 
-// Lines through every stage: input element k of line l at src(l) + k ss (loaded by ld, scaled by
-// scale(l) and f[k] where `scaled`), tiles a and b in turn, output position p of line l through
-// st(l, p, value).  Every thread calls; the caller synchronises before the tiles are reused.
-template <class Src, class Ld, class Fac, class St>
-__device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const ChunkTile &t, int a, int b,
-                                                int64_t ss, Src src, Ld ld, bool scaled, Fac fac, St st) {
-  const int R = ax.R, L = t.L, Lr = t.Lr, P = t.P;
-  const int total = ax.nst + (R > 1 ? 1 : 0);
-  auto sub = [&](int l, int &n1) {  // sub-line l = n1 L + line
-    n1 = R > 1 ? (int)fdiv((uint32_t)l, t.dL) : 0;
-    return l - n1 * L;
+// Where a tile's lines come from and go to, as byte offsets of 32 bits from a base that is the
+// same for the block.
+//   Src: at(l): offset of line l; load(offset); STEP(): bytes from element to element
+//   Dst: at(l): offset (ok(offset): the line exists); store(offset, v); step()
+// Lines through every stage, tiles a and b (byte addresses) in turn.  SCALED: element k of line
+// l is multiplied by f[k] c, (f, c) = src.factor(l).  Every thread calls; the caller
+// synchronises before the tiles are reused.
+template <int T, bool SCALED, class Src, class Dst>
+__device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const ChunkTile &t, unsigned a, unsigned b,
+                                                const Src &src, const Dst &dst) {
+  const int R = ax.R, L = t.L, Lr = t.Lr, total = ax.nst + (R > 1 ? 1 : 0);
+  const unsigned PB = t.P * 16u;
+  const FastDiv dLr = t.dLr;
+  auto put = [&](int l, int pos, int step, auto &v, auto rc) {  // elements pos + q step of line l
+    constexpr int Q = decltype(rc)::value;
+    const unsigned o = dst.at(l);
+    if (dst.ok(o)) {
+      unsigned p = o + pos * dst.step();
+      const unsigned d = step * dst.step();
+#pragma unroll
+      for (int q = 0; q < Q; ++q, p += d) dst.store(p, v[q]);
+    }
   };
-  int s0 = 0;
-  int in = b, out = a;  // tiles, as units of smc (pointers would lose the address space)
-  const int64_t rs = ss * R;
+  unsigned in = b, out = a;
+  int i0 = 0;
   if (ax.generic_first) {  // its inputs pass through the tile (R = 1)
-    for (int e = threadIdx.x; e < ax.n * L; e += kCT) {
+    for (int e = threadIdx.x; e < ax.n * L; e += T) {
       const int k = (int)fdiv((uint32_t)e, t.dL), l = e - k * L;
-      double2 v = ld(src(l) + k * ss);
-      if (scaled) {
+      double2 v = src.load(src.at(l) + k * src.step());
+      if constexpr (SCALED) {
         double c;
-        const double *f = fac(l, c);
+        const double *f = src.factor(l, c);
         const double sc = __ldg(f + k) * c;
         v = make_double2(__dmul_rn(v.x, sc), __dmul_rn(v.y, sc));
       }
-      smc[out + k * P + l] = v;
+      sts(out + k * PB + l * 16u, v);
     }
     __syncthreads();
-    in = a;
-    out = b;
   } else {
-    const Stage1 &s = ax.st[0];
+    const Stage1 s = ax.st[0];
     auto first = [&](auto rc) {
       constexpr int Q = decltype(rc)::value;
-      auto load = [&](int j, int l, double2(&v)[Q]) {
-        int n1;
-        const int line = sub(l, n1);
-        const double2 *p = src(line) + n1 * ss + (int64_t)j * rs;
-        const int64_t step = s.nb * rs;
+      const int items = s.nb * Lr;
+      const unsigned sub = src.step() * R, d = sub * s.nb;
+      for (int e = threadIdx.x; e < items; e += T) {
+        const int j = (int)fdiv((uint32_t)e, dLr), l = e - j * Lr;
+        const int n1 = R > 1 ? (int)fdiv((uint32_t)l, t.dL) : 0, line = l - n1 * L;
+        double2 v[Q];
+        unsigned p = src.at(line) + n1 * src.step() + j * sub;
 #pragma unroll
-        for (int r = 0; r < Q; ++r) v[r] = ld(p + r * step);
-        if (scaled) {
-          double c;
-          const double *f = fac(line, c) + n1 + j * R;
-          double sc[Q];
+        for (int r = 0; r < Q; ++r, p += d) v[r] = src.load(p);
+        bool done = false;
+        if constexpr (SCALED) {
+          double c, sc[Q];
+          const double *f = src.factor(line, c) + n1 + j * R;
+          const int fd = s.nb * R;
 #pragma unroll
-          for (int r = 0; r < Q; ++r) sc[r] = __ldg(f + r * s.nb * R) * c;
+          for (int r = 0; r < Q; ++r, f += fd) sc[r] = __ldg(f) * c;
           if constexpr (Q == 8) {
             if (ax.fused) {
               dft8_scaled(v, sc);
-              return true;
+              done = true;
             }
           }
+          if (!done) {
 #pragma unroll
-          for (int r = 0; r < Q; ++r) v[r] = make_double2(__dmul_rn(v[r].x, sc[r]), __dmul_rn(v[r].y, sc[r]));
+            for (int r = 0; r < Q; ++r) v[r] = make_double2(__dmul_rn(v[r].x, sc[r]), __dmul_rn(v[r].y, sc[r]));
+          }
         }
-        return false;
-      };
-      if (total == 1) {
-        line_stage<kCT, Q>(s, Lr, t.dLr, true, load, [&](int l, int pos, double2(&v)[Q]) {
+        if (!done) dft_r<Q>(v);
+        if (total == 1) {
+          put(l, j * Q, 1, v, rc);
+        } else {
+          unsigned o = out + j * Q * PB + l * 16u;
 #pragma unroll
-          for (int q = 0; q < Q; ++q) st(l, pos + q, v[q]);
-        });
-      } else {
-        line_stage<kCT, Q>(s, Lr, t.dLr, true, load, [&](int l, int pos, double2(&v)[Q]) {
-          double2 *o = smc + out + pos * P + l;
-#pragma unroll
-          for (int q = 0; q < Q; ++q) o[q * P] = v[q];
-        });
+          for (int q = 0; q < Q; ++q, o += PB) sts(o, v[q]);
+        }
       }
     };
     switch (s.R) {
@@ -190,34 +214,38 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
       default: first(std::integral_constant<int, 5>{}); break;
     }
     if (total > 1) __syncthreads();
-    in = a;
-    out = b;
-    s0 = 1;
+    i0 = 1;
   }
-  for (int i = s0; i < ax.nst; ++i) {
-    const Stage1 &s = ax.st[i];
+  in = a;
+  out = b;
+  for (int i = i0; i < ax.nst; ++i) {
+    const Stage1 s = ax.st[i];
     const bool last = i + 1 == total;
     auto stage = [&](auto rc) {
       constexpr int Q = decltype(rc)::value;
-      auto load = [&](int j, int l, double2(&v)[Q]) {
-        const double2 *p = smc + in + j * P + l;
-        const int step = s.nb * P;
+      const int items = s.nb * Lr, Ns = s.Ns;
+      const unsigned d = s.nb * PB, od = Ns * PB;
+      for (int e = threadIdx.x; e < items; e += T) {
+        const int j = (int)fdiv((uint32_t)e, dLr), l = e - j * Lr;
+        const int jq = (int)fdiv((uint32_t)j, s.dns), k = j - jq * Ns;
+        double2 v[Q];
+        unsigned p = in + j * PB + l * 16u;
 #pragma unroll
-        for (int r = 0; r < Q; ++r) v[r] = p[r * step];
-        return false;
-      };
-      if (last) {
-        line_stage<kCT, Q>(s, Lr, t.dLr, false, load, [&](int l, int pos, double2(&v)[Q]) {
+        for (int r = 0; r < Q; ++r, p += d) v[r] = lds(p);
+        if (k > 0) {
+          const double2 *w = s.tw + k * (Q - 1) - 1;
 #pragma unroll
-          for (int q = 0; q < Q; ++q) st(l, pos + q * s.Ns, v[q]);
-        });
-      } else {
-        line_stage<kCT, Q>(s, Lr, t.dLr, false, load, [&](int l, int pos, double2(&v)[Q]) {
-          double2 *o = smc + out + pos * P + l;
-          const int step = s.Ns * P;
+          for (int r = 1; r < Q; ++r) v[r] = cmul1(v[r], __ldg(w + r));
+        }
+        dft_r<Q>(v);
+        const int pos = j + jq * Ns * (Q - 1);
+        if (last) {
+          put(l, pos, Ns, v, rc);
+        } else {
+          unsigned o = out + pos * PB + l * 16u;
 #pragma unroll
-          for (int q = 0; q < Q; ++q) o[q * step] = v[q];
-        });
+          for (int q = 0; q < Q; ++q, o += od) sts(o, v[q]);
+        }
       }
     };
     switch (s.R) {
@@ -227,12 +255,18 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
       case 3: stage(std::integral_constant<int, 3>{}); break;
       case 5: stage(std::integral_constant<int, 5>{}); break;
       default:
-        if (last) line_stage_generic<kCT>(s, ax.n, Lr, t.dLr, smc + in, P, st);
-        else line_stage_generic<kCT>(s, ax.n, Lr, t.dLr, smc + in, P, [&](int l, int pos, double2 v) { smc[out + pos * P + l] = v; });
+        line_stage_generic<T>(s, ax.n, Lr, dLr, smc + (in - smem_of(smc)) / 16, t.P, [&](int l, int pos, double2 v) {
+          if (last) {
+            const unsigned o = dst.at(l);
+            if (dst.ok(o)) dst.store(o + pos * dst.step(), v);
+          } else {
+            sts(out + pos * PB + l * 16u, v);
+          }
+        });
         break;
     }
     if (!last) __syncthreads();
-    const int x = in;
+    const unsigned x = in;
     in = out;
     out = x;
   }
@@ -240,20 +274,20 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
     auto combine = [&](auto rc) {
       constexpr int Q = decltype(rc)::value;
       const int M = ax.M, items = M * L;
-      for (int e = threadIdx.x; e < items; e += kCT) {
+      for (int e = threadIdx.x; e < items; e += T) {
         const int k2 = (int)fdiv((uint32_t)e, t.dL), l = e - k2 * L;
         double2 y[Q];
+        unsigned p = in + k2 * PB + l * 16u;
 #pragma unroll
-        for (int n1 = 0; n1 < Q; ++n1) {
-          y[n1] = smc[in + k2 * P + n1 * L + l];
+        for (int n1 = 0; n1 < Q; ++n1, p += L * 16u) {
+          y[n1] = lds(p);
           if (n1 > 0) {  // the engine's combine fuses the other product of the imaginary part
             const double2 v = y[n1], w = __ldg(ax.twc + (n1 - 1) * M + k2);
             y[n1] = make_double2(__fma_rn(v.x, w.x, -__dmul_rn(v.y, w.y)), __fma_rn(v.x, w.y, __dmul_rn(v.y, w.x)));
           }
         }
         dft_r<Q>(y);
-#pragma unroll
-        for (int q = 0; q < Q; ++q) st(l, k2 + M * q, y[q]);
+        put(l, k2, M, y, rc);
       }
     };
     if (R == 3) combine(std::integral_constant<int, 3>{});
@@ -261,60 +295,80 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
   }
 }
 
-// Inverse FFT along one axis >= 2 of A arrays in each of C steps: tile = L consecutive lines
-// of the flattened (step, array, line) index.  SPECTRA: the first pass, from the spectra,
-// with the factors of every axis and the array's scalar; else in place.
+// Inverse FFT along one axis >= 2 of A arrays in each of C steps.  Tile = L consecutive lines of
+// a step's flattened (array, line) index; blocks run over the steps first, so that the steps of
+// a chunk read the same spectra while they are in the L2.  SPECTRA: the first pass, from the
+// spectra, with the factors of every axis and the array's scalar; else in place.
+template <bool SPECTRA>
+struct AxisSrc {
+  const char *base;
+  unsigned ss;
+  const unsigned *off;
+  const double *const *f;
+  const double *c;
+  __device__ __forceinline__ unsigned step() const { return ss; }
+  __device__ __forceinline__ unsigned at(int l) const { return off[l]; }
+  __device__ __forceinline__ double2 load(unsigned o) const {
+    const double2 *p = reinterpret_cast<const double2 *>(base + o);
+    return SPECTRA ? __ldg(p) : __ldcg(p);
+  }
+  __device__ __forceinline__ const double *factor(int l, double &cl) const {
+    cl = c[l];
+    return f[l];
+  }
+};
+struct AxisDst {
+  char *base;
+  unsigned ss;
+  const unsigned *off;
+  int valid;
+  __device__ __forceinline__ unsigned step() const { return ss; }
+  __device__ __forceinline__ unsigned at(int l) const { return l < valid ? off[l] : 0xffffffffu; }
+  __device__ __forceinline__ bool ok(unsigned o) const { return o != 0xffffffffu; }
+  __device__ __forceinline__ void store(unsigned o, double2 v) const {
+    __stcg(reinterpret_cast<double2 *>(base + o), v);
+  }
+};
+
 template <bool SPECTRA>
 __device__ __forceinline__ void axis_body(const AxisJob &job, unsigned block) {
   const ChunkAxis &ax = job.ax;
   const ChunkTile &t = job.t;
   const ChunkRun &run = job.run;
-  const double2 *in = job.in;
-  double2 *out = job.out;
-  int64_t *so = reinterpret_cast<int64_t *>(smc + axis_tiles_held(ax) * t.size);
-  int64_t *si = so + t.L;
-  const double **sf = reinterpret_cast<const double **>(si + t.L);
+  const double **sf = reinterpret_cast<const double **>(smc + axis_tiles_held(ax) * t.size);
   double *sc = reinterpret_cast<double *>(sf + t.L);
-  const int G = run.G;
-  {
-    const unsigned per = (unsigned)run.A * ax.lines, total = (unsigned)run.C * per;
-    for (int l = threadIdx.x; l < t.L; l += kCT) {
-      unsigned w = block * (unsigned)t.L + l;
-      const bool valid = w < total;
-      if (!valid) w = 0;
-      const unsigned c = w / per, r = w - c * per, arr = r / ax.lines;
-      unsigned li = r - arr * ax.lines;
-      const int64_t off = (int64_t)(li / ax.inner) * ax.n * ax.inner + li % ax.inner;
-      const int64_t dst = (int64_t)(c * run.A + arr) * G + off;
-      so[l] = valid ? dst : -1;
-      si[l] = SPECTRA ? (int64_t)(run.a0 + arr) * G + off : dst;
-      if (SPECTRA) {
-        const int64_t s = run.s0 + c;
-        const int ar = run.a0 + (int)arr;
-        const bool second = ar != run.mean && (ar & 1);
-        const double *tab = (second ? run.fw : run.fz) + s * run.tab_stride;
-        double f = second ? run.invG * run.cw[s] : run.invG;
-        for (int q = 0; q < run.N - 1; ++q) {
-          f *= tab[run.aoff[q] + li % run.dims[q]];
-          li /= run.dims[q];
-        }
-        sf[l] = tab + run.aoff[run.N - 1];
-        sc[l] = f;
+  unsigned *off = reinterpret_cast<unsigned *>(sc + t.L);
+  const unsigned G = run.G, lines = ax.lines, inner = ax.inner;
+  const unsigned tile = block / (unsigned)run.C, c = block - tile * run.C;
+  const unsigned w0 = tile * t.L, arr0 = w0 / lines, li0 = w0 - arr0 * lines;
+  const int valid = (int)min((unsigned)t.L, (unsigned)run.A * lines - w0);
+  for (int l = threadIdx.x; l < t.L; l += kCT) {
+    unsigned arr = arr0, li = li0 + (l < valid ? l : 0);
+    while (li >= lines) li -= lines, ++arr;
+    const unsigned o = li / inner;
+    off[l] = ((arr - arr0) * G + o * ax.n * inner + (li - o * inner)) * 16u;
+    if (SPECTRA) {
+      const int64_t s = run.s0 + c;
+      const int ar = run.a0 + (int)arr;
+      const bool second = ar != run.mean && (ar & 1);
+      const double *tab = (second ? run.fw : run.fz) + s * run.tab_stride;
+      double f = second ? run.invG * run.cw[s] : run.invG;
+      for (int q = 0; q < run.N - 1; ++q) {
+        const unsigned d = run.dims[q], up = li / d;
+        f *= tab[run.aoff[q] + (li - up * d)];
+        li = up;
       }
+      sf[l] = tab + run.aoff[run.N - 1];
+      sc[l] = f;
     }
   }
   __syncthreads();
-  chunk_transform(
-      ax, t, 0, t.size, ax.inner, [&](int l) { return in + si[l]; },
-      [](const double2 *p) { return SPECTRA ? __ldg(p) : __ldcg(p); }, SPECTRA,
-      [&](int l, double &c) {
-        c = sc[l];
-        return sf[l];
-      },
-      [&](int l, int pos, double2 v) {
-        const int64_t o = so[l];
-        if (o >= 0) __stcg(out + o + (int64_t)pos * ax.inner, v);
-      });
+  const int64_t base = (int64_t)(c * run.A + arr0) * G;
+  const AxisSrc<SPECTRA> src{
+      reinterpret_cast<const char *>(job.in + (SPECTRA ? (int64_t)(run.a0 + arr0) * G : base)), inner * 16u, off, sf, sc};
+  const AxisDst dst{reinterpret_cast<char *>(job.out + base), inner * 16u, off, valid};
+  const unsigned a = smem_of(smc);
+  chunk_transform<kCT, SPECTRA>(ax, t, a, a + t.size * 16u, src, dst);
 }
 
 template <bool SPECTRA>
@@ -335,133 +389,143 @@ __device__ __forceinline__ double chunk_vmr(double Mv, double Vv, double inv_n) 
   return div_nr(__fma_rn(-m, m, __dmul_rn(fabs(Vv), inv_n)), m);
 }
 
-__device__ __forceinline__ void cp_async16(double2 *dst, const double2 *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
+__device__ __forceinline__ void cp_async16(unsigned dst, const double2 *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// Inverse FFT along axis 1.  Tile = rows [blockIdx.x rt, + rt) of step blockIdx.z.  VMR: the z
-// and w rows of pairs [blockIdx.y np, + np) of the chunk's `pairs`, line l < rt the z row l,
-// line rt + l its w row; x[(step B + bootstrap) G + point] = the bootstrap's VMR.  The rows
-// of the next pair come in by cp.async while the VMR of this one is computed.  Else
-// the rows of the means' array, mu[step G + point] = their magnitudes.
-template <bool VMR>
+// The rows of a tile in shared memory, element k of line l at unit k PN + l.
+struct RowsTile {
+  unsigned base, ss;
+  __device__ __forceinline__ unsigned step() const { return ss; }
+  __device__ __forceinline__ unsigned at(int l) const { return base + l * 16u; }
+  __device__ __forceinline__ bool ok(unsigned) const { return true; }
+  __device__ __forceinline__ double2 load(unsigned o) const { return lds(o); }
+  __device__ __forceinline__ void store(unsigned o, double2 v) const { sts(o, v); }
+};
+
+// Inverse FFT along axis 1 of rows [tile rt, + rt) of one step.  VMR: the z and w rows of the
+// chunk's pairs in turn, line l < rt the z row l, line rt + l its w row, then the
+// variance-to-mean ratio of both bootstraps of a pair and its running variance, a thread's
+// points (at most kRowPts) in registers; the rows of the next pair come in by cp.async
+// meanwhile.  After the last pair of the estimation f = log(scaled variance); between the
+// groups of a step that is split the running (mean, m2) rests in memory.
+// Else the rows of the means' array and their magnitudes.
+template <int kRT, bool VMR>
 __device__ __forceinline__ void rows_body(const RowsJob &job, unsigned block) {
   const ChunkAxis &ax = job.ax;
   const ChunkTile &t = job.t;
-  const int G = job.G, rt = job.rt, nboot = job.nboot;
-  const double inv_n = job.inv_n;
-  const unsigned q = block / (unsigned)job.tiles, bx = block - q * job.tiles;
-  const unsigned bz = q / (unsigned)job.parts, by = q - bz * job.parts;
-  const int n = ax.n, PN = t.PN, row0 = bx * rt, nrow = min(rt, ax.lines - row0);
-  const int p0 = VMR ? by * job.np : 0, p1 = VMR ? min(p0 + job.np, job.pairs) : 1;
-  const double2 *base = job.in + ((int64_t)bz * job.A + job.arr0) * G + (int64_t)row0 * n;
-  auto load = [&](int p, int tile) {
-    double2 *dst = smc + tile;
-    const double2 *z = base + (VMR ? (int64_t)(2 * p) * G : 0);
-    const int count = nrow * n;
+  const int G = job.G, rt = job.rt, nboot = job.nboot, n = ax.n;
+  const unsigned bz = block / (unsigned)job.tiles, bx = block - bz * job.tiles;
+  const unsigned PB = t.PN * 16u, tile0 = smem_of(smc), tsize = t.size * 16u;
+  const int row0 = bx * rt, count = min(rt, ax.lines - row0) * n;
+  const double2 *z = job.in + ((int64_t)bz * job.A + job.arr0) * G + (int64_t)row0 * n;
+  // this thread's points e = threadIdx.x + q kRT of the tile: row l, element k at unit k PN + l
+  unsigned at[kRowPts];
+  {
     int l = threadIdx.x / n, k = threadIdx.x - l * n;
-    const int dl = kCT / n, dk = kCT - dl * n;
-    for (int e = threadIdx.x; e < count; e += kCT) {
-      cp_async16(dst + k * PN + l, z + e);
-      if (VMR) cp_async16(dst + k * PN + rt + l, z + G + e);
+    const int dl = kRT / n, dk = kRT - dl * n;
+#pragma unroll
+    for (int q = 0; q < kRowPts; ++q) {
+      at[q] = k * PB + l * 16u;
       l += dl;
       k += dk;
       if (k >= n) k -= n, ++l;
     }
+  }
+  auto load = [&](unsigned tile) {
+#pragma unroll
+    for (int q = 0; q < kRowPts; ++q) {
+      const int e = threadIdx.x + q * kRT;
+      if (e < count) {
+        cp_async16(tile + at[q], z + e);
+        if (VMR) cp_async16(tile + at[q] + rt * 16u, z + G + e);
+      }
+    }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  int cur = 0;  // the tile (of two) that holds the inputs
-  load(p0, 0);
-  for (int p = p0; p < p1; ++p) {
+  const int64_t o0 = (int64_t)bz * G + (int64_t)row0 * n;
+  double2 st[VMR ? kRowPts : 1];
+  if constexpr (VMR) {
+#pragma unroll
+    for (int q = 0; q < kRowPts; ++q) {
+      const int e = threadIdx.x + q * kRT;
+      st[q] = job.b0 > 0 && e < count ? job.state[o0 + e] : make_double2(0.0, 0.0);
+    }
+  }
+  const int total = ax.nst + (ax.R > 1 ? 1 : 0) + ax.generic_first;
+  unsigned cur = tile0;  // the tile (of two) that holds the inputs
+  const unsigned both = 2 * tile0 + tsize;
+  load(cur);
+  const int pairs = VMR ? job.pairs : 1;
+  for (int p = 0; p < pairs; ++p) {
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    // stage i reads one buffer and writes the other; the results lie in the buffer the last one wrote
-    const int total = ax.nst + (ax.R > 1 ? 1 : 0);
-    const int res = ((total + ax.generic_first) & 1) ? 1 - cur : cur;
-    const int dst = res * t.size, src = cur * t.size;
-    chunk_transform(
-        ax, t, t.size - src, src, PN, [&](int l) { return (const double2 *)smc + src + l; },
-        [](const double2 *q) { return *q; }, false,
-        [&](int, double &c) {
-          c = 1.0;
-          return (const double *)nullptr;
-        },
-        [&](int l, int pos, double2 v) { smc[dst + pos * PN + l] = v; });
+    // each stage reads one tile and writes the other
+    const unsigned res = (total & 1) ? both - cur : cur;
+    chunk_transform<kRT, false>(ax, t, both - cur, cur, RowsTile{cur, PB}, RowsTile{res, PB});
     __syncthreads();
-    cur = 1 - res;
-    if (p + 1 < p1) load(p + 1, cur * t.size);
-    const int count = nrow * n;
-    int l = threadIdx.x / n, k = threadIdx.x - l * n;
-    const int dl = kCT / n, dk = kCT - dl * n;
+    cur = both - res;
+    z += 2 * (int64_t)G;
+    if (p + 1 < pairs) load(cur);
     if constexpr (VMR) {
       const int b = job.b0 + 2 * p;
-      double *xa = job.out + ((int64_t)bz * nboot + b) * G + (int64_t)row0 * n;
-      for (int e = threadIdx.x; e < count; e += kCT) {
-        const double2 z = smc[dst + k * PN + l], w = smc[dst + k * PN + rt + l];
-        __stcg(xa + e, chunk_vmr(z.x, w.x, inv_n));
-        if (b + 1 < nboot) __stcg(xa + G + e, chunk_vmr(z.y, w.y, inv_n));
-        l += dl;
-        k += dk;
-        if (k >= n) k -= n, ++l;
+      const double ra = recip_of(b + 1), rb = recip_of(b + 2);
+      const bool has_b = b + 1 < nboot;
+#pragma unroll
+      for (int q = 0; q < kRowPts; ++q) {
+        if (threadIdx.x + q * kRT < count) {
+          const double2 zv = lds(res + at[q]), wv = lds(res + at[q] + rt * 16u);
+          const double xa = chunk_vmr(zv.x, wv.x, job.inv_n), xb = chunk_vmr(zv.y, wv.y, job.inv_n);
+          double delta = __dsub_rn(xa, st[q].x);
+          st[q].x = __fma_rn(delta, ra, st[q].x);
+          st[q].y = __fma_rn(delta, __dsub_rn(xa, st[q].x), st[q].y);
+          if (has_b) {
+            delta = __dsub_rn(xb, st[q].x);
+            st[q].x = __fma_rn(delta, rb, st[q].x);
+            st[q].y = __fma_rn(delta, __dsub_rn(xb, st[q].x), st[q].y);
+          }
+        }
       }
     } else {
-      for (int e = threadIdx.x; e < count; e += kCT) {
-        const double2 z = smc[dst + k * PN + l];
-        job.out[(int64_t)bz * G + (int64_t)row0 * n + e] = sqrt(__fma_rn(z.x, z.x, __dmul_rn(z.y, z.y)));
-        l += dl;
-        k += dk;
-        if (k >= n) k -= n, ++l;
+#pragma unroll
+      for (int q = 0; q < kRowPts; ++q) {
+        const int e = threadIdx.x + q * kRT;
+        if (e < count) {
+          const double2 zv = lds(res + at[q]);
+          job.out[o0 + e] = sqrt(__fma_rn(zv.x, zv.x, __dmul_rn(zv.y, zv.y)));
+        }
+      }
+    }
+  }
+  if constexpr (VMR) {
+    const bool done = job.b0 + 2 * pairs >= nboot;
+    const double vs = job.vscale[bz], bm1 = (double)(nboot - 1);
+#pragma unroll
+    for (int q = 0; q < kRowPts; ++q) {
+      const int e = threadIdx.x + q * kRT;
+      if (e < count) {
+        if (done) {
+          const double v = __ddiv_rn(__dmul_rn(vs, st[q].y), bm1);
+          job.out[o0 + e] = isfinite(v) ? log(v) : nan("");
+        } else {
+          job.state[o0 + e] = st[q];
+        }
       }
     }
   }
 }
 
-template <bool VMR>
-__global__ void __launch_bounds__(kCT, kCtas) chunk_rows_kernel(const __grid_constant__ RowsJob job) {
-  rows_body<VMR>(job, blockIdx.x);
+template <int T, bool VMR>
+__global__ void __launch_bounds__(T, row_ctas(T)) chunk_rows_kernel(const __grid_constant__ RowsJob job) {
+  rows_body<T, VMR>(job, blockIdx.x);
 }
-template <bool VMR>
-__global__ void __launch_bounds__(kCT, kCtas)
+template <int T, bool VMR>
+__global__ void __launch_bounds__(T, row_ctas(T))
     chunk_rows_many_kernel(const RowsJob *jobs, const unsigned *block0, int count) {
   __shared__ RowsJob job;
   unsigned first;
   find_job(jobs, block0, count, job, first);
-  rows_body<VMR>(job, blockIdx.x - first);
-}
-
-// Welford over the bootstraps in order, then f = log(scaled variance), of every point of the
-// job's steps.
-constexpr int kVT = 128;
-__global__ void __launch_bounds__(kVT) chunk_var_kernel(const VarJob *jobs, const unsigned *block0, int count) {
-  __shared__ VarJob J;
-  __shared__ double recip[1024];  // 1 / i, IEEE
-  unsigned first;
-  find_job(jobs, block0, count, J, first);
-  const int64_t G = J.G;
-  const unsigned step = (blockIdx.x - first) / (unsigned)J.blocks;
-  const int64_t i = (blockIdx.x - first - step * J.blocks) * (int64_t)kVT + threadIdx.x;
-  const double *p = J.x + (int64_t)step * J.nboot * G + i;
-  double mean = 0.0, m2 = 0.0;
-  for (int b0 = 0; b0 < J.nboot; b0 += 1024) {
-    const int nb = min(1024, J.nboot - b0);
-    __syncthreads();
-    for (int b = threadIdx.x; b < nb; b += kVT) recip[b] = 1.0 / (double)(b0 + b + 1);
-    __syncthreads();
-    if (i < G) {
-#pragma unroll 16
-      for (int b = 0; b < nb; ++b) {
-        const double v = __ldcg(p + (int64_t)(b0 + b) * G);
-        const double delta = __dsub_rn(v, mean);
-        mean = __fma_rn(delta, recip[b], mean);
-        m2 = __fma_rn(delta, __dsub_rn(v, mean), m2);
-      }
-    }
-  }
-  if (i < G) {
-    const double v = __ddiv_rn(__dmul_rn(J.vscale[step], m2), (double)(J.nboot - 1));
-    J.f[(int64_t)step * G + i] = isfinite(v) ? log(v) : nan("");
-  }
+  rows_body<T, VMR>(job, blockIdx.x - first);
 }
 
 // The convergence state machine over the C steps of a chunk from s0 on, state in memory.
@@ -518,69 +582,77 @@ struct ChunkShape {
   bool all_steps; // f and the means of every step are kept, the convergence walk runs once
 };
 
-// Chunks hold up to 64 MB of intermediates (half of the L2 beside the spectra and the x
-// values being written); f and means of all steps are kept up to 512 MB.
-constexpr int64_t kChunkBytes = int64_t(64) << 20, kKeepBytes = int64_t(512) << 20;
-ChunkShape chunk_shape(int64_t G, int npairs, int S) {
+// Intermediates of a chunk and f and means of all steps are held up to these many bytes.  The
+// larger the chunk the fewer launches drain the SMs; that its intermediates leave the L2
+// costs less (100 x 100, 100 bootstraps, 250 steps, 64 / 256 / 1024 / 2048 MB: 9.5 / 6.9 / 6.2 / 6.2 ms;
+// 96^3, 32, 100: 94 / 87 / 85 from 256 MB on).  Level 1 for serving lanes, whose memory admission counts on
+// it, and where the device has no room for level 0; level 2 where it has none for that.
+constexpr int64_t kChunkBytes[3] = {int64_t(1) << 30, int64_t(256) << 20, int64_t(16) << 20};
+constexpr int64_t kKeepBytes[3] = {int64_t(512) << 20, int64_t(128) << 20, int64_t(4) << 20};
+ChunkShape chunk_shape(int64_t G, int npairs, int S, int level) {
   ChunkShape c;
   const int64_t step = (int64_t)sizeof(double2) * (2 * npairs + 1) * G;
-  c.C = (int)std::max<int64_t>(1, std::min<int64_t>(S, kChunkBytes / step));
+  c.C = (int)std::max<int64_t>(1, std::min<int64_t>(S, kChunkBytes[level] / step));
   const int chunks = (S + c.C - 1) / c.C;
   c.C = (S + chunks - 1) / chunks;
   c.g = npairs;
-  if (c.C == 1 && step > kChunkBytes) {
-    c.g = (int)std::max<int64_t>(1, kChunkBytes / (2 * (int64_t)sizeof(double2) * G));
+  if (c.C == 1 && step > kChunkBytes[level]) {
+    c.g = (int)std::max<int64_t>(1, kChunkBytes[level] / (2 * (int64_t)sizeof(double2) * G));
     const int groups = (npairs + c.g - 1) / c.g;
     c.g = (npairs + groups - 1) / groups;
   }
-  c.all_steps = (int64_t)sizeof(double) * 2 * S * G <= kKeepBytes;
+  c.all_steps = (int64_t)sizeof(double) * 2 * S * G <= kKeepBytes[level];
   return c;
 }
 
 }  // namespace
 
-// Grids with an axis that is neither a power of two nor 3 or 5 times one: the engine's
-// shared-memory tiles hold few lines there (100 x 100, 100 bootstraps, 250 steps: 66 ms
-// against 8.1 ms here; 50 x 41 x 36, 32 bootstraps, 100 steps: 148 against 16.6 ms).  Small grids of
-// any lengths: a step has too few tiles for the engine's order of items (64 x 64, 33 bootstraps,
-// 40 steps: 2.0 against 0.4 ms; 64^3: 7 against 11 ms).
+// Grids with an axis that is not a power of two, and small grids of any lengths.  Against the
+// engine: its shared-memory tiles hold few lines of a length that is not 2^m, 3 2^m or 5 2^m (100 x 100,
+// 100 bootstraps, 250 steps: 66 ms, here 4.6; 50 x 41 x 36, 32 bootstraps, 100 steps: 148 and 11.9); its
+// mixed-radix tiles leave a quarter of the threads idle in their sub-transforms (96^3, 32,
+// 100: 97 and 69 ms; 24^4: 36.5 and 27); on a small grid a step has too few tiles for its order of
+// items (64 x 64, 33, 40: 2.0 and 0.4 ms).  Larger powers of two stay there (512 x 512, 64, 200: 53 ms,
+// here 69; 128^3, 32, 150: 200 and 267).
 constexpr int64_t kSmallGrid = 65536;
 bool chunk_ok(const pkde_grid *g) {
   if (g->ndim < 2) return false;
   const int64_t G = grid_size(g);
-  if (G > (int64_t(1) << 28)) return false;
-  bool any = false;
+  if (G > (int64_t(1) << 26)) return false;  // byte offsets within a tile's arrays are 32 bits
+  bool other = false;
   for (int j = 0; j < g->ndim; ++j) {
     const EngineAxis k = engine_axis(g, j);
     if (g->dims[j] > 1024 || !k.ok) return false;
-    if (!k.pow2 && k.R == 1) {
-      any = true;
-      if (!stages_ok((int)g->dims[j])) return false;
+    if (!k.pow2) {
+      other = true;
+      if (k.R == 1 && !stages_ok((int)g->dims[j])) return false;
     }
   }
-  return any || G < kSmallGrid;
+  return other || G < kSmallGrid;
 }
 
-// Scratch of one estimation: [intermediates][x][f][means].
-static void chunk_scratch(int64_t G, int npairs, int nboot, int S, const ChunkShape &c, size_t off[5]) {
+// Scratch of one estimation: [intermediates][running variance][f][means].
+static void chunk_scratch(int64_t G, int npairs, int S, const ChunkShape &c, size_t off[5]) {
   auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
   const int64_t arrays = c.g == npairs ? 2 * npairs + 1 : 2 * c.g;
   const int64_t keep = c.all_steps ? S : c.C;
   off[0] = 0;
   off[1] = off[0] + al(sizeof(double2) * (size_t)(c.C * arrays * G));
-  off[2] = off[1] + al(sizeof(double) * (size_t)((int64_t)c.C * nboot * G));
+  off[2] = off[1] + (c.g == npairs ? 0 : al(sizeof(double2) * (size_t)(c.C * G)));
   off[3] = off[2] + al(sizeof(double) * (size_t)(keep * G));
   off[4] = off[3] + al(sizeof(double) * (size_t)(keep * G));
 }
 
-size_t chunk_scratch_bytes(const pkde_grid *g, int npairs, int nboot, int S) {
+size_t chunk_scratch_bytes(const pkde_grid *g, int npairs, int S, int level) {
   const int64_t G = grid_size(g);
   size_t off[5];
-  chunk_scratch(G, npairs, nboot, S, chunk_shape(G, npairs, S), off);
+  chunk_scratch(G, npairs, S, chunk_shape(G, npairs, S, level), off);
   return off[4];
 }
 
-bool chunk_keeps_all(const pkde_grid *g, int npairs, int S) { return chunk_shape(grid_size(g), npairs, S).all_steps; }
+bool chunk_keeps_all(const pkde_grid *g, int npairs, int S, int level) {
+  return chunk_shape(grid_size(g), npairs, S, level).all_steps;
+}
 
 namespace {
 
@@ -601,8 +673,7 @@ struct Launch {
 // The launches of chunk k: axis passes (first the one that reads the spectra), rows, variances.
 struct ChunkLaunches {
   Launch<AxisJob> axis[3];
-  Launch<RowsJob> vmr, means;
-  Launch<VarJob> var;
+  Launch<RowsJob> vmr[2], means[2];  // 128 and 256 threads
 };
 
 struct ChunkPlan {
@@ -610,18 +681,19 @@ struct ChunkPlan {
   ChunkRun run;
   ChunkShape c;
   double2 *mid;
-  double *x, *f, *mu;
+  double2 *state;
+  double *f, *mu;
 };
 
 ChunkPlan plan_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch) {
   ChunkPlan P{};
   const pkde_grid *g = A.grid;
   const int N = g->ndim, G = (int)grid_size(g);
-  P.c = chunk_shape(G, A.npairs, A.S);
+  P.c = chunk_shape(G, A.npairs, A.S, A.level);
   size_t off[5];
-  chunk_scratch(G, A.npairs, A.nboot, A.S, P.c, off);
+  chunk_scratch(G, A.npairs, A.S, P.c, off);
   P.mid = (double2 *)(scratch + off[0]);
-  P.x = (double *)(scratch + off[1]);
+  P.state = (double2 *)(scratch + off[1]);
   P.f = (double *)(scratch + off[2]);
   P.mu = (double *)(scratch + off[3]);
   int inner = 1;
@@ -666,21 +738,21 @@ void add_axes(ChunkLaunches &L, const ChunkArgs &A, const ChunkPlan &P, int64_t 
     J.run.C = C;
     J.run.a0 = a0;
     J.run.A = arrays;
-    const int64_t lines = (int64_t)C * arrays * J.ax.lines;
+    const int64_t lines = (int64_t)arrays * J.ax.lines;
     const int most = kTilePts / J.ax.n;
-    J.t = make_tile(J.ax.n, J.ax.R, std::min<int64_t>(lines, most), most, false);
+    J.t = make_tile(J.ax.n, J.ax.R, lines, most, false);
     J.in = j == N - 1 ? A.spectra : P.mid;
     J.out = P.mid;
-    const size_t smem = sizeof(double2) * (size_t)axis_tiles_held(J.ax) * J.t.size + 32 * (size_t)J.t.L;
-    L.axis[N - 1 - j].add(J, (unsigned)((lines + J.t.L - 1) / J.t.L), smem);
+    const size_t smem = sizeof(double2) * (size_t)axis_tiles_held(J.ax) * J.t.size + 20 * (size_t)J.t.L;
+    L.axis[N - 1 - j].add(J, (unsigned)((lines + J.t.L - 1) / J.t.L * C), smem);
   }
 }
 
-void add_rows(pkde_ctx *ctx, Launch<RowsJob> &L, const ChunkArgs &A, const ChunkPlan &P, int C, int arrays, int arr0,
+void add_rows(Launch<RowsJob> (&Ls)[2], const ChunkArgs &A, const ChunkPlan &P, int64_t s0, int C, int arrays, int arr0,
               bool vmr, int pairs, int b0, double *out) {
   RowsJob J{};
   J.ax = P.ax[0];
-  const int per = vmr ? 2 : 1, most = std::max(1, kTilePts / (per * J.ax.n));
+  const int per = vmr ? 2 : 1, T = row_threads(J.ax.n), most = T * kRowPts / J.ax.n;
   J.rt = make_tile(J.ax.n, 1, J.ax.lines, most, false).L;
   J.t = make_tile(J.ax.n, J.ax.R, per * J.rt, per * J.rt, true);
   J.G = P.run.G;
@@ -690,20 +762,12 @@ void add_rows(pkde_ctx *ctx, Launch<RowsJob> &L, const ChunkArgs &A, const Chunk
   J.b0 = b0;
   J.nboot = A.nboot;
   J.inv_n = A.inv_n;
+  J.vscale = A.vscale + s0;
   J.in = P.mid;
+  J.state = P.state;
   J.out = out;
   J.tiles = (J.ax.lines + J.rt - 1) / J.rt;
-  // pairs per CTA: enough CTAs for a few waves, at most 8 pairs (the rows of the next pair are
-  // fetched while this one's ratios are computed)
-  J.np = 1;
-  J.parts = 1;
-  if (vmr) {
-    J.np = (int)std::max<int64_t>(
-        1, std::min<int64_t>(8, (int64_t)J.tiles * C * pairs / (6 * kCtas * (int64_t)ctx->sm_count)));
-    J.parts = (pairs + J.np - 1) / J.np;
-    J.np = (pairs + J.parts - 1) / J.parts;
-  }
-  L.add(J, (unsigned)J.tiles * J.parts * C, sizeof(double2) * 2 * (size_t)J.t.size);
+  Ls[T == 128 ? 0 : 1].add(J, (unsigned)J.tiles * C, sizeof(double2) * 2 * (size_t)J.t.size);
 }
 
 size_t al256c(size_t x) { return (x + 255) & ~size_t(255); }
@@ -744,61 +808,61 @@ void run_chunk(pkde_ctx *ctx, const ChunkArgs *args, int count, char *const *scr
       if (P.c.g == A.npairs) {
         ChunkLaunches &L = group(at);
         add_axes(L, A, P, s0, C, 0, 2 * A.npairs + 1);
-        add_rows(ctx, L.vmr, A, P, C, 2 * A.npairs + 1, 0, true, A.npairs, 0, P.x);
-        add_rows(ctx, L.means, A, P, C, 2 * A.npairs + 1, 2 * A.npairs, false, 0, 0, ms);
+        add_rows(L.vmr, A, P, s0, C, 2 * A.npairs + 1, 0, true, A.npairs, 0, fs);
+        add_rows(L.means, A, P, s0, C, 2 * A.npairs + 1, 2 * A.npairs, false, 0, 0, ms);
       } else {
         for (int p0 = 0; p0 < A.npairs; p0 += P.c.g, ++at) {
           const int np = std::min(P.c.g, A.npairs - p0);
           ChunkLaunches &L = group(at);
           add_axes(L, A, P, s0, C, 2 * p0, 2 * np);
-          add_rows(ctx, L.vmr, A, P, C, 2 * np, 0, true, np, 2 * p0, P.x);
+          add_rows(L.vmr, A, P, s0, C, 2 * np, 0, true, np, 2 * p0, fs);
         }
         ChunkLaunches &L = group(at);
         add_axes(L, A, P, s0, C, 2 * A.npairs, 1);
-        add_rows(ctx, L.means, A, P, C, 1, 0, false, 0, 0, ms);
+        add_rows(L.means, A, P, s0, C, 1, 0, false, 0, 0, ms);
       }
-      VarJob V{};
-      V.G = G;
-      V.nboot = A.nboot;
-      V.blocks = (int)((G + kVT - 1) / kVT);
-      V.x = P.x;
-      V.vscale = A.vscale + s0;
-      V.f = fs;
-      group(at).var.add(V, (unsigned)(V.blocks * C), 0);
       if (!P.c.all_steps) converge[at].push_back({e, (int)s0});
     }
   }
   // job arrays to the device in one copy
   size_t bytes = 0;
-  auto place = [&](auto &L, bool always) {
+  auto place = [&](auto &L) {
     const size_t at = bytes;
-    if (L.jobs.size() < 2 && !always) return at;  // one job: a kernel parameter
+    if (L.jobs.size() < 2) return at;  // one job: a kernel parameter
     bytes += al256c(L.jobs.size() * sizeof(L.jobs[0])) + al256c(L.jobs.size() * sizeof(unsigned));
     return at;
   };
-  std::vector<std::array<size_t, 6>> at(all.size());
+  std::vector<std::array<size_t, 7>> at(all.size());
   for (size_t i = 0; i < all.size(); ++i) {
-    for (int j = 0; j < 3; ++j) at[i][j] = place(all[i].axis[j], false);
-    at[i][3] = place(all[i].vmr, false);
-    at[i][4] = place(all[i].means, false);
-    at[i][5] = place(all[i].var, true);
+    for (int j = 0; j < 3; ++j) at[i][j] = place(all[i].axis[j]);
+    for (int j = 0; j < 2; ++j) {
+      at[i][3 + j] = place(all[i].vmr[j]);
+      at[i][5 + j] = place(all[i].means[j]);
+    }
   }
-  char *dev = (char *)ensure(ctx, BUF_CHUNK, bytes);
+  char *dev = bytes ? (char *)ensure(ctx, BUF_CHUNK, bytes) : nullptr;
   std::vector<char> host(bytes);
-  auto store = [&](auto &L, size_t o, bool always) {
-    if (L.jobs.empty() || (L.jobs.size() < 2 && !always)) return;
+  auto store = [&](auto &L, size_t o) {
+    if (L.jobs.size() < 2) return;
     std::memcpy(host.data() + o, L.jobs.data(), L.jobs.size() * sizeof(L.jobs[0]));
     std::memcpy(host.data() + o + al256c(L.jobs.size() * sizeof(L.jobs[0])), L.block0.data(),
                 L.block0.size() * sizeof(unsigned));
   };
   for (size_t i = 0; i < all.size(); ++i) {
-    for (int j = 0; j < 3; ++j) store(all[i].axis[j], at[i][j], false);
-    store(all[i].vmr, at[i][3], false);
-    store(all[i].means, at[i][4], false);
-    store(all[i].var, at[i][5], true);
+    for (int j = 0; j < 3; ++j) store(all[i].axis[j], at[i][j]);
+    for (int j = 0; j < 2; ++j) {
+      store(all[i].vmr[j], at[i][3 + j]);
+      store(all[i].means[j], at[i][5 + j]);
+    }
   }
-  PKDE_CUDA_TRY(cudaMemcpyAsync(dev, host.data(), bytes, cudaMemcpyHostToDevice, st));
-  auto launch = [&](auto &L, size_t o, int phase, auto one, auto many) {
+  if (bytes) PKDE_CUDA_TRY(cudaMemcpyAsync(dev, host.data(), bytes, cudaMemcpyHostToDevice, st));
+  if (!ctx->chunk_recip_ready) {
+    std::vector<double> r(kChunkRecip, 0.0);
+    for (int i = 1; i < kChunkRecip; ++i) r[i] = 1.0 / (double)i;
+    PKDE_CUDA_TRY(cudaMemcpyToSymbol(c_chunk_recip, r.data(), sizeof(double) * kChunkRecip));
+    ctx->chunk_recip_ready = true;
+  }
+  auto launch = [&](auto &L, size_t o, int threads, int phase, auto one, auto many) {
     if (L.jobs.empty()) return;
     using J = std::decay_t<decltype(L.jobs[0])>;
     const J *jobs = reinterpret_cast<const J *>(dev + o);
@@ -807,29 +871,25 @@ void run_chunk(pkde_ctx *ctx, const ChunkArgs *args, int count, char *const *scr
       Trace tr(ctx, phase, st);
       if (L.jobs.size() == 1) {
         allow_dynamic_smem(ctx, one, L.smem);
-        one<<<L.blocks, kCT, L.smem, st>>>(L.jobs[0]);
+        one<<<L.blocks, threads, L.smem, st>>>(L.jobs[0]);
       } else {
         allow_dynamic_smem(ctx, many, L.smem);
-        many<<<L.blocks, kCT, L.smem, st>>>(jobs, block0, (int)L.jobs.size());
+        many<<<L.blocks, threads, L.smem, st>>>(jobs, block0, (int)L.jobs.size());
       }
     }
     PKDE_CHECK_LAUNCH();
   };
   for (size_t i = 0; i < all.size(); ++i) {
     ChunkLaunches &L = all[i];
-    launch(L.axis[0], at[i][0], PKDE_PHASE_STEP_FFT, chunk_axis_kernel<true>, chunk_axis_many_kernel<true>);
+    launch(L.axis[0], at[i][0], kCT, PKDE_PHASE_STEP_FFT, chunk_axis_kernel<true>, chunk_axis_many_kernel<true>);
     for (int j = 1; j < 3; ++j)
-      launch(L.axis[j], at[i][j], PKDE_PHASE_STEP_FFT, chunk_axis_kernel<false>, chunk_axis_many_kernel<false>);
-    launch(L.vmr, at[i][3], PKDE_PHASE_STEP_VMR, chunk_rows_kernel<true>, chunk_rows_many_kernel<true>);
-    launch(L.means, at[i][4], PKDE_PHASE_STEP_MEANS, chunk_rows_kernel<false>, chunk_rows_many_kernel<false>);
-    if (!L.var.jobs.empty()) {
-      const char *o = dev + at[i][5];
-      Trace tr(ctx, PKDE_PHASE_STEP_MEANS, st);
-      chunk_var_kernel<<<L.var.blocks, kVT, 0, st>>>(
-          reinterpret_cast<const VarJob *>(o),
-          reinterpret_cast<const unsigned *>(o + al256c(L.var.jobs.size() * sizeof(VarJob))), (int)L.var.jobs.size());
-    }
-    PKDE_CHECK_LAUNCH();
+      launch(L.axis[j], at[i][j], kCT, PKDE_PHASE_STEP_FFT, chunk_axis_kernel<false>, chunk_axis_many_kernel<false>);
+    launch(L.vmr[0], at[i][3], 128, PKDE_PHASE_STEP_VMR, chunk_rows_kernel<128, true>, chunk_rows_many_kernel<128, true>);
+    launch(L.vmr[1], at[i][4], 256, PKDE_PHASE_STEP_VMR, chunk_rows_kernel<256, true>, chunk_rows_many_kernel<256, true>);
+    launch(L.means[0], at[i][5], 128, PKDE_PHASE_STEP_MEANS, chunk_rows_kernel<128, false>,
+           chunk_rows_many_kernel<128, false>);
+    launch(L.means[1], at[i][6], 256, PKDE_PHASE_STEP_MEANS, chunk_rows_kernel<256, false>,
+           chunk_rows_many_kernel<256, false>);
     for (const auto &c : converge[i]) {
       const ChunkArgs &A = args[c[0]];
       const ChunkPlan &P = plan[c[0]];

@@ -798,7 +798,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     arena += dirac_job_scratch(P.g, ests[e].n, P.B);
     if (P.path == StepPath::Chunk) {
       chunk_e.push_back(e);
-      chunk_bytes.push_back(chunk_scratch_bytes(P.g, (int)P.npairs, (int)P.B, (int)P.L.S));
+      chunk_bytes.push_back(0);
     }
     if (P.path == StepPath::Generic) {
       generic_wel = std::max(generic_wel, sizeof(double) * 2 * (size_t)P.G);
@@ -811,8 +811,28 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   // estimations in chunks of steps share launches as far as their scratch together fits the
   // memory budget: chunk_group[i] = first of the i-th set
   std::vector<size_t> chunk_group{0};
-  {
-    const size_t budget = chunk_e.size() > 1 ? shared_budget(ctx, BUF_SCRATCH) : 0;
+  int chunk_level = ctx->tune_wide ? 0 : 1;
+  if (!chunk_e.empty()) {
+    // the device's free memory is asked for only where the kept scratch does not suffice
+    size_t budget = chunk_e.size() > 1 ? shared_budget(ctx, BUF_SCRATCH) : ctx->buf[BUF_SCRATCH].bytes;
+    auto largest = [&] {
+      size_t most = 0;
+      for (size_t i = 0; i < chunk_e.size(); ++i) {
+        const Plan &P = plans[chunk_e[i]];
+        chunk_bytes[i] = chunk_scratch_bytes(P.g, (int)P.npairs, (int)P.L.S, chunk_level);
+        most = std::max(most, chunk_bytes[i]);
+      }
+      return most;
+    };
+    size_t most = largest();
+    if (most > budget) {
+      size_t freeb = 0, totalb = 0;
+      PKDE_CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
+      while (chunk_level < 2 && most > (freeb + ctx->buf[BUF_SCRATCH].bytes) / 2) {
+        ++chunk_level;
+        most = largest();
+      }
+    }
     size_t need = 0;
     for (size_t i = 0; i < chunk_e.size(); ++i) {
       if (i > chunk_group.back() && need + chunk_bytes[i] > budget) {
@@ -969,7 +989,8 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
       A.steps_low = L.steps_low;
       A.steps_over = L.steps_over;
       A.cs = P.cs;
-      P.final_state = chunk_keeps_all(P.g, A.npairs, A.S);
+      A.level = chunk_level;
+      P.final_state = chunk_keeps_all(P.g, A.npairs, A.S, chunk_level);
       if (!P.final_state) init_state();
       chunk.push_back(A);
       continue;

@@ -147,6 +147,7 @@ const double2 *combine_twiddles_device(pkde_ctx *ctx, int R, int M);
 struct ChunkArgs {
   const pkde_grid *grid;
   int npairs, nboot, S;
+  int level;  // of the scratch
   const double2 *spectra;
   const double *fz, *fw;
   int64_t tab_stride;
@@ -159,10 +160,11 @@ struct ChunkArgs {
 bool chunk_ok(const pkde_grid *g);
 // Whether an estimation that chunk_ok takes runs in chunks (a schedule file may say otherwise).
 bool chunk_schedule(pkde_ctx *ctx, const pkde_grid *g, int npairs);
-size_t chunk_scratch_bytes(const pkde_grid *g, int npairs, int nboot, int S);
+// Scratch at a memory level (0: the largest chunks .. 2).
+size_t chunk_scratch_bytes(const pkde_grid *g, int npairs, int S, int level);
 // Whether density and selected step come out final (else the caller initialises the state
 // before and fills the points without a selected step after).
-bool chunk_keeps_all(const pkde_grid *g, int npairs, int S);
+bool chunk_keeps_all(const pkde_grid *g, int npairs, int S, int level);
 void run_chunk(pkde_ctx *ctx, const ChunkArgs *args, int count, char *const *scratch, cudaStream_t st);
 
 // Bandwidth steps of 1-D estimations (pkde_steps1d.cu).  f_out and mu_out: S x n1, each
