@@ -16,8 +16,7 @@
 #include <algorithm>
 #include <cstring>
 
-#include "pkde_lines.cuh"
-#include "pkde_step.cuh"
+#include "pkde_chunk.cuh"
 
 namespace pkde {
 namespace {
@@ -30,33 +29,6 @@ constexpr int kCtas = 768 / kCT;   // CTAs per SM (80 registers a thread)
 constexpr int kRowPts = 4;
 constexpr int row_threads(int n) { return n <= 128 * kRowPts ? 128 : 256; }
 constexpr int row_ctas(int T) { return 640 / T; }  // CTAs per SM (96 or 128 registers a thread)
-
-// One grid axis.  Lines of n = R M points: R = 1, plain Stockham stages; R = 3 or 5 (M a power
-// of two from 8), the R interleaved sub-lines x[R n2 + n1] through the stages of M, then
-// one radix-R combine X[k2 + M q] = sum_n1 W_n^(n1 k2) Y_n1[k2] W_R^(n1 q) (the step
-// engine's mixed-radix arithmetic).
-struct ChunkAxis {
-  int n, M, R, nst, inner, lines;
-  int generic_first;   // the first stage has a generic radix: one more exchange
-  int fused;           // the first stage's sums fuse the scaling of one operand (power-of-two register tiles)
-  const double2 *twc;  // combine twiddles [n1 - 1][k2]
-  Stage1 st[kStages1];
-};
-// Lines of a tile: L (pitch PN where a tile holds lines), Lr = L R sub-lines (pitch P); size: units
-// of one tile.
-struct ChunkTile {
-  int L, Lr, P, PN, size;
-  FastDiv dL, dLr;
-};
-
-struct ChunkRun {
-  int N, G, A, a0, C, mean;  // A arrays from a0 per step, C steps from s0; mean: index of the means' array
-  int64_t s0, tab_stride;
-  const double *fz, *fw, *cw;
-  double invG;
-  int dims[4];
-  int64_t aoff[4];
-};
 
 // Tiles an axis pass holds: the first stage reads global memory and the last one writes it.
 __host__ __device__ __forceinline__ int axis_tiles_held(const ChunkAxis &ax) {
@@ -76,31 +48,6 @@ __device__ __forceinline__ double2 lds(unsigned a) {
 __device__ __forceinline__ void sts(unsigned a, double2 v) {
   asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
 }
-
-// A launch covers one or several estimations: blocks [block0, next job's block0) are the job's.
-struct AxisJob {
-  ChunkAxis ax;
-  ChunkTile t;
-  ChunkRun run;
-  const double2 *in;
-  double2 *out;
-};
-struct RowsJob {
-  ChunkAxis ax;
-  ChunkTile t;
-  int G, A, arr0, rt, pairs, b0, nboot, tiles;  // blocks: tiles x steps
-  double inv_n;
-  const double *vscale;
-  const double2 *in;
-  double2 *state;
-  double *out;
-};
-
-// 1 / i for the running variance over bootstraps, i < kChunkRecip: the IEEE quotients, filled once
-// per device; read with an index that is the same for the block.
-constexpr int kChunkRecip = 2048;
-__constant__ double c_chunk_recip[kChunkRecip];
-__device__ __forceinline__ double recip_of(int i) { return i < kChunkRecip ? c_chunk_recip[i] : 1.0 / (double)i; }
 
 // The job of this block: of several (job array and first blocks in device memory) copied into
 // shared memory, of one the kernel's own parameter.
@@ -384,11 +331,6 @@ __global__ void __launch_bounds__(kCT, kCtas)
   axis_body<SPECTRA>(job, blockIdx.x - first);
 }
 
-__device__ __forceinline__ double chunk_vmr(double Mv, double Vv, double inv_n) {
-  const double m = __dmul_rn(fabs(Mv), inv_n);
-  return div_nr(__fma_rn(-m, m, __dmul_rn(fabs(Vv), inv_n)), m);
-}
-
 __device__ __forceinline__ void cp_async16(unsigned dst, const double2 *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -469,21 +411,15 @@ __device__ __forceinline__ void rows_body(const RowsJob &job, unsigned block) {
     if (p + 1 < pairs) load(cur);
     if constexpr (VMR) {
       const int b = job.b0 + 2 * p;
-      const double ra = recip_of(b + 1), rb = recip_of(b + 2);
+      const double ra = recip_of(job.recip, b + 1), rb = recip_of(job.recip, b + 2);
       const bool has_b = b + 1 < nboot;
 #pragma unroll
       for (int q = 0; q < kRowPts; ++q) {
         if (threadIdx.x + q * kRT < count) {
           const double2 zv = lds(res + at[q]), wv = lds(res + at[q] + rt * 16u);
           const double xa = chunk_vmr(zv.x, wv.x, job.inv_n), xb = chunk_vmr(zv.y, wv.y, job.inv_n);
-          double delta = __dsub_rn(xa, st[q].x);
-          st[q].x = __fma_rn(delta, ra, st[q].x);
-          st[q].y = __fma_rn(delta, __dsub_rn(xa, st[q].x), st[q].y);
-          if (has_b) {
-            delta = __dsub_rn(xb, st[q].x);
-            st[q].x = __fma_rn(delta, rb, st[q].x);
-            st[q].y = __fma_rn(delta, __dsub_rn(xb, st[q].x), st[q].y);
-          }
+          chunk_welford(xa, ra, st[q]);
+          if (has_b) chunk_welford(xb, rb, st[q]);
         }
       }
     } else {
@@ -607,28 +543,23 @@ ChunkShape chunk_shape(int64_t G, int npairs, int S, int level) {
 
 }  // namespace
 
-// Grids with an axis that is not a power of two, and small grids of any lengths.  Against the
-// engine: its shared-memory tiles hold few lines of a length that is not 2^m, 3 2^m or 5 2^m (100 x 100,
-// 100 bootstraps, 250 steps: 66 ms, here 4.6; 50 x 41 x 36, 32 bootstraps, 100 steps: 148 and 11.9); its
-// mixed-radix tiles leave a quarter of the threads idle in their sub-transforms (96^3, 32,
-// 100: 97 and 69 ms; 24^4: 36.5 and 27); on a small grid a step has too few tiles for its order of
-// items (64 x 64, 33, 40: 2.0 and 0.4 ms).  Larger powers of two stay there (512 x 512, 64, 200: 53 ms,
-// here 69; 128^3, 32, 150: 200 and 267).
-constexpr int64_t kSmallGrid = 65536;
+// Grids this path takes.  Against the persistent engine (step times): its shared-memory tiles hold
+// few lines of a length that is not 2^m, 3 2^m or 5 2^m (100 x 100, 100 bootstraps, 250 steps: 66
+// ms, here 4.3; 50 x 41 x 36, 32, 100: 148 and 11.7); its mixed-radix tiles leave a quarter of the
+// threads idle (96^3, 32, 100: 97 and 69); on a small grid a step has too few tiles for its order
+// of items (64 x 64, 33, 40: 2.0 and 0.4); on large powers of two it waits for dependencies and
+// spills (512 x 512, 64, 200: 52.7 and 43.4; 128^3, 32, 150: 199 and 182).  It keeps axes of
+// 1025 to 2048 points, and runs where a schedule file or a wait limit of its own asks for it.
 bool chunk_ok(const pkde_grid *g) {
   if (g->ndim < 2) return false;
   const int64_t G = grid_size(g);
   if (G > (int64_t(1) << 26)) return false;  // byte offsets within a tile's arrays are 32 bits
-  bool other = false;
   for (int j = 0; j < g->ndim; ++j) {
     const EngineAxis k = engine_axis(g, j);
     if (g->dims[j] > 1024 || !k.ok) return false;
-    if (!k.pow2) {
-      other = true;
-      if (k.R == 1 && !stages_ok((int)g->dims[j])) return false;
-    }
+    if (!k.pow2 && k.R == 1 && !stages_ok((int)g->dims[j])) return false;
   }
-  return other || G < kSmallGrid;
+  return true;
 }
 
 // Scratch of one estimation: [intermediates][running variance][f][means].
@@ -656,6 +587,8 @@ bool chunk_keeps_all(const pkde_grid *g, int npairs, int S, int level) {
 
 namespace {
 
+constexpr unsigned kSoloBlocks = 600;  // two waves of the general kernels
+
 // One launch of a pass over the jobs of several estimations.
 template <class J>
 struct Launch {
@@ -663,7 +596,14 @@ struct Launch {
   std::vector<unsigned> block0;
   unsigned blocks = 0;
   size_t smem = 0;
-  void add(const J &j, unsigned n, size_t bytes) {
+  // power-of-two jobs with a kernel of their own, launched one by one: alone in their pass, or
+  // large enough to fill the device
+  std::vector<J> solo;
+  void add(const J &j, unsigned n, size_t bytes, bool alone) {
+    if (j.ax.fused && (alone || n >= kSoloBlocks)) {
+      solo.push_back(j);
+      return;
+    }
     jobs.push_back(j);
     block0.push_back(blocks);
     blocks += n;
@@ -683,13 +623,26 @@ struct ChunkPlan {
   double2 *mid;
   double2 *state;
   double *f, *mu;
+  const double *recip;
 };
+
+const double *recip_table(pkde_ctx *ctx) {
+  DevBuf &b = ctx->chunk_recip;
+  if (!b.ptr) {
+    std::vector<double> r(kChunkRecip, 0.0);
+    for (int i = 1; i < kChunkRecip; ++i) r[i] = 1.0 / (double)i;
+    b.ensure(sizeof(double) * kChunkRecip);
+    PKDE_CUDA_TRY(cudaMemcpy(b.ptr, r.data(), sizeof(double) * kChunkRecip, cudaMemcpyHostToDevice));
+  }
+  return b.as<double>();
+}
 
 ChunkPlan plan_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch) {
   ChunkPlan P{};
   const pkde_grid *g = A.grid;
   const int N = g->ndim, G = (int)grid_size(g);
   P.c = chunk_shape(G, A.npairs, A.S, A.level);
+  P.recip = recip_table(ctx);
   size_t off[5];
   chunk_scratch(G, A.npairs, A.S, P.c, off);
   P.mid = (double2 *)(scratch + off[0]);
@@ -728,7 +681,8 @@ ChunkPlan plan_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch) {
 }
 
 // Passes over axes N..2 of `arrays` arrays from a0 in C steps from s0.
-void add_axes(ChunkLaunches &L, const ChunkArgs &A, const ChunkPlan &P, int64_t s0, int C, int a0, int arrays) {
+void add_axes(ChunkLaunches &L, const ChunkArgs &A, const ChunkPlan &P, int64_t s0, int C, int a0, int arrays,
+              bool alone) {
   const int N = P.run.N;
   for (int j = N - 1; j >= 1; --j) {
     AxisJob J{};
@@ -744,12 +698,12 @@ void add_axes(ChunkLaunches &L, const ChunkArgs &A, const ChunkPlan &P, int64_t 
     J.in = j == N - 1 ? A.spectra : P.mid;
     J.out = P.mid;
     const size_t smem = sizeof(double2) * (size_t)axis_tiles_held(J.ax) * J.t.size + 20 * (size_t)J.t.L;
-    L.axis[N - 1 - j].add(J, (unsigned)((lines + J.t.L - 1) / J.t.L * C), smem);
+    L.axis[N - 1 - j].add(J, (unsigned)((lines + J.t.L - 1) / J.t.L * C), smem, alone);
   }
 }
 
 void add_rows(Launch<RowsJob> (&Ls)[2], const ChunkArgs &A, const ChunkPlan &P, int64_t s0, int C, int arrays, int arr0,
-              bool vmr, int pairs, int b0, double *out) {
+              bool vmr, int pairs, int b0, double *out, bool alone) {
   RowsJob J{};
   J.ax = P.ax[0];
   const int per = vmr ? 2 : 1, T = row_threads(J.ax.n), most = T * kRowPts / J.ax.n;
@@ -763,11 +717,14 @@ void add_rows(Launch<RowsJob> (&Ls)[2], const ChunkArgs &A, const ChunkPlan &P, 
   J.nboot = A.nboot;
   J.inv_n = A.inv_n;
   J.vscale = A.vscale + s0;
+  J.recip = P.recip;
   J.in = P.mid;
   J.state = P.state;
   J.out = out;
   J.tiles = (J.ax.lines + J.rt - 1) / J.rt;
-  Ls[T == 128 ? 0 : 1].add(J, (unsigned)J.tiles * C, sizeof(double2) * 2 * (size_t)J.t.size);
+  J.C = C;
+  if (!vmr) J.ax.fused = 0;  // no kernel of its own
+  Ls[T == 128 ? 0 : 1].add(J, (unsigned)J.tiles * C, sizeof(double2) * 2 * (size_t)J.t.size, alone);
 }
 
 size_t al256c(size_t x) { return (x + 255) & ~size_t(255); }
@@ -807,19 +764,19 @@ void run_chunk(pkde_ctx *ctx, const ChunkArgs *args, int count, char *const *scr
       };
       if (P.c.g == A.npairs) {
         ChunkLaunches &L = group(at);
-        add_axes(L, A, P, s0, C, 0, 2 * A.npairs + 1);
-        add_rows(L.vmr, A, P, s0, C, 2 * A.npairs + 1, 0, true, A.npairs, 0, fs);
-        add_rows(L.means, A, P, s0, C, 2 * A.npairs + 1, 2 * A.npairs, false, 0, 0, ms);
+        add_axes(L, A, P, s0, C, 0, 2 * A.npairs + 1, count == 1);
+        add_rows(L.vmr, A, P, s0, C, 2 * A.npairs + 1, 0, true, A.npairs, 0, fs, count == 1);
+        add_rows(L.means, A, P, s0, C, 2 * A.npairs + 1, 2 * A.npairs, false, 0, 0, ms, count == 1);
       } else {
         for (int p0 = 0; p0 < A.npairs; p0 += P.c.g, ++at) {
           const int np = std::min(P.c.g, A.npairs - p0);
           ChunkLaunches &L = group(at);
-          add_axes(L, A, P, s0, C, 2 * p0, 2 * np);
-          add_rows(L.vmr, A, P, s0, C, 2 * np, 0, true, np, 2 * p0, fs);
+          add_axes(L, A, P, s0, C, 2 * p0, 2 * np, count == 1);
+          add_rows(L.vmr, A, P, s0, C, 2 * np, 0, true, np, 2 * p0, fs, count == 1);
         }
         ChunkLaunches &L = group(at);
-        add_axes(L, A, P, s0, C, 2 * A.npairs, 1);
-        add_rows(L.means, A, P, s0, C, 1, 0, false, 0, 0, ms);
+        add_axes(L, A, P, s0, C, 2 * A.npairs, 1, count == 1);
+        add_rows(L.means, A, P, s0, C, 1, 0, false, 0, 0, ms, count == 1);
       }
       if (!P.c.all_steps) converge[at].push_back({e, (int)s0});
     }
@@ -856,13 +813,8 @@ void run_chunk(pkde_ctx *ctx, const ChunkArgs *args, int count, char *const *scr
     }
   }
   if (bytes) PKDE_CUDA_TRY(cudaMemcpyAsync(dev, host.data(), bytes, cudaMemcpyHostToDevice, st));
-  if (!ctx->chunk_recip_ready) {
-    std::vector<double> r(kChunkRecip, 0.0);
-    for (int i = 1; i < kChunkRecip; ++i) r[i] = 1.0 / (double)i;
-    PKDE_CUDA_TRY(cudaMemcpyToSymbol(c_chunk_recip, r.data(), sizeof(double) * kChunkRecip));
-    ctx->chunk_recip_ready = true;
-  }
-  auto launch = [&](auto &L, size_t o, int threads, int phase, auto one, auto many) {
+  auto launch = [&](auto &L, size_t o, int threads, int phase, auto one, auto many, auto pow2) {
+    for (const auto &j : L.solo) pow2(j);
     if (L.jobs.empty()) return;
     using J = std::decay_t<decltype(L.jobs[0])>;
     const J *jobs = reinterpret_cast<const J *>(dev + o);
@@ -881,15 +833,20 @@ void run_chunk(pkde_ctx *ctx, const ChunkArgs *args, int count, char *const *scr
   };
   for (size_t i = 0; i < all.size(); ++i) {
     ChunkLaunches &L = all[i];
-    launch(L.axis[0], at[i][0], kCT, PKDE_PHASE_STEP_FFT, chunk_axis_kernel<true>, chunk_axis_many_kernel<true>);
+    launch(L.axis[0], at[i][0], kCT, PKDE_PHASE_STEP_FFT, chunk_axis_kernel<true>, chunk_axis_many_kernel<true>,
+           [&](const AxisJob &J) { return chunk_pow2_axis(ctx, J, true, st); });
     for (int j = 1; j < 3; ++j)
-      launch(L.axis[j], at[i][j], kCT, PKDE_PHASE_STEP_FFT, chunk_axis_kernel<false>, chunk_axis_many_kernel<false>);
-    launch(L.vmr[0], at[i][3], 128, PKDE_PHASE_STEP_VMR, chunk_rows_kernel<128, true>, chunk_rows_many_kernel<128, true>);
-    launch(L.vmr[1], at[i][4], 256, PKDE_PHASE_STEP_VMR, chunk_rows_kernel<256, true>, chunk_rows_many_kernel<256, true>);
+      launch(L.axis[j], at[i][j], kCT, PKDE_PHASE_STEP_FFT, chunk_axis_kernel<false>, chunk_axis_many_kernel<false>,
+             [&](const AxisJob &J) { return chunk_pow2_axis(ctx, J, false, st); });
+    auto pow2_rows = [&](const RowsJob &J) { return chunk_pow2_rows(ctx, J, st); };
+    launch(L.vmr[0], at[i][3], 128, PKDE_PHASE_STEP_VMR, chunk_rows_kernel<128, true>, chunk_rows_many_kernel<128, true>,
+           pow2_rows);
+    launch(L.vmr[1], at[i][4], 256, PKDE_PHASE_STEP_VMR, chunk_rows_kernel<256, true>, chunk_rows_many_kernel<256, true>,
+           pow2_rows);
     launch(L.means[0], at[i][5], 128, PKDE_PHASE_STEP_MEANS, chunk_rows_kernel<128, false>,
-           chunk_rows_many_kernel<128, false>);
+           chunk_rows_many_kernel<128, false>, [](const RowsJob &) {});
     launch(L.means[1], at[i][6], 256, PKDE_PHASE_STEP_MEANS, chunk_rows_kernel<256, false>,
-           chunk_rows_many_kernel<256, false>);
+           chunk_rows_many_kernel<256, false>, [](const RowsJob &) {});
     for (const auto &c : converge[i]) {
       const ChunkArgs &A = args[c[0]];
       const ChunkPlan &P = plan[c[0]];

@@ -1,0 +1,79 @@
+// Job descriptors of the chunked bandwidth steps (pkde_chunk.cu, pkde_chunk_pow2.cu).
+#pragma once
+
+#include "pkde_lines.cuh"
+#include "pkde_step.cuh"
+
+namespace pkde {
+
+// One grid axis.  Lines of n = R M points: R = 1, plain Stockham stages; R = 3 or 5 (M a power
+// of two from 8), the R interleaved sub-lines x[R n2 + n1] through the stages of M, then
+// one radix-R combine X[k2 + M q] = sum_n1 W_n^(n1 k2) Y_n1[k2] W_R^(n1 q) (the step
+// engine's mixed-radix arithmetic).
+struct ChunkAxis {
+  int n, M, R, nst, inner, lines;
+  int generic_first;   // the first stage has a generic radix: one more exchange
+  int fused;           // the first stage's sums fuse the scaling of one operand (power-of-two register tiles)
+  const double2 *twc;  // combine twiddles [n1 - 1][k2]
+  Stage1 st[kStages1];
+};
+// Lines of a tile: L (pitch PN where a tile holds lines), Lr = L R sub-lines (pitch P); size: units
+// of one tile.
+struct ChunkTile {
+  int L, Lr, P, PN, size;
+  FastDiv dL, dLr;
+};
+
+struct ChunkRun {
+  int N, G, A, a0, C, mean;  // A arrays from a0 per step, C steps from s0; mean: index of the means' array
+  int64_t s0, tab_stride;
+  const double *fz, *fw, *cw;
+  double invG;
+  int dims[4];
+  int64_t aoff[4];
+};
+
+// A launch covers one or several estimations: blocks [block0, next job's block0) are the job's.
+struct AxisJob {
+  ChunkAxis ax;
+  ChunkTile t;
+  ChunkRun run;
+  const double2 *in;
+  double2 *out;
+};
+struct RowsJob {
+  ChunkAxis ax;
+  ChunkTile t;
+  int G, A, C, arr0, rt, pairs, b0, nboot, tiles;  // blocks: tiles x steps
+  double inv_n;
+  const double *vscale, *recip;
+  const double2 *in;
+  double2 *state;
+  double *out;
+};
+
+// 1 / i for the running variance over bootstraps: a table of the IEEE quotients for i < kChunkRecip,
+// read with an index that is the same for the block.
+constexpr int kChunkRecip = 4096;
+__device__ __forceinline__ double recip_of(const double *table, int i) {
+  return i < kChunkRecip ? __ldg(table + i) : 1.0 / (double)i;
+}
+
+// VMR of one bootstrap at one point (DirectSpace.jl:550-552), 1 / n as a product.
+__device__ __forceinline__ double chunk_vmr(double Mv, double Vv, double inv_n) {
+  const double m = __dmul_rn(fabs(Mv), inv_n);
+  return div_nr(__fma_rn(-m, m, __dmul_rn(fabs(Vv), inv_n)), m);
+}
+
+__device__ __forceinline__ void chunk_welford(double x, double inv, double2 &st) {
+  const double delta = __dsub_rn(x, st.x);
+  st.x = __fma_rn(delta, inv, st.x);
+  st.y = __fma_rn(delta, __dsub_rn(x, st.x), st.y);
+}
+
+// Passes along power-of-two axes (ax.fused, 16 to 1024 points) on register tiles
+// (pkde_chunk_pow2.cu).
+void chunk_pow2_axis(pkde_ctx *ctx, const AxisJob &J, bool spectra, cudaStream_t st);
+void chunk_pow2_rows(pkde_ctx *ctx, const RowsJob &J, cudaStream_t st);
+
+}  // namespace pkde

@@ -78,6 +78,7 @@ int pkde_destroy(pkde_ctx *ctx) {
   for (auto &b : ctx->buf) b.release();
   for (auto &t : ctx->twiddles) t.second.release();
   for (auto &t : ctx->stage_tw) t.second.release();
+  ctx->chunk_recip.release();
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
   if (ctx->engine_flags) cudaFreeHost(ctx->engine_flags);
   delete ctx;

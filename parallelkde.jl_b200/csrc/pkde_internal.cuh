@@ -101,6 +101,11 @@ enum BufId {
 
 }  // namespace pkde
 
+// Polls a step-engine dependency wait makes before it gives up (pkde_set_wait_limit).
+namespace pkde {
+constexpr int64_t kDefaultWaitLimit = 20000000;
+}
+
 struct pkde_ctx {
   int device = 0;
   pkde::DevBuf buf[pkde::BUF_COUNT_];
@@ -119,10 +124,10 @@ struct pkde_ctx {
   bool tune_wide = true;
   bool tune_loaded = false;
   bool recip_ready = false;  // the step engine's table of 1/i is in this device's constant memory
-  bool chunk_recip_ready = false;  // the same for the chunked steps' table
+  pkde::DevBuf chunk_recip;  // the chunked steps' table of 1/i
   std::map<std::string, std::array<int, 3>> tune;
   // polls a step-engine dependency wait makes before it gives up (pkde_set_wait_limit)
-  int64_t wait_limit = 20000000;
+  int64_t wait_limit = pkde::kDefaultWaitLimit;
   // host-side fault injection for tests (pkde_set_fault): one-shot
   int fault_point = PKDE_FAULT_NONE;
   // step-engine error flags, copied back without a synchronisation of their own and

@@ -23,7 +23,12 @@ pytestmark = pytest.mark.gpu
     ((100, 40, 16), 5000, 4, 5),      # mixed-radix columns that read the spectra
     ((20, 48, 10), 5000, 4, 6),       # mixed-radix columns in place
     ((10, 12, 14, 9), 4000, 3, 4),    # 4-D
-    ((64, 64), 5000, 6, 20),          # powers of two
+    ((64, 64), 5000, 6, 20),          # powers of two: register tiles
+    ((16, 16), 500, 5, 40),           # shortest lines; more steps than a CTA holds spectra for
+    ((1024, 16), 5000, 3, 5),         # longest rows: z and w are the whole CTA
+    ((16, 1024), 5000, 4, 5),         # longest columns
+    ((256, 32, 64), 8000, 5, 6),      # a pass in place between the two
+    ((64, 48, 32), 8000, 4, 6),       # register tiles first and last, mixed radix between
     ((300, 300), 20000, 35, 4),       # several pair groups a step
     ((1000, 900), 20000, 2, 38),      # f and means of one chunk at a time
 ])
