@@ -137,15 +137,13 @@ __global__ void quantize_kernel(GridDev g, const double *__restrict__ rh, int64_
 }
 
 // Scatter of the quantised terms.  Destination u64 slot of (resample b, cell, array):
-//   paired layout (spectra): ((2*(b/2) + arr) * G + cell) * 2 + (b % 2), identity slot
-//   (b == nboot) at (2*npairs*G + cell) * 2;  plain layout: arr_base[arr] + b*G + cell.
-template <bool PAIRED>
+//   arr_base[arr] + b*G + cell.
 __global__ void weight_kernel(const uint32_t *__restrict__ cell, int64_t n, int64_t nslots, int64_t nboot,
                               int64_t G, int ndim, const int64_t *__restrict__ corner_off,
                               const int32_t *__restrict__ idx, uint64_t seed,
                               const unsigned long long *__restrict__ qm,
                               const unsigned long long *__restrict__ qv, unsigned long long *__restrict__ outM,
-                              unsigned long long *__restrict__ outV, int64_t npairs, int *err) {
+                              unsigned long long *__restrict__ outV, int *err) {
   const int64_t total = nslots * n;
   const int nc = 1 << ndim;
   for (int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; d < total;
@@ -157,290 +155,8 @@ __global__ void weight_kernel(const uint32_t *__restrict__ cell, int64_t n, int6
     for (int c = 0; c < nc; ++c) {
       int64_t cc = c0 + corner_off[c];
       unsigned long long m = qm[c * n + s];
-      if (PAIRED) {
-        if (b == nboot) {
-          atomicAdd(&outM[(2 * npairs * G + cc) * 2], m);
-        } else {
-          int64_t p = b >> 1, lane = b & 1;
-          atomicAdd(&outM[((2 * p) * G + cc) * 2 + lane], m);
-          if (qv) atomicAdd(&outM[((2 * p + 1) * G + cc) * 2 + lane], qv[c * n + s]);
-        }
-      } else {
-        atomicAdd(&outM[b * G + cc], m);
-        if (qv && outV && b < nboot) atomicAdd(&outV[b * G + cc], qv[c * n + s]);
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Estimator scatter in cell order.  The samples are sorted by lower cell once (a counting
-// sort from the identity counts); each bootstrap's draws become per-sample
-// multiplicities m[b][i] (i = position in cell order); the scatter then walks (b, i) in
-// order and adds m * term.  Neighbouring threads hit neighbouring cells, and within a
-// warp the contributions of equal cells are summed (segmented scan) before one atomic.
-// All sums are exact 64-bit integers, so the result equals the per-draw scatter's.
-
-constexpr int kScanChunk = 2048;  // cells per block in the scans
-
-// per-chunk sums of the identity counts (the samples per cell)
-__global__ void cell_chunk_sum_kernel(const uint32_t *__restrict__ cnt, int64_t G, uint32_t *__restrict__ csum) {
-  __shared__ uint32_t sh[kThreads / 32];
-  const int64_t c0 = (int64_t)blockIdx.x * kScanChunk;
-  uint32_t v = 0;
-  for (int k = threadIdx.x; k < kScanChunk; k += blockDim.x)
-    if (c0 + k < G) v += cnt[c0 + k];
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (int w = 0; w < kThreads / 32; ++w) t += sh[w];
-    csum[blockIdx.x] = t;
-  }
-}
-
-// exclusive scan of the chunk sums (one block, in order)
-__global__ void chunk_scan_kernel(uint32_t *csum, int64_t nchunks) {
-  if (threadIdx.x != 0) return;
-  uint32_t run = 0;
-  for (int64_t k = 0; k < nchunks; ++k) {
-    const uint32_t v = csum[k];
-    csum[k] = run;
-    run += v;
-  }
-}
-
-// cstart[c] = first position of cell c in cell order (exclusive scan of the counts);
-// also clears the per-cell fill counters
-__global__ void cell_start_kernel(const uint32_t *__restrict__ cnt, int64_t G, const uint32_t *__restrict__ csum,
-                                  uint32_t *__restrict__ cstart, uint32_t *__restrict__ cfill) {
-  __shared__ uint32_t part[kThreads];
-  const int64_t c0 = (int64_t)blockIdx.x * kScanChunk;
-  constexpr int PER = kScanChunk / kThreads;
-  uint32_t v[PER];
-  uint32_t t = 0;
-#pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int64_t c = c0 + threadIdx.x * PER + q;
-    v[q] = c < G ? cnt[c] : 0u;
-    t += v[q];
-  }
-  part[threadIdx.x] = t;
-  __syncthreads();
-  if (threadIdx.x == 0) {  // exclusive scan of the per-thread sums (256 values)
-    uint32_t run = csum[blockIdx.x];
-    for (int k = 0; k < kThreads; ++k) {
-      const uint32_t x = part[k];
-      part[k] = run;
-      run += x;
-    }
-  }
-  __syncthreads();
-  uint32_t run = part[threadIdx.x];
-#pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int64_t c = c0 + threadIdx.x * PER + q;
-    if (c < G) {
-      cstart[c] = run;
-      cfill[c] = 0u;
-    }
-    run += v[q];
-  }
-}
-
-// pos[s] = position of sample s in cell order; cell_sorted[pos] = its lower cell
-__global__ void cell_sort_kernel(const uint32_t *__restrict__ cell, int64_t n, const uint32_t *__restrict__ cstart,
-                                 uint32_t *__restrict__ cfill, uint32_t *__restrict__ pos,
-                                 uint32_t *__restrict__ cell_sorted) {
-  for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t c = cell[s];
-    const uint32_t p = cstart[c] + atomicAdd(&cfill[c], 1u);
-    pos[s] = p;
-    cell_sorted[p] = c;
-  }
-}
-
-// mult[b * n + pos[s]] = how often resample b draws sample s
-__global__ void mult_kernel(int64_t n, int64_t nboot, const int32_t *__restrict__ idx, uint64_t seed,
-                            const uint32_t *__restrict__ pos, uint32_t *__restrict__ mult, int *err) {
-  const int64_t total = nboot * n;
-  for (int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; d < total; d += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = d / n;
-    const int64_t j = d - b * n;
-    const int64_t s = draw_sample(b, j, n, nboot, idx, seed, err);
-    atomicAdd(&mult[b * n + pos[s]], 1u);
-  }
-}
-
-// counts[b][cell] for the bootstrap resamples, summed from the multiplicities in cell
-// order instead of one atomic per draw: the lanes of a warp hold consecutive (resample,
-// position) entries, a segmented shuffle scan sums equal (resample, cell) keys, and the
-// last lane of each run adds the run's sum with one atomic.
-__global__ void resample_count_kernel(const uint32_t *__restrict__ cell_sorted, int64_t n, int64_t nboot, int64_t G,
-                                      const uint32_t *__restrict__ mult, uint32_t *__restrict__ counts) {
-  const int lane = threadIdx.x & 31;
-  const int64_t total = nboot * n;
-  // the loop bound is rounded up to whole warps, so the shuffles always see all 32 lanes
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; d - lane < total; d += stride) {
-    const bool act = d < total;
-    const int64_t b = act ? d / n : 0;
-    const int64_t i = act ? d - b * n : 0;
-    uint32_t v = act ? mult[d] : 0u;
-    const uint32_t c0 = act ? cell_sorted[i] : 0u;
-    const unsigned long long key = act ? (((unsigned long long)b << 32) | c0) : ~0ull - (unsigned long long)lane;
-    bool same[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      const unsigned long long up = __shfl_up_sync(0xffffffffu, key, 1 << k);
-      same[k] = lane >= (1 << k) && up == key;
-    }
-    const bool last = __shfl_down_sync(0xffffffffu, key, 1) != key || lane == 31;
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      const uint32_t u = __shfl_up_sync(0xffffffffu, v, 1 << k);
-      if (same[k]) v += u;
-    }
-    if (act && last && v) atomicAdd(&counts[b * G + c0], v);
-  }
-}
-
-// The quantised corner terms of DirectSpace.jl:227-237, stored at the sample's position
-// in cell order (quantize_kernel's arithmetic).
-__device__ __forceinline__ void quantize2(double v, int e, int L, unsigned long long &hi, long long &lo) {
-  // v 2^e = hi + f (hi the nearest integer, |f| <= 1/2, both exact), lo = f 2^L rounded
-  const double x = ldexp(v, e);
-  const double xr = rint(x);
-  hi = (unsigned long long)xr;
-  lo = __double2ll_rn(ldexp(x - xr, L));
-}
-
-__global__ void quantize_sorted_kernel(GridDev g, const double *__restrict__ rh, int64_t n, double denom,
-                                       const int *__restrict__ esc, const uint32_t *__restrict__ pos,
-                                       unsigned long long *__restrict__ qm, unsigned long long *__restrict__ qv,
-                                       long long *__restrict__ qm_lo, long long *__restrict__ qv_lo) {
-  int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  const int e_m = esc[0], e_v = esc[1], L = esc[2];
-  const int N = g.ndim;
-  const int64_t ps = pos[s];
-  double r_h[4], r_l[4];
-  for (int j = 0; j < N; ++j) {
-    r_h[j] = rh[j * n + s];
-    r_l[j] = __dsub_rn(g.h[j], r_h[j]);
-  }
-  const int nc = 1 << N;
-  for (int c = 0; c < nc; ++c) {
-    double pl = 1.0, ph = 1.0;
-    bool fl = false, fh = false;
-    for (int j = 0; j < N; ++j) {
-      if ((c >> (N - 1 - j)) & 1) {
-        pl = fl ? __dmul_rn(pl, r_l[j]) : r_l[j];
-        fl = true;
-      } else {
-        ph = fh ? __dmul_rn(ph, r_h[j]) : r_h[j];
-        fh = true;
-      }
-    }
-    double term = __ddiv_rn(__dmul_rn(pl, ph), denom);
-    double sq = __dmul_rn(term, term);
-    quantize2(term, e_m, L, qm[c * n + ps], qm_lo[c * n + ps]);
-    quantize2(sq, e_v, L, qv[c * n + ps], qv_lo[c * n + ps]);
-  }
-}
-
-// Scatter in cell order into the paired spectra slots.  Work item d = (chunk c, i),
-// c-major: sample position i (cell order) for the BC resamples b = c BC .. c BC + BC - 1
-// (b = nboot the identity, multiplicity 1).  The thread loads its sample's quantised
-// corner terms once and reuses them for every resample of its chunk (the term arrays,
-// 4 x 2^N x n words, need not stay in L2 across resamples).  Warp lanes hold consecutive
-// items of one chunk, so in every iteration they share b and their keys (b, cell) are
-// non-decreasing along the warp: equal keys are contiguous and an inclusive segmented
-// scan sums each run; the run's last lane adds it with one atomic per part.
-template <int N>
-__global__ void weight_sorted_kernel(const uint32_t *__restrict__ cell_sorted, int64_t n, int64_t nboot, int64_t G,
-                                     const int64_t *__restrict__ corner_off, const uint32_t *__restrict__ mult,
-                                     const unsigned long long *__restrict__ qm,
-                                     const unsigned long long *__restrict__ qv, const long long *__restrict__ qm_lo,
-                                     const long long *__restrict__ qv_lo, unsigned long long *__restrict__ out,
-                                     unsigned long long *__restrict__ out_lo, int64_t npairs, int BC, int64_t nchunk) {
-  constexpr int nc = 1 << N;
-  constexpr bool REG = N <= 3;  // terms held in registers (4-D: re-read, from L1)
-  const int lane = threadIdx.x & 31;
-  const int64_t total = nchunk * n;
-  // every lane of a warp runs the same number of iterations (the loop bound is rounded
-  // up to whole warps, the resample loop has the same trip count in every lane), so the
-  // shuffles always see all 32 lanes
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; d - lane < total; d += stride) {
-    const bool act = d < total;
-    const int64_t c = act ? d / n : 0;
-    const int64_t i = act ? d - c * n : 0;
-    const uint32_t c0 = act ? cell_sorted[i] : 0u;
-    const unsigned long long key = act ? (((unsigned long long)c << 32) | c0) : ~0ull - (unsigned long long)lane;
-    bool same[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      const unsigned long long up = __shfl_up_sync(0xffffffffu, key, 1 << k);
-      same[k] = lane >= (1 << k) && up == key;
-    }
-    const bool last = __shfl_down_sync(0xffffffffu, key, 1) != key || lane == 31;
-    unsigned long long rqm[REG ? nc : 1], rqv[REG ? nc : 1];
-    long long rlm[REG ? nc : 1], rlv[REG ? nc : 1];
-    if constexpr (REG) {
-#pragma unroll
-      for (int q = 0; q < nc; ++q) {
-        rqm[q] = act ? qm[q * n + i] : 0ull;
-        rqv[q] = act ? qv[q * n + i] : 0ull;
-        rlm[q] = act ? qm_lo[q * n + i] : 0ll;
-        rlv[q] = act ? qv_lo[q * n + i] : 0ll;
-      }
-    }
-    for (int bb = 0; bb < BC; ++bb) {
-      const int64_t b = c * BC + bb;
-      const bool ab = act && b <= nboot;
-      const uint32_t m = ab ? (b == nboot ? 1u : mult[b * n + i]) : 0u;
-      const int64_t p = b >> 1, half = b & 1;
-#pragma unroll
-      for (int q = 0; q < nc; ++q) {
-        const int64_t cc = (int64_t)c0 + (act ? corner_off[q] : 0);
-        const unsigned long long tm = REG ? rqm[q] : (m ? __ldg(qm + q * n + i) : 0ull);
-        const unsigned long long tv = REG ? rqv[q] : (m ? __ldg(qv + q * n + i) : 0ull);
-        const long long tlm = REG ? rlm[q] : (m ? __ldg(qm_lo + q * n + i) : 0ll);
-        const long long tlv = REG ? rlv[q] : (m ? __ldg(qv_lo + q * n + i) : 0ll);
-        unsigned long long vm = m ? (unsigned long long)m * tm : 0ull;
-        unsigned long long vv = (m && b < nboot) ? (unsigned long long)m * tv : 0ull;
-        // low parts: signed, summed modulo 2^64 (the true sums fit in 63 bits)
-        unsigned long long lm = m ? (unsigned long long)((long long)m * tlm) : 0ull;
-        unsigned long long lv = (m && b < nboot) ? (unsigned long long)((long long)m * tlv) : 0ull;
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-          const unsigned long long um = __shfl_up_sync(0xffffffffu, vm, 1 << k);
-          const unsigned long long uv = __shfl_up_sync(0xffffffffu, vv, 1 << k);
-          const unsigned long long ulm = __shfl_up_sync(0xffffffffu, lm, 1 << k);
-          const unsigned long long ulv = __shfl_up_sync(0xffffffffu, lv, 1 << k);
-          if (same[k]) {
-            vm += um;
-            vv += uv;
-            lm += ulm;
-            lv += ulv;
-          }
-        }
-        if (ab && last) {
-          if (b == nboot) {
-            const int64_t o = (2 * npairs * G + cc) * 2;
-            if (vm) atomicAdd(&out[o], vm);
-            if (lm) atomicAdd(&out_lo[o], lm);
-          } else {
-            const int64_t om = ((2 * p) * G + cc) * 2 + half, ov = ((2 * p + 1) * G + cc) * 2 + half;
-            if (vm) atomicAdd(&out[om], vm);
-            if (vv) atomicAdd(&out[ov], vv);
-            if (lm) atomicAdd(&out_lo[om], lm);
-            if (lv) atomicAdd(&out_lo[ov], lv);
-          }
-        }
-      }
+      atomicAdd(&outM[b * G + cc], m);
+      if (qv && outV && b < nboot) atomicAdd(&outV[b * G + cc], qv[c * n + s]);
     }
   }
 }
@@ -453,53 +169,6 @@ __global__ void dequant_kernel(unsigned long long *v, int64_t m, double scale) {
   }
 }
 
-__global__ void dequant_paired_kernel(unsigned long long *v, int64_t G, int64_t npairs, double sm, double sv) {
-  // arrays: [z0, w0, z1, w1, ..., zF]; w arrays use sv
-  const int64_t total = (2 * npairs + 1) * G * 2;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t arr = i / (2 * G);
-    double sc = (arr < 2 * npairs && (arr & 1)) ? sv : sm;
-    unsigned long long x = v[i];
-    reinterpret_cast<double *>(v)[i] = (double)x * sc;
-  }
-}
-
-// The fixed-point exponents of a binning job from its largest count (misc[1]), on the
-// device so that phase B needs no read-back: a cell sums at most 2^N * cmax terms, each
-// <= tmax (means) or tmax^2 (second moments); e = 62 - the binary exponent of that bound.
-// esc[0] = e_m, esc[1] = e_v.  The same operations, in the same order, as on the host.
-__global__ void scale_exponents_kernel(const int *misc, double nc, double tmax, int *esc) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const double cmax = (double)(uint32_t)misc[1];
-  const double bm = __dmul_rn(__dmul_rn(nc, cmax > 1.0 ? cmax : 1.0), tmax);
-  const double bv = __dmul_rn(bm, tmax);
-  int ex_m, ex_v;
-  frexp(bm, &ex_m);
-  frexp(bv, &ex_v);
-  esc[0] = 62 - ex_m;
-  esc[1] = 62 - ex_v;
-  // low parts (|lo| <= 2^(L-1) a term) of at most nc * cmax terms a cell stay below 2^62
-  const unsigned long long terms = (unsigned long long)nc * (unsigned long long)(cmax > 1.0 ? cmax : 1.0);
-  const int lg = terms <= 1 ? 0 : 64 - __clzll((long long)(terms - 1));
-  esc[2] = 62 - lg;
-}
-
-// Conversion of the two-part fixed-point sums to FP64, in place: hi 2^-e + lo 2^-(e+L)
-// with the exponents from device memory (w arrays use e_v).
-__global__ void dequant_paired_esc_kernel(unsigned long long *v, const unsigned long long *lo, int64_t G,
-                                          int64_t npairs, const int *esc) {
-  const int L = esc[2];
-  const double sm = ldexp(1.0, -esc[0]), sv = ldexp(1.0, -esc[1]);
-  const int64_t total = (2 * npairs + 1) * G * 2;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t arr = i / (2 * G);
-    double sc = (arr < 2 * npairs && (arr & 1)) ? sv : sm;
-    const unsigned long long x = v[i];
-    const double xl = (double)(long long)lo[i];
-    reinterpret_cast<double *>(v)[i] = fma(ldexp(xl, -L), sc, (double)x * sc);
-  }
-}
-
 int grid_blocks(pkde_ctx *ctx, int64_t work) {
   int64_t b = (work + kThreads - 1) / kThreads;
   int64_t cap = (int64_t)ctx->sm_count * 16;
@@ -508,17 +177,15 @@ int grid_blocks(pkde_ctx *ctx, int64_t work) {
 
 }  // namespace
 
-// Shared driver.  d_data, d_idx are device pointers.  If `paired_out` is given, the
-// bootstrap means/squares are written as the paired complex layout used by the
-// estimator (z_p = M_2p + i M_2p+1, w_p = V_2p + i V_2p+1, zF = M_identity + 0i);
-// otherwise plain G x nboot FP64 arrays (and/or the identity when nboot == 0).
+// Shared driver.  d_data, d_idx are device pointers; plain G x nboot FP64 arrays (the identity
+// when nboot == 0).
 struct DiracScales {
   double sm, sv;
 };
 
 static DiracScales dirac_core(pkde_ctx *ctx, const pkde_grid *g, const double *d_data, int64_t n,
                               const int32_t *d_idx, int64_t nboot, bool with_identity, uint64_t seed,
-                              bool want_sq, double2 *paired_out, double *plain_m, double *plain_v,
+                              bool want_sq, double *plain_m, double *plain_v,
                               uint32_t *d_counts_out, cudaStream_t st) {
   grid_validate(g);
   if (n < 1 || n >= (int64_t(1) << 31)) throw invalid("number of samples must be in [1, 2^31)");
@@ -594,30 +261,15 @@ static DiracScales dirac_core(pkde_ctx *ctx, const pkde_grid *g, const double *d
   }
   PKDE_CHECK_LAUNCH();
   const double sm = std::ldexp(1.0, -e_m), sv = std::ldexp(1.0, -e_v);
-  if (paired_out) {
-    const int64_t npairs = (nboot + 1) / 2;
-    unsigned long long *acc = reinterpret_cast<unsigned long long *>(paired_out);
-    PKDE_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(double2) * (2 * npairs + 1) * G, st));
-    {
-      ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-      weight_kernel<true><<<grid_blocks(ctx, nslots * n), kThreads, 0, st>>>(
-          cell, n, nslots, nboot, G, N, corner_off, d_idx, seed, qm, want_sq ? qv : nullptr, acc, nullptr, npairs, err);
-    }
-    PKDE_CHECK_LAUNCH();
-    {
-      ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-      dequant_paired_kernel<<<grid_blocks(ctx, (2 * npairs + 1) * G * 2), kThreads, 0, st>>>(acc, G, npairs, sm, sv);
-    }
-    PKDE_CHECK_LAUNCH();
-  } else {
+  {
     unsigned long long *am = reinterpret_cast<unsigned long long *>(plain_m);
     unsigned long long *av = reinterpret_cast<unsigned long long *>(plain_v);
     PKDE_CUDA_TRY(cudaMemsetAsync(am, 0, sizeof(double) * nslots * G, st));
     if (av) PKDE_CUDA_TRY(cudaMemsetAsync(av, 0, sizeof(double) * nboot * G, st));
     {
       ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-      weight_kernel<false><<<grid_blocks(ctx, nslots * n), kThreads, 0, st>>>(
-          cell, n, nslots, nboot, G, N, corner_off, d_idx, seed, qm, (want_sq && av) ? qv : nullptr, am, av, 0, err);
+      weight_kernel<<<grid_blocks(ctx, nslots * n), kThreads, 0, st>>>(
+          cell, n, nslots, nboot, G, N, corner_off, d_idx, seed, qm, (want_sq && av) ? qv : nullptr, am, av, err);
     }
     PKDE_CHECK_LAUNCH();
     {
@@ -636,206 +288,6 @@ static DiracScales dirac_core(pkde_ctx *ctx, const pkde_grid *g, const double *d
   if (d_counts_out) PKDE_CUDA_TRY(cudaMemcpyAsync(d_counts_out, counts, sizeof(uint32_t) * nslots * G,
                                                   cudaMemcpyDeviceToDevice, st));
   return DiracScales{sm, sv};
-}
-
-// Estimator entry: paired spectra-ready layout (nboot resamples + identity), in two
-// phases around one host read-back of the error flags and the largest count, so that
-// the estimations of a batch share one synchronisation.
-size_t dirac_job_scratch(const pkde_grid *g, int64_t n, int64_t nboot) {
-  const int N = g->ndim;
-  const int64_t nc = int64_t(1) << N;
-  const int64_t G = grid_size(g);
-  const int64_t nchunk = (G + kScanChunk - 1) / kScanChunk;
-  auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-  const int64_t npairs = (nboot + 1) / 2;
-  return al(sizeof(uint32_t) * n) + al(sizeof(double) * N * n + sizeof(unsigned long long) * 4 * nc * n) +
-         al(sizeof(uint32_t) * (nboot + 1) * G) + 2 * al(sizeof(uint32_t) * n) + 2 * al(sizeof(uint32_t) * G) +
-         al(sizeof(uint32_t) * nchunk) + al(sizeof(uint32_t) * std::max<int64_t>(nboot, 1) * n) +
-         al(sizeof(double2) * (2 * npairs + 1) * G);
-}
-
-void dirac_job_bind(DiracJob &j, char *scratch, int *misc) {
-  const int N = j.g->ndim;
-  const int64_t nc = int64_t(1) << N;
-  const int64_t G = grid_size(j.g);
-  const int64_t nchunk = (G + kScanChunk - 1) / kScanChunk;
-  auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-  j.cell = (uint32_t *)scratch;
-  scratch += al(sizeof(uint32_t) * j.n);
-  j.rh = (double *)scratch;
-  j.qm_lo = reinterpret_cast<long long *>(j.rh + N * j.n) + 2 * nc * j.n;  // after the high parts
-  j.qv_lo = j.qm_lo + nc * j.n;
-  scratch += al(sizeof(double) * N * j.n + sizeof(unsigned long long) * 4 * nc * j.n);
-  j.counts = (uint32_t *)scratch;  // draws per lower cell and resample (slot nboot: identity)
-  scratch += al(sizeof(uint32_t) * (j.nboot + 1) * G);
-  j.pos = (uint32_t *)scratch;
-  scratch += al(sizeof(uint32_t) * j.n);
-  j.cell_sorted = (uint32_t *)scratch;
-  scratch += al(sizeof(uint32_t) * j.n);
-  j.cstart = (uint32_t *)scratch;
-  scratch += al(sizeof(uint32_t) * G);
-  j.cfill = (uint32_t *)scratch;
-  scratch += al(sizeof(uint32_t) * G);
-  j.csum = (uint32_t *)scratch;
-  scratch += al(sizeof(uint32_t) * nchunk);
-  j.mult = (uint32_t *)scratch;
-  scratch += al(sizeof(uint32_t) * std::max<int64_t>(j.nboot, 1) * j.n);
-  j.acc_lo = (unsigned long long *)scratch;
-  j.misc = misc;
-}
-
-// Phase A: bounds check and cell pre-pass, exact counts, largest count (misc[0] error
-// bits, misc[1] max count).  Nothing is read back here.
-void dirac_job_phase_a(pkde_ctx *ctx, DiracJob &j, cudaStream_t st) {
-  const pkde_grid *g = j.g;
-  grid_validate(g);
-  const int64_t n = j.n;
-  if (n < 1 || n >= (int64_t(1) << 31)) throw invalid("number of samples must be in [1, 2^31)");
-  GridDev gd = to_dev(g);
-  const int64_t G = grid_size(g);
-  const int N = g->ndim;
-  const int nc = 1 << N;
-  const int64_t nslots = j.nboot + 1;
-  int *misc = j.misc;
-  unsigned int *maxc = reinterpret_cast<unsigned int *>(misc + 1);
-  int64_t *corner_off = reinterpret_cast<int64_t *>(misc + 8);  // 16 entries
-  for (int c = 0; c < nc; ++c) {
-    int64_t o = 0;
-    for (int q = 0; q < N; ++q)
-      if (!((c >> (N - 1 - q)) & 1)) o += gd.stride[q];
-    j.corner_off_h[c] = o;
-  }
-  PKDE_CUDA_TRY(cudaMemsetAsync(misc, 0, 64, st));
-  PKDE_CUDA_TRY(cudaMemcpyAsync(corner_off, j.corner_off_h, sizeof(int64_t) * nc, cudaMemcpyHostToDevice, st));
-  PKDE_CUDA_TRY(cudaMemsetAsync(j.counts, 0, sizeof(uint32_t) * nslots * G, st));
-  {
-    ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-    prepass_kernel<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, st>>>(gd, j.d_data, n, j.cell, j.rh,
-                                                                                    misc);
-  }
-  PKDE_CHECK_LAUNCH();
-  {
-    // samples per lower cell (the identity slot); the resamples' counts are summed from
-    // their multiplicities once the samples are in cell order
-    ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-    count_kernel<<<grid_blocks(ctx, n), kThreads, 0, st>>>(j.cell, n, 1, 0, G, nullptr, 0, j.counts + j.nboot * G,
-                                                          misc);
-  }
-  PKDE_CHECK_LAUNCH();
-  // samples in lower-cell order (counting sort from the identity counts), then each
-  // resample's draws as per-sample multiplicities in that order
-  const uint32_t *idc = j.counts + j.nboot * G;
-  const int64_t nchunk = (G + kScanChunk - 1) / kScanChunk;
-  {
-    ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-    cell_chunk_sum_kernel<<<(unsigned)nchunk, kThreads, 0, st>>>(idc, G, j.csum);
-  }
-  PKDE_CHECK_LAUNCH();
-  {
-    ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-    chunk_scan_kernel<<<1, 32, 0, st>>>(j.csum, nchunk);
-  }
-  PKDE_CHECK_LAUNCH();
-  {
-    ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-    cell_start_kernel<<<(unsigned)nchunk, kThreads, 0, st>>>(idc, G, j.csum, j.cstart, j.cfill);
-  }
-  PKDE_CHECK_LAUNCH();
-  {
-    ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-    cell_sort_kernel<<<grid_blocks(ctx, n), kThreads, 0, st>>>(j.cell, n, j.cstart, j.cfill, j.pos, j.cell_sorted);
-  }
-  PKDE_CHECK_LAUNCH();
-  if (j.nboot > 0) {
-    PKDE_CUDA_TRY(cudaMemsetAsync(j.mult, 0, sizeof(uint32_t) * j.nboot * n, st));
-    {
-      ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-      mult_kernel<<<grid_blocks(ctx, j.nboot * n), kThreads, 0, st>>>(n, j.nboot, j.d_idx, j.seed, j.pos, j.mult,
-                                                                     misc);
-    }
-    PKDE_CHECK_LAUNCH();
-  }
-  if (j.nboot > 0) {
-    ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-    resample_count_kernel<<<grid_blocks(ctx, j.nboot * n), kThreads, 0, st>>>(j.cell_sorted, n, j.nboot, G, j.mult,
-                                                                              j.counts);
-  }
-  PKDE_CHECK_LAUNCH();
-  {
-    ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-    max_kernel<<<grid_blocks(ctx, nslots * G), kThreads, 0, st>>>(j.counts, nslots * G, maxc);
-  }
-  PKDE_CHECK_LAUNCH();
-}
-
-// Phase B, given misc[0..1] read back: error check, fixed-point scales, quantised
-// corner terms, scatter into the paired spectra slots, conversion to FP64.
-void binning_flags_check(const int *hmisc) {
-  if (hmisc[0] & 1) throw invalid("Data points lie beyond grid. Remove them or increase grid boundaries.");
-  if (hmisc[0] & 2)
-    throw invalid("Data points lie within one rounding of the upper grid bound. Remove them or increase grid boundaries.");
-  if (hmisc[0] & 4) throw invalid("Bootstrap indices must lie in 1:n_samples.");
-}
-
-void dirac_job_phase_b(pkde_ctx *ctx, DiracJob &j, const int *hmisc, cudaStream_t st) {
-  const pkde_grid *g = j.g;
-  if (hmisc) binning_flags_check(hmisc);
-  GridDev gd = to_dev(g);
-  const int64_t G = grid_size(g);
-  const int N = g->ndim;
-  const int nc = 1 << N;
-  const int64_t n = j.n;
-  const int64_t nboot = j.nboot;
-  const int64_t nslots = nboot + 1;
-  unsigned long long *qm = reinterpret_cast<unsigned long long *>(j.rh + N * n);
-  unsigned long long *qv = qm + (int64_t)nc * n;
-  const int64_t *corner_off = reinterpret_cast<const int64_t *>(j.misc + 8);
-  int *esc = j.misc + 48;
-  // term <= prod(h) / (n prod(h)^2); a cell sums at most 2^N * cmax terms.
-  double sp = g->h[0];
-  for (int q = 1; q < N; ++q) sp = sp * g->h[q];
-  const double denom = (double)n * (sp * sp);
-  const double tmax = (1.0 / ((double)n * sp)) * (1.0 + 1e-12);
-  {
-    ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-    scale_exponents_kernel<<<1, 32, 0, st>>>(j.misc, (double)nc, tmax, esc);
-  }
-  PKDE_CHECK_LAUNCH();
-  {
-    ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-    quantize_sorted_kernel<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, st>>>(gd, j.rh, n, denom, esc,
-                                                                                            j.pos, qm, qv, j.qm_lo,
-                                                                                            j.qv_lo);
-  }
-  PKDE_CHECK_LAUNCH();
-  const int64_t npairs = (nboot + 1) / 2;
-  unsigned long long *acc = reinterpret_cast<unsigned long long *>(j.paired_out);
-  PKDE_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(double2) * (2 * npairs + 1) * G, st));
-  PKDE_CUDA_TRY(cudaMemsetAsync(j.acc_lo, 0, sizeof(double2) * (2 * npairs + 1) * G, st));
-  {
-    ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-    // resamples in chunks of at most 16, as even as possible (65 = 5 x 13, 33 = 3 x 11)
-    const int64_t nchunk = (nslots + 15) / 16;
-    const int BC = (int)((nslots + nchunk - 1) / nchunk);
-    const int blocks = grid_blocks(ctx, nchunk * n);
-#define PKDE_WS(NN)                                                                                          \
-  weight_sorted_kernel<NN><<<blocks, kThreads, 0, st>>>(j.cell_sorted, n, nboot, G, corner_off, j.mult, qm, qv,   \
-                                                        j.qm_lo, j.qv_lo, acc, j.acc_lo, npairs, BC, nchunk)
-    switch (N) {
-      case 1: PKDE_WS(1); break;
-      case 2: PKDE_WS(2); break;
-      case 3: PKDE_WS(3); break;
-      default: PKDE_WS(4); break;
-    }
-#undef PKDE_WS
-  }
-  PKDE_CHECK_LAUNCH();
-  {
-    ::pkde::Trace _tr(ctx, PKDE_PHASE_BINNING, st);
-    dequant_paired_esc_kernel<<<grid_blocks(ctx, (2 * npairs + 1) * G * 2), kThreads, 0, st>>>(acc, j.acc_lo, G,
-                                                                                                npairs, esc);
-  }
-  PKDE_CHECK_LAUNCH();
 }
 
 }  // namespace pkde
@@ -869,7 +321,7 @@ extern "C" int pkde_dirac_sequence(pkde_ctx *ctx, const pkde_grid *grid, const d
     double *om = (double *)ensure(ctx, BUF_OUT, sizeof(double) * (2 * nslots * G) + sizeof(uint32_t) * nslots * G);
     double *ov = om + nslots * G;
     uint32_t *oc = reinterpret_cast<uint32_t *>(ov + nslots * G);
-    dirac_core(ctx, grid, d_data, n, d_idx, nb, identity, seed, sq_out != nullptr && !identity, nullptr, om,
+    dirac_core(ctx, grid, d_data, n, d_idx, nb, identity, seed, sq_out != nullptr && !identity, om,
                (sq_out && !identity) ? ov : nullptr, oc, st);
     if (means_out) copy_out(means_out, om, sizeof(double) * nslots * G, dout, st);
     if (sq_out && !identity) copy_out(sq_out, ov, sizeof(double) * nslots * G, dout, st);
@@ -1033,8 +485,8 @@ extern "C" int pkde_dirac_sequence_noalloc(pkde_ctx *ctx, const pkde_grid *grid,
     unsigned long long *av = want_sq ? reinterpret_cast<unsigned long long *>(sq_out) : nullptr;
     PKDE_CUDA_TRY(cudaMemsetAsync(am, 0, sizeof(double) * nslots * G, st));
     if (av) PKDE_CUDA_TRY(cudaMemsetAsync(av, 0, sizeof(double) * nb * G, st));
-    weight_kernel<false><<<noalloc_blocks(sms, nslots * n), kThreads, 0, st>>>(
-        cell, n, nslots, nb, G, N, corner_off, boot_idx, seed, qm, av ? qv : nullptr, am, av, 0, err);
+    weight_kernel<<<noalloc_blocks(sms, nslots * n), kThreads, 0, st>>>(
+        cell, n, nslots, nb, G, N, corner_off, boot_idx, seed, qm, av ? qv : nullptr, am, av, err);
     PKDE_CHECK_LAUNCH();
     dequant_kernel<<<noalloc_blocks(sms, nslots * G), kThreads, 0, st>>>(am, nslots * G,
                                                                                        std::ldexp(1.0, -e_m));

@@ -17,6 +17,7 @@
 #include <cstring>
 
 #include "pkde_chunk.cuh"
+#include "pkde_jobs.cuh"
 
 namespace pkde {
 namespace {
@@ -47,31 +48,6 @@ __device__ __forceinline__ double2 lds(unsigned a) {
 }
 __device__ __forceinline__ void sts(unsigned a, double2 v) {
   asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
-}
-
-// The job of this block: of several (job array and first blocks in device memory) copied into
-// shared memory, of one the kernel's own parameter.
-template <class J>
-__device__ __forceinline__ void find_job(const J *jobs, const unsigned *block0, int count, J &sj, unsigned &first) {
-  __shared__ int s_job;
-  if (threadIdx.x < 32) {
-    int job = 0;
-    for (;;) {  // block0 increases: the lanes at or below this block form a prefix
-      const int k = job + 1 + (int)threadIdx.x;
-      const bool le = k < count && __ldg(block0 + k) <= blockIdx.x;
-      const int c = __popc(__ballot_sync(0xffffffffu, le));
-      job += c;
-      if (c < 32) break;
-    }
-    if (threadIdx.x == 0) s_job = job;
-  }
-  __syncthreads();
-  const int job = s_job;
-  const int *src = reinterpret_cast<const int *>(jobs + job);
-  int *dst = reinterpret_cast<int *>(&sj);
-  for (int i = threadIdx.x; i < (int)(sizeof(J) / sizeof(int)); i += blockDim.x) dst[i] = __ldg(src + i);
-  first = __ldg(block0 + job);
-  __syncthreads();
 }
 
 // Where a tile's lines come from and go to, as byte offsets of 32 bits from a base that is the

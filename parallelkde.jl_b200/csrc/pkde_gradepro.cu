@@ -215,7 +215,8 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
 
 // Sums over the samples of one estimation per blockIdx.y: per axis, of x (mean ==
 // nullptr) or of (x - mean)^2.  Each of the job's nb blocks writes its partial sums
-// (fixed tree order); moments_final_kernel adds a job's partials in order.  The
+// (fixed tree order); the job's last block adds the partials in order, read through shared
+// memory (one thread that reads them itself, 1184 dependent loads: 87 us; 8 so).  The
 // partition depends only on the job's own n, so an estimation gets the same sums alone
 // and in a batch.
 struct MomentJob {
@@ -225,39 +226,54 @@ struct MomentJob {
   int nb;
   double *partial;     // nb x ndim
   const double *mean;  // ndim, or nullptr
-  double *out;         // ndim
+  double *out;         // ndim: the means (sum / n, one correctly rounded division), or the squared deviations
+  unsigned done;       // blocks that have written their partials
 };
 
-__global__ void moments_partial_kernel(const MomentJob *jobs) {
+__global__ void __launch_bounds__(kThreads) moments_kernel(MomentJob *jobs) {
   __shared__ double sh[32];
+  __shared__ double part[kThreads][4];
+  __shared__ bool last;
   const MomentJob J = jobs[blockIdx.y];
   if ((int)blockIdx.x >= J.nb) return;  // uniform over the block
-  for (int j = 0; j < J.ndim; ++j) {
-    const double mu = J.mean ? J.mean[j] : 0.0;
-    double s = 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < J.n; i += (int64_t)J.nb * blockDim.x) {
-      const double x = J.data[i * J.ndim + j];
-      s += J.mean ? (x - mu) * (x - mu) : x;
+  double mu[4], s[4];
+  for (int j = 0; j < 4; ++j) {
+    mu[j] = J.mean && j < J.ndim ? J.mean[j] : 0.0;
+    s[j] = 0.0;
+  }
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < J.n; i += (int64_t)J.nb * blockDim.x) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (j < J.ndim) {
+        const double x = J.data[i * J.ndim + j];
+        s[j] += J.mean ? (x - mu[j]) * (x - mu[j]) : x;
+      }
     }
-    const double t = block_sum(s, sh);
-    if (threadIdx.x == 0) J.partial[blockIdx.x * J.ndim + j] = t;
   }
-}
-
-__global__ void moments_final_kernel(const MomentJob *jobs) {
-  const MomentJob J = jobs[blockIdx.x];
-  if ((int)threadIdx.x < J.ndim) {
-    double s = 0.0;
-    for (int b = 0; b < J.nb; ++b) s += J.partial[b * J.ndim + threadIdx.x];
-    J.out[threadIdx.x] = s;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (j < J.ndim) {
+      const double t = block_sum(s[j], sh);
+      if (threadIdx.x == 0) J.partial[blockIdx.x * J.ndim + j] = t;
+    }
   }
-}
-
-// The means of the first pass, sum / n with one correctly rounded division per axis (the
-// same value the host's division gives), written where the second pass's jobs read them.
-__global__ void moments_mean_kernel(const MomentJob *jobs, double *means) {
-  const MomentJob J = jobs[blockIdx.x];
-  if ((int)threadIdx.x < J.ndim) means[4 * blockIdx.x + threadIdx.x] = __ddiv_rn(J.out[threadIdx.x], (double)J.n);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&jobs[blockIdx.y].done, 1u) == (unsigned)J.nb - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  double t = 0.0;
+  for (int b0 = 0; b0 < J.nb; b0 += kThreads) {
+    const int nb = min(kThreads, J.nb - b0);
+    for (int k = threadIdx.x; k < nb * J.ndim; k += kThreads)
+      part[k / J.ndim][k % J.ndim] = __ldcg(J.partial + (int64_t)b0 * J.ndim + k);
+    __syncthreads();
+    if ((int)threadIdx.x < J.ndim)
+      for (int b = 0; b < nb; ++b) t += part[b][threadIdx.x];
+    __syncthreads();
+  }
+  if ((int)threadIdx.x < J.ndim) J.out[threadIdx.x] = J.mean ? t : __ddiv_rn(t, (double)J.n);
 }
 
 int blocks_for(pkde_ctx *ctx, int64_t work) {
@@ -358,24 +374,39 @@ Ladder make_ladder(const pkde_gradepro_params *p, const double *bw_final, int64_
   return L;
 }
 
+// Page-locked staging buffer of the context (grow-only), for asynchronous uploads.
+static void *pinned_staging(pkde_ctx *ctx, size_t bytes) {
+  if (bytes > ctx->pinned_bytes) {
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    ctx->pinned = nullptr;
+    ctx->pinned_bytes = 0;
+    PKDE_CUDA_TRY(cudaMallocHost(&ctx->pinned, bytes));
+    ctx->pinned_bytes = bytes;
+  }
+  return ctx->pinned;
+}
+
 // Per-axis sums of squared deviations from the mean, sum_i (x_ji - mean_j)^2, of several
-// sample sets at once (FP64, deterministic): a reduction for the sums, the means on the
-// device, a reduction for the squared deviations, and one read-back for the whole set.
+// sample sets at once (FP64, deterministic): a reduction for the means, one for the squared
+// deviations, and one read-back for the whole set (it ends with a synchronisation).
 // data[e] is N[e] x n[e]; the result goes to centered[4e .. 4e+N[e]-1].
 void sample_centered_sums(pkde_ctx *ctx, int count, const double *const *data, const int64_t *n, const int *N,
                           double *centered, cudaStream_t st) {
   if (count < 1) return;
-  // jobs[0..count): the sums; jobs[count..2 count): the squared deviations from the means
-  std::vector<MomentJob> jobs(2 * (size_t)count);
+  // page-locked: jobs[0..count) the means, jobs[count..2 count) the squared deviations; the results
+  const size_t jb = (sizeof(MomentJob) * 2 * count + 255) & ~size_t(255);
+  char *hp = (char *)pinned_staging(ctx, jb + sizeof(double) * 4 * (size_t)count);
+  MomentJob *jobs = (MomentJob *)hp;
+  double *h = (double *)(hp + jb);
   int maxnb = 1;
   size_t npart = 0;
   for (int e = 0; e < count; ++e) {
+    jobs[e] = MomentJob{};
     jobs[e].nb = blocks_for(ctx, n[e]);
     maxnb = std::max(maxnb, jobs[e].nb);
     npart += 4 * (size_t)jobs[e].nb;
   }
-  // device: [jobs][sums count x 4][means count x 4][partials]
-  const size_t jb = (sizeof(MomentJob) * 2 * count + 255) & ~size_t(255);
+  // device: [jobs][squared deviations count x 4][means count x 4][partials]
   char *m = (char *)ensure(ctx, BUF_MISC, jb + sizeof(double) * (8 * (size_t)count + npart));
   MomentJob *djobs = (MomentJob *)m;
   double *sums = (double *)(m + jb), *means = sums + 4 * count, *partial = means + 4 * count;
@@ -386,33 +417,22 @@ void sample_centered_sums(pkde_ctx *ctx, int count, const double *const *data, c
     jobs[e].partial = partial;
     partial += 4 * (size_t)jobs[e].nb;
     jobs[e].mean = nullptr;
-    jobs[e].out = sums + 4 * e;
+    jobs[e].out = means + 4 * e;
     jobs[count + e] = jobs[e];
     jobs[count + e].mean = means + 4 * e;
+    jobs[count + e].out = sums + 4 * e;
   }
-  PKDE_CUDA_TRY(cudaMemcpyAsync(djobs, jobs.data(), sizeof(MomentJob) * 2 * count, cudaMemcpyHostToDevice, st));
+  PKDE_CUDA_TRY(cudaMemcpyAsync(djobs, jobs, sizeof(MomentJob) * 2 * count, cudaMemcpyHostToDevice, st));
   for (int pass = 0; pass < 2; ++pass) {
-    const MomentJob *pj = djobs + (size_t)pass * count;
     {
       ::pkde::Trace _tr(ctx, PKDE_PHASE_OTHER, st);
-      moments_partial_kernel<<<dim3((unsigned)maxnb, (unsigned)count), kThreads, 0, st>>>(pj);
+      moments_kernel<<<dim3((unsigned)maxnb, (unsigned)count), kThreads, 0, st>>>(djobs + (size_t)pass * count);
     }
     PKDE_CHECK_LAUNCH();
-    {
-      ::pkde::Trace _tr(ctx, PKDE_PHASE_OTHER, st);
-      moments_final_kernel<<<(unsigned)count, 32, 0, st>>>(pj);
-    }
-    PKDE_CHECK_LAUNCH();
-    if (pass == 0) {
-      ::pkde::Trace _tr(ctx, PKDE_PHASE_OTHER, st);
-      moments_mean_kernel<<<(unsigned)count, 32, 0, st>>>(pj, means);
-    }
-    if (pass == 0) PKDE_CHECK_LAUNCH();
   }
-  std::vector<double> h(4 * (size_t)count);
-  PKDE_CUDA_TRY(cudaMemcpyAsync(h.data(), sums, sizeof(double) * 4 * count, cudaMemcpyDeviceToHost, st));
+  PKDE_CUDA_TRY(cudaMemcpyAsync(h, sums, sizeof(double) * 4 * count, cudaMemcpyDeviceToHost, st));
   PKDE_CUDA_TRY(cudaStreamSynchronize(st));
-  std::memcpy(centered, h.data(), sizeof(double) * 4 * count);
+  std::memcpy(centered, h, sizeof(double) * 4 * count);
 }
 
 namespace {
@@ -529,18 +549,6 @@ static size_t shared_budget(pkde_ctx *ctx, BufId id) {
   if (const char *cap = getenv("PKDE_RING_BUDGET_MB"); cap && *cap)
     budget = std::min(budget, (size_t)std::max(0LL, atoll(cap)) << 20);
   return budget;
-}
-
-// Page-locked staging buffer of the context (grow-only), for asynchronous uploads.
-static void *pinned_staging(pkde_ctx *ctx, size_t bytes) {
-  if (bytes > ctx->pinned_bytes) {
-    if (ctx->pinned) cudaFreeHost(ctx->pinned);
-    ctx->pinned = nullptr;
-    ctx->pinned_bytes = 0;
-    PKDE_CUDA_TRY(cudaMallocHost(&ctx->pinned, bytes));
-    ctx->pinned_bytes = bytes;
-  }
-  return ctx->pinned;
 }
 
 // One estimation of a call (device pointers).
@@ -751,7 +759,9 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   std::vector<double> sbw(4 * sd.size());
   silverman_batch(ctx, (int)sd.size(), sd.data(), sn.data(), sN.data(), sbw.data(), st);
   // ---- ladders, factor tables, paths
-  size_t arena = al256(256 * (size_t)count);  // misc blocks first (one read-back)
+  // memory that starts at zero first (one fill): misc blocks (one read-back), then spectra, low
+  // parts, counts and multiplicities of every estimation
+  size_t arena = al256(256 * (size_t)count);
   size_t tables_bytes = 0;
   size_t generic_wel = 0, generic_scr = 0, chunk_scr = 0;
   std::vector<int> chunk_e;           // estimations that run in chunks of steps, their scratch
@@ -776,7 +786,13 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     if (ctx->step_path == PKDE_STEPS_PER_STEP_LAUNCH) P.path = StepPath::Generic;
     tables_bytes += al256(sizeof(double) * 2 * P.L.S * P.tot);
   }
-  // arena: [misc blocks][tables of every estimation][per estimation: spectra, state,
+  std::vector<size_t> off_zero(count);
+  for (int e = 0; e < count; ++e) {
+    off_zero[e] = arena;
+    arena += dirac_zero_bytes(plans[e].g, ests[e].n, plans[e].B);
+  }
+  const size_t zero_bytes = arena;
+  // arena: [zero][tables of every estimation][job descriptors][per estimation: state,
   // 1-D per-step arrays, binning scratch]
   const size_t off_tables = arena;
   arena += tables_bytes;
@@ -790,16 +806,17 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   const size_t tjob_bytes = al256(sizeof(TableJob) * count) + al256(sizeof(double) * times_doubles);
   const size_t off_tjobs = arena;
   arena += tjob_bytes;
+  const size_t off_bjobs = arena;
+  arena += al256(binning_desc_bytes(count));
   const size_t off_rjobs = arena;
   arena += al256(steps1d_job_bytes() * n1d);
   for (int e = 0; e < count; ++e) {
     Plan &P = plans[e];
     off[e] = arena;
-    arena += al256(sizeof(double2) * (2 * P.npairs + 1) * P.G);
     arena += state_bytes(P.G);
     if (P.path == StepPath::Steps1D)
       arena += al256(sizeof(double) * 2 * P.L.S * P.G) + al256(steps1d_state_bytes((int)P.G, (int)P.npairs, P.L.S));
-    arena += dirac_job_scratch(P.g, ests[e].n, P.B);
+    arena += dirac_job_scratch(P.g, ests[e].n);
     if (P.path == StepPath::Chunk) {
       chunk_e.push_back(e);
       chunk_bytes.push_back(0);
@@ -862,8 +879,6 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     toffs[e] = toff;
     toff += al256(sizeof(double) * 2 * S * P.tot);
     char *q = base + off[e];
-    P.spectra = (double2 *)q;
-    q += al256(sizeof(double2) * (2 * P.npairs + 1) * P.G);
     P.cs = bind_state(q, P.G);
     q += state_bytes(P.G);
     P.per_step = nullptr;
@@ -880,15 +895,21 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     P.job.d_idx = ests[e].d_idx;
     P.job.nboot = P.B;
     P.job.seed = ests[e].seed;
-    P.job.paired_out = P.spectra;
-    dirac_job_bind(P.job, P.bin_scratch, P.misc);
+    dirac_job_bind(P.job, base + off_zero[e], P.bin_scratch, P.misc);
+    P.spectra = P.job.paired_out;
   }
-  // ---- binning: phase A for all (queued first, so that the host work below overlaps it)
-  for (int e = 0; e < count; ++e) dirac_job_phase_a(ctx, plans[e].job, st);
-  // ---- propagation factor tables, on the device: the ladders' times and the job
-  // descriptors go up in one copy from page-locked memory, one kernel fills every table
-  char *hp = (char *)pinned_staging(ctx, al256(tjob_bytes) + 256 * (size_t)count + al256(steps1d_job_bytes() * n1d));
-  if (tables_bytes) {
+  PKDE_CUDA_TRY(cudaMemsetAsync(base, 0, zero_bytes, st));
+  // ---- job descriptors (factor tables, binning, 1-D steps) and the ladders' times: one copy from
+  // page-locked memory
+  const size_t desc_bytes = off_rjobs + al256(steps1d_job_bytes() * n1d) - off_tjobs;
+  char *hp = (char *)pinned_staging(ctx, desc_bytes + 256 * (size_t)count);
+  std::vector<DiracJob> bins;
+  for (int e = 0; e < count; ++e) bins.push_back(plans[e].job);
+  BinningPlan bplan;
+  binning_describe(bins.data(), count, hp + (off_bjobs - off_tjobs), bplan);
+  std::vector<Steps1dArgs> line;
+  Steps1dPlan lplan;
+  {
     TableJob *hj = (TableJob *)hp;
     double *ht = (double *)(hp + al256(sizeof(TableJob) * count));
     const double *dt = (const double *)(base + off_tjobs + al256(sizeof(TableJob) * count));
@@ -918,36 +939,10 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
       }
       maxtotal = std::max<int64_t>(maxtotal, P.L.S * P.tot);
     }
-    PKDE_CUDA_TRY(cudaMemcpyAsync(base + off_tjobs, hp, tjob_bytes, cudaMemcpyHostToDevice, st));
-    {
-      ::pkde::Trace _tr(ctx, PKDE_PHASE_OTHER, st);
-      const unsigned bx = (unsigned)std::min<int64_t>((maxtotal + kThreads - 1) / kThreads, (int64_t)ctx->sm_count * 4);
-      factor_table_kernel<<<dim3(bx, (unsigned)count), kThreads, 0, st>>>((const TableJob *)(base + off_tjobs));
-    }
-    PKDE_CHECK_LAUNCH();
-  }
-  // the binning error flags come back with the call's final synchronisation (invalid data
-  // is reported then; what runs on it meanwhile stays in bounds: such samples bin to cell 0)
-  int *hflags = (int *)(hp + al256(tjob_bytes));
-  PKDE_CUDA_TRY(cudaMemcpyAsync(hflags, base, 256 * (size_t)count, cudaMemcpyDeviceToHost, st));
-  ctx->bin_flags = hflags;
-  ctx->bin_flags_count = count;
-  for (int e = 0; e < count; ++e) dirac_job_phase_b(ctx, plans[e].job, nullptr, st);
-  fault_point(ctx, PKDE_FAULT_AFTER_BINNING);
-  // ---- forward FFT of every array
-  for (int e = 0; e < count; ++e)
-    fft_nd(ctx, plans[e].N, plans[e].g->dims, plans[e].spectra, 2 * plans[e].npairs + 1, -1, st,
-           PKDE_PHASE_FORWARD_FFT);
-  // ---- bandwidth steps
-  std::vector<EngineArgs> eng;
-  std::vector<Steps1dArgs> line;
-  std::vector<ChunkArgs> chunk;
-  for (int e = 0; e < count; ++e) {
-    Plan &P = plans[e];
-    const Ladder &L = P.L;
-    const int64_t S = L.S;
-    const double *dfz = P.tables, *dfw = P.tables + S * P.tot;
-    if (P.path == StepPath::Steps1D) {
+    for (int e = 0; e < count; ++e) {
+      Plan &P = plans[e];
+      if (P.path != StepPath::Steps1D) continue;
+      const int64_t S = P.L.S;
       Steps1dArgs A{};
       A.n1 = (int)P.G;
       A.npairs = (int)P.npairs;
@@ -956,8 +951,8 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
       A.fused = P.G >= 256 && (P.G & (P.G - 1)) == 0;
       A.n = ests[e].n;
       A.spectra = P.spectra;
-      A.fz = dfz;
-      A.fw = dfw;
+      A.fz = P.tables;
+      A.fw = P.tables + S * P.tot;
       A.tab_stride = P.tot;
       A.cw = P.d_scal;
       A.vscale = P.d_scal + S;
@@ -965,8 +960,37 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
       A.mu_out = P.per_step + S * P.G;
       A.state = P.state1d;
       line.push_back(A);
-      continue;
     }
+    steps1d_describe(ctx, line.data(), (int)line.size(), hp + (off_rjobs - off_tjobs), lplan);
+    PKDE_CUDA_TRY(cudaMemcpyAsync(base + off_tjobs, hp, desc_bytes, cudaMemcpyHostToDevice, st));
+    {
+      ::pkde::Trace _tr(ctx, PKDE_PHASE_OTHER, st);
+      const unsigned bx = (unsigned)std::min<int64_t>((maxtotal + kThreads - 1) / kThreads, (int64_t)ctx->sm_count * 4);
+      factor_table_kernel<<<dim3(bx, (unsigned)count), kThreads, 0, st>>>((const TableJob *)(base + off_tjobs));
+    }
+    PKDE_CHECK_LAUNCH();
+  }
+  binning_run(ctx, bplan, base + off_bjobs, st);
+  // the binning error flags come back with the call's final synchronisation (invalid data
+  // is reported then; what runs on it meanwhile stays in bounds: such samples bin to cell 0)
+  int *hflags = (int *)(hp + desc_bytes);
+  PKDE_CUDA_TRY(cudaMemcpyAsync(hflags, base, 256 * (size_t)count, cudaMemcpyDeviceToHost, st));
+  ctx->bin_flags = hflags;
+  ctx->bin_flags_count = count;
+  fault_point(ctx, PKDE_FAULT_AFTER_BINNING);
+  // ---- forward FFT of every array
+  for (int e = 0; e < count; ++e)
+    fft_nd(ctx, plans[e].N, plans[e].g->dims, plans[e].spectra, 2 * plans[e].npairs + 1, -1, st,
+           PKDE_PHASE_FORWARD_FFT);
+  // ---- bandwidth steps
+  std::vector<EngineArgs> eng;
+  std::vector<ChunkArgs> chunk;
+  for (int e = 0; e < count; ++e) {
+    Plan &P = plans[e];
+    const Ladder &L = P.L;
+    const int64_t S = L.S;
+    const double *dfz = P.tables, *dfw = P.tables + S * P.tot;
+    if (P.path == StepPath::Steps1D) continue;
     auto init_state = [&] {
       {
         ::pkde::Trace _tr(ctx, PKDE_PHASE_OTHER, st);
@@ -1038,7 +1062,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   }
   // 1-D estimations: every bandwidth step of all of them in one launch, then the
   // convergence state machine over the stored per-step f_s and means
-  steps1d(ctx, line.data(), (int)line.size(), hp + al256(tjob_bytes) + 256 * (size_t)count, base + off_rjobs, st);
+  steps1d_run(ctx, lplan, base + off_rjobs, st);
   for (int e = 0; e < count; ++e) {
     Plan &P = plans[e];
     if (P.path != StepPath::Steps1D) continue;
@@ -1139,25 +1163,32 @@ void run_rot(pkde_ctx *ctx, const pkde_grid *g, int rule, const double *d_data, 
   std::vector<int64_t> aoff;
   factor_tables(g, L, fz, fw, aoff);
   const int64_t tot = aoff[N];
-  // device: [misc block][factor tables][spectrum][binning scratch]
-  const size_t off_tab = 256, off_spec = off_tab + al256(sizeof(double) * tot),
-               off_scr = off_spec + al256(sizeof(double2) * G);
-  char *base = (char *)ensure(ctx, BUF_BATCH, off_scr + dirac_job_scratch(g, n, 0));
-  double *tables = (double *)(base + off_tab);
-  double2 *spec = (double2 *)(base + off_spec);
-  PKDE_CUDA_TRY(cudaMemcpyAsync(tables, fz.data(), sizeof(double) * tot, cudaMemcpyHostToDevice, st));
+  // device: [zero: misc block, spectrum, ...][job descriptor][factor tables][binning scratch]
+  const size_t zero_bytes = 256 + dirac_zero_bytes(g, n, 0), desc_bytes = al256(binning_desc_bytes(1)),
+               tab_bytes = al256(sizeof(double) * tot);
+  char *base = (char *)ensure(ctx, BUF_BATCH, zero_bytes + desc_bytes + tab_bytes + dirac_job_scratch(g, n));
+  char *desc = base + zero_bytes;
+  double *tables = (double *)(desc + desc_bytes);
   DiracJob j;
   j.g = g;
   j.d_data = d_data;
   j.n = n;
   j.nboot = 0;
-  j.paired_out = spec;
-  dirac_job_bind(j, base + off_scr, (int *)base);
-  dirac_job_phase_a(ctx, j, st);
-  int h[64];
-  PKDE_CUDA_TRY(cudaMemcpyAsync(h, base, 256, cudaMemcpyDeviceToHost, st));
-  PKDE_CUDA_TRY(cudaStreamSynchronize(st));
-  dirac_job_phase_b(ctx, j, h, st);
+  dirac_job_bind(j, base + 256, (char *)tables + tab_bytes, (int *)base);
+  double2 *spec = j.paired_out;
+  // page-locked: [job descriptor][factor tables][error flags]
+  char *hp = (char *)pinned_staging(ctx, desc_bytes + tab_bytes + 256);
+  BinningPlan plan;
+  binning_describe(&j, 1, hp, plan);
+  std::memcpy(hp + desc_bytes, fz.data(), sizeof(double) * tot);
+  PKDE_CUDA_TRY(cudaMemsetAsync(base, 0, zero_bytes, st));
+  PKDE_CUDA_TRY(cudaMemcpyAsync(desc, hp, desc_bytes + tab_bytes, cudaMemcpyHostToDevice, st));
+  binning_run(ctx, plan, desc, st);
+  // invalid data is reported after the call's final synchronisation
+  int *flags = (int *)(hp + desc_bytes + tab_bytes);
+  PKDE_CUDA_TRY(cudaMemcpyAsync(flags, base, 256, cudaMemcpyDeviceToHost, st));
+  ctx->bin_flags = flags;
+  ctx->bin_flags_count = 1;
   fft_nd(ctx, N, g->dims, spec, 1, -1, st, PKDE_PHASE_FORWARD_FFT);
   for (int a = 0; a < N; ++a) {
     LineSet ls = axis_lines(N, g->dims, a, 1);
@@ -1289,6 +1320,7 @@ int pkde_rot_estimate(pkde_ctx *ctx, const pkde_grid *grid, int32_t rule, const 
     if (!dout) copy_out(density_out, dens, sizeof(double) * G, false, st);
     PKDE_CUDA_TRY(cudaStreamSynchronize(st));
     collect_trace(ctx);
+    check_binning_flags(ctx);
   });
 }
 

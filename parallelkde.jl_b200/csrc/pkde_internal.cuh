@@ -553,8 +553,7 @@ void copy_out(void *dst, const void *src, size_t bytes, bool dst_on_device, cuda
 void validate_gradepro_params(const pkde_gradepro_params *p, int64_t n);
 void stop_server(pkde_ctx *ctx);
 
-// Binning of one estimation into the paired spectra layout (pkde_binning.cu), in two
-// phases around one host read-back of misc[0..1] (error bits, largest count).
+// Binning of estimations into the paired spectra layout (pkde_resample.cu), several jobs a launch.
 struct DiracJob {
   const pkde_grid *g = nullptr;
   const double *d_data = nullptr;
@@ -563,25 +562,25 @@ struct DiracJob {
   int64_t nboot = 0;
   uint64_t seed = 0;
   double2 *paired_out = nullptr;
-  uint32_t *cell = nullptr;
-  double *rh = nullptr;
-  uint32_t *counts = nullptr;
-  uint32_t *pos = nullptr, *cell_sorted = nullptr;  // samples in lower-cell order
-  uint32_t *cstart = nullptr, *cfill = nullptr, *csum = nullptr;
-  uint32_t *mult = nullptr;  // nboot x n draws per sample (cell order)
-  // low parts of the two-part fixed point: per sample and corner (signed), and the sums
-  // (one 64-bit word per real value of the paired spectra)
-  long long *qm_lo = nullptr, *qv_lo = nullptr;
-  unsigned long long *acc_lo = nullptr;
-  int *misc = nullptr;  // 256-byte device block
-  int64_t corner_off_h[16] = {};
+  uint32_t *cell = nullptr, *pos = nullptr;  // per sample: lower cell, position in cell order
+  uint32_t *cell_sorted = nullptr;           // in cell order: cell,
+  double *rhs = nullptr;                     // remainders
+  uint32_t *cstart = nullptr, *csum = nullptr;
+  uint32_t *counts = nullptr;             // (nboot + 1) x G, the samples' own last
+  uint32_t *mult = nullptr;               // nboot x n draws per sample (cell order)
+  unsigned long long *acc_lo = nullptr;   // low parts of the fixed-point sums
+  int *misc = nullptr;                    // 256-byte device block: error bits, largest count
 };
-size_t dirac_job_scratch(const pkde_grid *g, int64_t n, int64_t nboot);
-void dirac_job_bind(DiracJob &j, char *scratch, int *misc);
-void dirac_job_phase_a(pkde_ctx *ctx, DiracJob &j, cudaStream_t st);
-// hmisc: misc[0..1] read back (checked here), or nullptr: the caller checks the error flags
-// (binning_flags_check) after the call has synchronised; the scales come from the device.
-void dirac_job_phase_b(pkde_ctx *ctx, DiracJob &j, const int *hmisc, cudaStream_t st);
+struct BinningPlan {
+  int count, first[5];  // jobs by dimension
+  unsigned blocks[13];  // per kernel
+};
+size_t dirac_zero_bytes(const pkde_grid *g, int64_t n, int64_t nboot);
+size_t dirac_job_scratch(const pkde_grid *g, int64_t n);
+void dirac_job_bind(DiracJob &j, char *zero, char *scratch, int *misc);
+size_t binning_desc_bytes(int count);
+void binning_describe(const DiracJob *jobs, int count, void *host, BinningPlan &plan);
+void binning_run(pkde_ctx *ctx, const BinningPlan &plan, const void *dev, cudaStream_t st);
 void binning_flags_check(const int *hmisc);
 
 void fft_nd(pkde_ctx *ctx, int ndim, const int64_t *dims, double2 *data, int64_t batch, int dir,
@@ -592,16 +591,6 @@ const double2 *twiddles_device(pkde_ctx *ctx, int n);
 // axis taken from factors[a % nfac][k] * scal[a % nfac] (factors may be null).
 void fft_axis(pkde_ctx *ctx, const LineSet &ls, const double2 *in, double2 *out, int dir,
               const double *const *factors, const double *scal, int nfac, cudaStream_t st, int phase);
-
-// binning (pkde_binning.cu): fills spectra-ready FP64 arrays
-struct BinResult {
-  double *means;   // G x nb
-  double *sq;      // G x nb (null if not requested)
-  uint32_t *counts;
-};
-void dirac_device(pkde_ctx *ctx, const pkde_grid *g, const double *d_data, int64_t n,
-                  const int32_t *d_idx, int64_t nboot, bool identity, uint64_t seed, double *d_means,
-                  double *d_sq, uint32_t *d_counts, cudaStream_t st);
 
 }  // namespace pkde
 

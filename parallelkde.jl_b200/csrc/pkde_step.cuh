@@ -183,8 +183,14 @@ struct Steps1dArgs {
 bool steps1d_ok(const pkde_grid *g);
 size_t steps1d_job_bytes();
 size_t steps1d_state_bytes(int n1, int npairs, int64_t S);
-// host_jobs (page-locked) and dev_jobs: count x steps1d_job_bytes() each.
-void steps1d(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs, void *dev_jobs, cudaStream_t st);
+// Descriptors (count x steps1d_job_bytes()) and launches of several estimations.
+struct Steps1dPlan {
+  static constexpr int kClasses = 5;  // kernels
+  int first[kClasses + 1], S[kClasses];
+  size_t smem[kClasses];
+};
+void steps1d_describe(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs, Steps1dPlan &plan);
+void steps1d_run(pkde_ctx *ctx, const Steps1dPlan &plan, const void *dev_jobs, cudaStream_t st);
 // The convergence state machine over all steps (density and selected step of every point).
 void converge_steps(pkde_ctx *ctx, int64_t G, int S, const double *f_all, const double *mu_all, const double *dlogt,
                     double eps, int64_t steps_low, int64_t steps_over, const StepState &cs, cudaStream_t st);

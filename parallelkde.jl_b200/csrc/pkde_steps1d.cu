@@ -490,8 +490,8 @@ const double2 *stage_twiddles_device(pkde_ctx *ctx, int logn);
 
 size_t steps1d_job_bytes() { return sizeof(Job1); }
 
-void steps1d(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs, void *dev_jobs, cudaStream_t st) {
-  if (count < 1) return;
+void steps1d_describe(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs, Steps1dPlan &plan) {
+  plan = Steps1dPlan{};
   Job1 *hj = reinterpret_cast<Job1 *>(host_jobs);
   // classes: the general kernel's three forms, then the power-of-two lengths 1024 and 2048
   constexpr int NC = 5;
@@ -499,8 +499,9 @@ void steps1d(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs,
     if (n == 1024 || n == 2048) return n == 1024 ? 3 : 4;
     return sh.seq ? 2 : (sh.T == 512 ? 0 : 1);
   };
-  int first[NC + 1] = {}, S[NC] = {};
-  size_t smem[NC] = {};
+  static_assert(NC == Steps1dPlan::kClasses, "classes");
+  int(&first)[NC + 1] = plan.first, (&S)[NC] = plan.S;
+  size_t(&smem)[NC] = plan.smem;
   int k = 0;
   for (int c = 0; c < NC; ++c) {  // the jobs of one kernel lie together
     for (int e = 0; e < count; ++e) {
@@ -540,7 +541,12 @@ void steps1d(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs,
     }
     first[c + 1] = k;
   }
-  PKDE_CUDA_TRY(cudaMemcpyAsync(dev_jobs, hj, sizeof(Job1) * count, cudaMemcpyHostToDevice, st));
+}
+
+void steps1d_run(pkde_ctx *ctx, const Steps1dPlan &plan, const void *dev_jobs, cudaStream_t st) {
+  const int(&first)[Steps1dPlan::kClasses + 1] = plan.first;
+  const int(&S)[Steps1dPlan::kClasses] = plan.S;
+  const size_t(&smem)[Steps1dPlan::kClasses] = plan.smem;
   auto launch = [&](int c, int threads, size_t bytes, auto kern, auto... more) {
     const int m = first[c + 1] - first[c];
     if (!m) return;
@@ -548,7 +554,7 @@ void steps1d(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs,
     {
       Trace tr(ctx, PKDE_PHASE_STEP_VMR, st);
       kern<<<dim3((unsigned)S[c], (unsigned)m), threads, bytes, st>>>(
-          reinterpret_cast<const Job1 *>(dev_jobs) + first[c], more...);
+          static_cast<const Job1 *>(dev_jobs) + first[c], more...);
     }
     PKDE_CHECK_LAUNCH();
   };
