@@ -495,12 +495,13 @@ struct ChunkShape {
 };
 
 // Intermediates of a chunk and f and means of all steps are held up to these many bytes.  The
-// larger the chunk the fewer launches drain the SMs; that its intermediates leave the L2
-// costs less (100 x 100, 100 bootstraps, 250 steps, 64 / 256 / 1024 / 2048 MB: 9.5 / 6.9 / 6.2 / 6.2 ms;
-// 96^3, 32, 100: 94 / 87 / 85 from 256 MB on).  Level 1 for serving lanes, whose memory admission counts on
-// it, and where the device has no room for level 0; level 2 where it has none for that.
-constexpr int64_t kChunkBytes[3] = {int64_t(1) << 30, int64_t(256) << 20, int64_t(16) << 20};
-constexpr int64_t kKeepBytes[3] = {int64_t(512) << 20, int64_t(128) << 20, int64_t(4) << 20};
+// larger the chunk the fewer launches drain the SMs, and the more steps share a reading of the
+// spectra; that its intermediates leave the L2 costs less (100 x 100, 100 bootstraps, 250 steps, with
+// 64 MB / 256 MB / 1 GB / 8 GB: 9.5 / 6.9 / 4.9 / 4.7 ms; 512 x 512, 64, 200, 1 / 2 / 4 / 8 GB: 45.2 / 41.3 /
+// 40.0 / 39.7; 128^3, 32, 150: 194 / 193 / 173 / 167).  Level kServeLevel for serving lanes, whose memory
+// admission counts on it; a higher one where the device has no room.
+constexpr int64_t kChunkBytes[kChunkLevels] = {int64_t(8) << 30, int64_t(1) << 30, int64_t(256) << 20, int64_t(16) << 20};
+constexpr int64_t kKeepBytes[kChunkLevels] = {int64_t(8) << 30, int64_t(512) << 20, int64_t(128) << 20, int64_t(4) << 20};
 ChunkShape chunk_shape(int64_t G, int npairs, int S, int level) {
   ChunkShape c;
   const int64_t step = (int64_t)sizeof(double2) * (2 * npairs + 1) * G;
@@ -699,7 +700,6 @@ void add_rows(Launch<RowsJob> (&Ls)[2], const ChunkArgs &A, const ChunkPlan &P, 
   J.out = out;
   J.tiles = (J.ax.lines + J.rt - 1) / J.rt;
   J.C = C;
-  if (!vmr) J.ax.fused = 0;  // no kernel of its own
   Ls[T == 128 ? 0 : 1].add(J, (unsigned)J.tiles * C, sizeof(double2) * 2 * (size_t)J.t.size, alone);
 }
 
@@ -810,19 +810,20 @@ void run_chunk(pkde_ctx *ctx, const ChunkArgs *args, int count, char *const *scr
   for (size_t i = 0; i < all.size(); ++i) {
     ChunkLaunches &L = all[i];
     launch(L.axis[0], at[i][0], kCT, PKDE_PHASE_STEP_FFT, chunk_axis_kernel<true>, chunk_axis_many_kernel<true>,
-           [&](const AxisJob &J) { return chunk_pow2_axis(ctx, J, true, st); });
+           [&](const AxisJob &J) { chunk_pow2_axis(ctx, J, true, st); });
     for (int j = 1; j < 3; ++j)
       launch(L.axis[j], at[i][j], kCT, PKDE_PHASE_STEP_FFT, chunk_axis_kernel<false>, chunk_axis_many_kernel<false>,
-             [&](const AxisJob &J) { return chunk_pow2_axis(ctx, J, false, st); });
-    auto pow2_rows = [&](const RowsJob &J) { return chunk_pow2_rows(ctx, J, st); };
+             [&](const AxisJob &J) { chunk_pow2_axis(ctx, J, false, st); });
+    auto pow2_rows = [&](const RowsJob &J) { chunk_pow2_rows(ctx, J, st); };
+    auto pow2_means = [&](const RowsJob &J) { chunk_pow2_means(ctx, J, st); };
     launch(L.vmr[0], at[i][3], 128, PKDE_PHASE_STEP_VMR, chunk_rows_kernel<128, true>, chunk_rows_many_kernel<128, true>,
            pow2_rows);
     launch(L.vmr[1], at[i][4], 256, PKDE_PHASE_STEP_VMR, chunk_rows_kernel<256, true>, chunk_rows_many_kernel<256, true>,
            pow2_rows);
     launch(L.means[0], at[i][5], 128, PKDE_PHASE_STEP_MEANS, chunk_rows_kernel<128, false>,
-           chunk_rows_many_kernel<128, false>, [](const RowsJob &) {});
+           chunk_rows_many_kernel<128, false>, pow2_means);
     launch(L.means[1], at[i][6], 256, PKDE_PHASE_STEP_MEANS, chunk_rows_kernel<256, false>,
-           chunk_rows_many_kernel<256, false>, [](const RowsJob &) {});
+           chunk_rows_many_kernel<256, false>, pow2_means);
     for (const auto &c : converge[i]) {
       const ChunkArgs &A = args[c[0]];
       const ChunkPlan &P = plan[c[0]];

@@ -75,5 +75,6 @@ __device__ __forceinline__ void chunk_welford(double x, double inv, double2 &st)
 // (pkde_chunk_pow2.cu).
 void chunk_pow2_axis(pkde_ctx *ctx, const AxisJob &J, bool spectra, cudaStream_t st);
 void chunk_pow2_rows(pkde_ctx *ctx, const RowsJob &J, cudaStream_t st);
+void chunk_pow2_means(pkde_ctx *ctx, const RowsJob &J, cudaStream_t st);
 
 }  // namespace pkde

@@ -238,6 +238,47 @@ __global__ void __launch_bounds__(kT, 2)
   }
 }
 
+// The means' rows: `per` tiles of NL rows in turn, magnitudes out.
+template <int LOGN>
+__global__ void __launch_bounds__(kT, 2)
+    p2_means_kernel(const __grid_constant__ RowsJob job, const double2 *__restrict__ tw_g, int per, unsigned tiles) {
+  using P = PT<LOGN>;
+  using I = TileIdx<LOGN, false, P::NL>;
+  double2 *tile = smp, *sm_tw = smp + 2 * P::TILE;
+  const unsigned tpa = job.ax.lines / P::NL;
+  const int t = I::bfly(), l = I::line();
+  const unsigned u0 = blockIdx.x * per, u1 = min(u0 + per, tiles);
+  auto row_of = [&](unsigned u, unsigned &c) {
+    c = u / tpa;
+    return (int64_t)((u - c * tpa) * P::NL + l) * P::N;
+  };
+  unsigned c;
+  int64_t row = row_of(u0, c);
+  double2 nx[8];
+  auto load = [&] {
+    const double2 *src = job.in + ((int64_t)c * job.A + job.arr0) * job.G + row;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) nx[r] = __ldcg(src + in_pos<LOGN>(t, r));
+  };
+  load();
+  p2_twiddles<LOGN>(sm_tw, tw_g);
+  __syncthreads();
+  for (unsigned u = u0; u < u1; ++u) {
+    double2 v[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) v[r] = nx[r];
+    double *o = job.out + (int64_t)c * job.G + row;
+    if (u + 1 < u1) {
+      row = row_of(u + 1, c);
+      load();
+    }
+    dft_r<8>(v);
+    p2_rest<LOGN, 0, false, P::NL, false>(tile + l * P::LP, nullptr, v, t, sm_tw, l);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[out_pos<LOGN>(t, i)] = sqrt(__fma_rn(v[i].x, v[i].x, __dmul_rn(v[i].y, v[i].y)));
+  }
+}
+
 int log2_of(int n) {
   int l = 0;
   while ((1 << l) < n) ++l;
@@ -300,6 +341,21 @@ void chunk_pow2_rows(pkde_ctx *ctx, const RowsJob &J, cudaStream_t st) {
     allow_dynamic_smem(ctx, p2_rows_kernel<L>, p2_smem<L>());                                                     \
     Trace tr(ctx, PKDE_PHASE_STEP_VMR, st);                                                                       \
     p2_rows_kernel<L><<<blocks, kT, p2_smem<L>(), st>>>(J, stage_twiddles_device(ctx, L));                        \
+  }
+  PKDE_P2_SWITCH(J.ax.n, PKDE_CALL)
+#undef PKDE_CALL
+  PKDE_CHECK_LAUNCH();
+}
+
+void chunk_pow2_means(pkde_ctx *ctx, const RowsJob &J, cudaStream_t st) {
+#define PKDE_CALL(L)                                                                                                \
+  {                                                                                                                 \
+    const int64_t tiles = (int64_t)(J.ax.lines / PT<L>::NL) * J.C;                                                  \
+    const int per = per_cta(ctx, tiles, tiles);                                                                     \
+    allow_dynamic_smem(ctx, p2_means_kernel<L>, p2_smem<L>());                                                      \
+    Trace tr(ctx, PKDE_PHASE_STEP_MEANS, st);                                                                       \
+    p2_means_kernel<L><<<(unsigned)((tiles + per - 1) / per), kT, p2_smem<L>(), st>>>(J, stage_twiddles_device(ctx, L), \
+                                                                                     per, (unsigned)tiles);         \
   }
   PKDE_P2_SWITCH(J.ax.n, PKDE_CALL)
 #undef PKDE_CALL

@@ -832,7 +832,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   // estimations in chunks of steps share launches as far as their scratch together fits the
   // memory budget: chunk_group[i] = first of the i-th set
   std::vector<size_t> chunk_group{0};
-  int chunk_level = ctx->tune_wide ? 0 : 1;
+  int chunk_level = ctx->tune_wide ? 0 : kServeLevel;
   if (!chunk_e.empty()) {
     // the device's free memory is asked for only where the kept scratch does not suffice
     size_t budget = chunk_e.size() > 1 ? shared_budget(ctx, BUF_SCRATCH) : ctx->buf[BUF_SCRATCH].bytes;
@@ -849,7 +849,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     if (most > budget) {
       size_t freeb = 0, totalb = 0;
       PKDE_CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
-      while (chunk_level < 2 && most > (freeb + ctx->buf[BUF_SCRATCH].bytes) / 2) {
+      while (chunk_level + 1 < kChunkLevels && most > (freeb + ctx->buf[BUF_SCRATCH].bytes) / 2) {
         ++chunk_level;
         most = largest();
       }

@@ -77,7 +77,7 @@ size_t footprint(const pkde_gradepro_params *p, int64_t n, bool has_idx) {
   if (N == 1) b += sizeof(double) * 4 * S * G;                                            // 1-D steps
   const size_t slot = std::max<size_t>(32u << 20, sizeof(double2) * 2 * (size_t)G);
   const size_t engine = 8 * slot + 32 * (size_t)G + sizeof(int) * (size_t)S * (P + 1) * (N + G / 16 + 1);
-  b += N > 1 && chunk_ok(&p->grid) ? std::max(engine, chunk_scratch_bytes(&p->grid, (int)P, (int)S, 1)) : engine;
+  b += N > 1 && chunk_ok(&p->grid) ? std::max(engine, chunk_scratch_bytes(&p->grid, (int)P, (int)S, kServeLevel)) : engine;
   return b + (4u << 20);
 }
 

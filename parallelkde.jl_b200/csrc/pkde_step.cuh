@@ -160,7 +160,8 @@ struct ChunkArgs {
 bool chunk_ok(const pkde_grid *g);
 // Whether an estimation that chunk_ok takes runs in chunks (a schedule file may say otherwise).
 bool chunk_schedule(pkde_ctx *ctx, const pkde_grid *g, int npairs);
-// Scratch at a memory level (0: the largest chunks .. 2).
+// Scratch at a memory level (0: the largest chunks .. kChunkLevels - 1).
+constexpr int kChunkLevels = 4, kServeLevel = 2;
 size_t chunk_scratch_bytes(const pkde_grid *g, int npairs, int S, int level);
 // Whether density and selected step come out final (else the caller initialises the state
 // before and fills the points without a selected step after).
