@@ -18,6 +18,7 @@
 
 #include "pkde_chunk.cuh"
 #include "pkde_jobs.cuh"
+#include "pkde_tile.cuh"
 
 namespace pkde {
 namespace {
@@ -38,17 +39,6 @@ __host__ __device__ __forceinline__ int axis_tiles_held(const ChunkAxis &ax) {
 }
 
 extern __shared__ double2 smc[];
-
-// Shared memory by byte address: strided accesses then cost one 32-bit addition each.
-__device__ __forceinline__ unsigned smem_of(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ double2 lds(unsigned a) {
-  double2 v;
-  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ void sts(unsigned a, double2 v) {
-  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
-}
 
 // Where a tile's lines come from and go to, as byte offsets of 32 bits from a base that is the
 // same for the block.
@@ -204,10 +194,7 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
 #pragma unroll
         for (int n1 = 0; n1 < Q; ++n1, p += L * 16u) {
           y[n1] = lds(p);
-          if (n1 > 0) {  // the engine's combine fuses the other product of the imaginary part
-            const double2 v = y[n1], w = __ldg(ax.twc + (n1 - 1) * M + k2);
-            y[n1] = make_double2(__fma_rn(v.x, w.x, -__dmul_rn(v.y, w.y)), __fma_rn(v.x, w.y, __dmul_rn(v.y, w.x)));
-          }
+          if (n1 > 0) y[n1] = combine_cmul(y[n1], __ldg(ax.twc + (n1 - 1) * M + k2));
         }
         dft_r<Q>(y);
         put(l, k2, M, y, rc);
@@ -307,10 +294,6 @@ __global__ void __launch_bounds__(kCT, kCtas)
   axis_body<SPECTRA>(job, blockIdx.x - first);
 }
 
-__device__ __forceinline__ void cp_async16(unsigned dst, const double2 *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-
 // The rows of a tile in shared memory, element k of line l at unit k PN + l.
 struct RowsTile {
   unsigned base, ss;
@@ -393,7 +376,8 @@ __device__ __forceinline__ void rows_body(const RowsJob &job, unsigned block) {
       for (int q = 0; q < kRowPts; ++q) {
         if (threadIdx.x + q * kRT < count) {
           const double2 zv = lds(res + at[q]), wv = lds(res + at[q] + rt * 16u);
-          const double xa = chunk_vmr(zv.x, wv.x, job.inv_n), xb = chunk_vmr(zv.y, wv.y, job.inv_n);
+          double xa, xb;
+          chunk_vmr2(zv, wv, job.inv_n, xa, xb);
           chunk_welford(xa, ra, st[q]);
           if (has_b) chunk_welford(xb, rb, st[q]);
         }
@@ -573,11 +557,12 @@ struct Launch {
   std::vector<unsigned> block0;
   unsigned blocks = 0;
   size_t smem = 0;
-  // power-of-two jobs with a kernel of their own, launched one by one: alone in their pass, or
-  // large enough to fill the device
+  // jobs with a kernel for their length (chunk of steps of 96^3, 32 bootstraps, 100 steps: 69.5 ms in
+  // the general kernels, 50.9; 100 x 100, 100, 250: 4.7 and 3.6), launched one by one: alone in
+  // their pass, or large enough to fill the device
   std::vector<J> solo;
   void add(const J &j, unsigned n, size_t bytes, bool alone) {
-    if (j.ax.fused && (alone || n >= kSoloBlocks)) {
+    if ((j.ax.fused || j.ax.fixed) && (alone || n >= kSoloBlocks)) {
       solo.push_back(j);
       return;
     }
@@ -638,6 +623,7 @@ ChunkPlan plan_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch) {
     a.fused = k.pow2;
     a.twc = k.R > 1 ? combine_twiddles_device(ctx, k.R, a.M) : nullptr;
     a.nst = make_stages(ctx, a.M, a.st);
+    a.fixed = chunk_len_known(a.n, a.R);
     a.generic_first = a.st[0].R > 5 && a.st[0].R != 8;
     inner *= a.n;
   }
@@ -789,8 +775,8 @@ void run_chunk(pkde_ctx *ctx, const ChunkArgs *args, int count, char *const *scr
     }
   }
   if (bytes) PKDE_CUDA_TRY(cudaMemcpyAsync(dev, host.data(), bytes, cudaMemcpyHostToDevice, st));
-  auto launch = [&](auto &L, size_t o, int threads, int phase, auto one, auto many, auto pow2) {
-    for (const auto &j : L.solo) pow2(j);
+  auto launch = [&](auto &L, size_t o, int threads, int phase, auto one, auto many, auto solo) {
+    for (const auto &j : L.solo) solo(j);
     if (L.jobs.empty()) return;
     using J = std::decay_t<decltype(L.jobs[0])>;
     const J *jobs = reinterpret_cast<const J *>(dev + o);
@@ -810,20 +796,20 @@ void run_chunk(pkde_ctx *ctx, const ChunkArgs *args, int count, char *const *scr
   for (size_t i = 0; i < all.size(); ++i) {
     ChunkLaunches &L = all[i];
     launch(L.axis[0], at[i][0], kCT, PKDE_PHASE_STEP_FFT, chunk_axis_kernel<true>, chunk_axis_many_kernel<true>,
-           [&](const AxisJob &J) { chunk_pow2_axis(ctx, J, true, st); });
+           [&](const AxisJob &J) { (J.ax.fused ? chunk_pow2_axis : chunk_len_axis)(ctx, J, true, st); });
     for (int j = 1; j < 3; ++j)
       launch(L.axis[j], at[i][j], kCT, PKDE_PHASE_STEP_FFT, chunk_axis_kernel<false>, chunk_axis_many_kernel<false>,
-             [&](const AxisJob &J) { chunk_pow2_axis(ctx, J, false, st); });
-    auto pow2_rows = [&](const RowsJob &J) { chunk_pow2_rows(ctx, J, st); };
-    auto pow2_means = [&](const RowsJob &J) { chunk_pow2_means(ctx, J, st); };
+             [&](const AxisJob &J) { (J.ax.fused ? chunk_pow2_axis : chunk_len_axis)(ctx, J, false, st); });
+    auto solo_rows = [&](const RowsJob &J) { (J.ax.fused ? chunk_pow2_rows : chunk_len_rows)(ctx, J, st); };
+    auto solo_means = [&](const RowsJob &J) { (J.ax.fused ? chunk_pow2_means : chunk_len_means)(ctx, J, st); };
     launch(L.vmr[0], at[i][3], 128, PKDE_PHASE_STEP_VMR, chunk_rows_kernel<128, true>, chunk_rows_many_kernel<128, true>,
-           pow2_rows);
+           solo_rows);
     launch(L.vmr[1], at[i][4], 256, PKDE_PHASE_STEP_VMR, chunk_rows_kernel<256, true>, chunk_rows_many_kernel<256, true>,
-           pow2_rows);
+           solo_rows);
     launch(L.means[0], at[i][5], 128, PKDE_PHASE_STEP_MEANS, chunk_rows_kernel<128, false>,
-           chunk_rows_many_kernel<128, false>, pow2_means);
+           chunk_rows_many_kernel<128, false>, solo_means);
     launch(L.means[1], at[i][6], 256, PKDE_PHASE_STEP_MEANS, chunk_rows_kernel<256, false>,
-           chunk_rows_many_kernel<256, false>, pow2_means);
+           chunk_rows_many_kernel<256, false>, solo_means);
     for (const auto &c : converge[i]) {
       const ChunkArgs &A = args[c[0]];
       const ChunkPlan &P = plan[c[0]];

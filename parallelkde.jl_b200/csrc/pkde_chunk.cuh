@@ -14,6 +14,7 @@ struct ChunkAxis {
   int n, M, R, nst, inner, lines;
   int generic_first;   // the first stage has a generic radix: one more exchange
   int fused;           // the first stage's sums fuse the scaling of one operand (power-of-two register tiles)
+  int fixed;           // a length with passes of its own (pkde_chunk_len.cuh)
   const double2 *twc;  // combine twiddles [n1 - 1][k2]
   Stage1 st[kStages1];
 };
@@ -59,10 +60,10 @@ __device__ __forceinline__ double recip_of(const double *table, int i) {
   return i < kChunkRecip ? __ldg(table + i) : 1.0 / (double)i;
 }
 
-// VMR of one bootstrap at one point (DirectSpace.jl:550-552), 1 / n as a product.
-__device__ __forceinline__ double chunk_vmr(double Mv, double Vv, double inv_n) {
-  const double m = __dmul_rn(fabs(Mv), inv_n);
-  return div_nr(__fma_rn(-m, m, __dmul_rn(fabs(Vv), inv_n)), m);
+// VMR of the two bootstraps of a pair at one point (DirectSpace.jl:550-552), 1 / n as a product.
+__device__ __forceinline__ void chunk_vmr2(double2 z, double2 w, double inv_n, double &xa, double &xb) {
+  const double ma = __dmul_rn(fabs(z.x), inv_n), mb = __dmul_rn(fabs(z.y), inv_n);
+  div_nr2(__fma_rn(-ma, ma, __dmul_rn(fabs(w.x), inv_n)), ma, __fma_rn(-mb, mb, __dmul_rn(fabs(w.y), inv_n)), mb, xa, xb);
 }
 
 __device__ __forceinline__ void chunk_welford(double x, double inv, double2 &st) {
@@ -76,5 +77,11 @@ __device__ __forceinline__ void chunk_welford(double x, double inv, double2 &st)
 void chunk_pow2_axis(pkde_ctx *ctx, const AxisJob &J, bool spectra, cudaStream_t st);
 void chunk_pow2_rows(pkde_ctx *ctx, const RowsJob &J, cudaStream_t st);
 void chunk_pow2_means(pkde_ctx *ctx, const RowsJob &J, cudaStream_t st);
+
+// Passes along axes of the lengths known at compile time (pkde_chunk_len.cuh).
+bool chunk_len_known(int n, int R);
+void chunk_len_axis(pkde_ctx *ctx, const AxisJob &J, bool spectra, cudaStream_t st);
+void chunk_len_rows(pkde_ctx *ctx, const RowsJob &J, cudaStream_t st);
+void chunk_len_means(pkde_ctx *ctx, const RowsJob &J, cudaStream_t st);
 
 }  // namespace pkde

@@ -220,7 +220,8 @@ __global__ void __launch_bounds__(kT, 2)
     for (int i = 0; i < 4; ++i) {
       const double2 o = other[i * P::NB8 + t];
       const double2 z = h ? o : v[i], w = h ? v[i + 4] : o;
-      const double xa = chunk_vmr(z.x, w.x, job.inv_n), xb = chunk_vmr(z.y, w.y, job.inv_n);
+      double xa, xb;
+      chunk_vmr2(z, w, job.inv_n, xa, xb);
       chunk_welford(xa, ra, st[i]);
       if (has_b) chunk_welford(xb, rb, st[i]);
     }

@@ -668,6 +668,25 @@ __device__ __forceinline__ double div_nr(double v, double m) {
   if (em - 3u > 2041u || er - 1u > 2045u) return __ddiv_rn(v, m);
   return r;
 }
+// Two quotients of m >= 0, bit for bit those of div_nr.  One test covers both: alone, the IEEE
+// division is short enough for the compiler to issue it predicated on every call.
+__device__ __forceinline__ void div_nr2(double va, double ma, double vb, double mb, double &xa, double &xb) {
+  double ya, yb;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ya) : "d"(ma));
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(yb) : "d"(mb));
+  ya = fma(ya, fma(-ma, ya, 1.0), ya);
+  yb = fma(yb, fma(-mb, yb, 1.0), yb);
+  const double qa = __dmul_rn(va, ya), qb = __dmul_rn(vb, yb);
+  xa = fma(fma(-ma, qa, va), ya, qa);
+  xb = fma(fma(-mb, qb, vb), yb, qb);
+  // the tests of div_nr on the high words: exponent of m in [3, 2044], of the quotient in [1, 2046]
+  const unsigned ha = (unsigned)__double2hiint(ma) - (3u << 20), hb = (unsigned)__double2hiint(mb) - (3u << 20);
+  const unsigned ra = 2u * (unsigned)__double2hiint(xa) - (1u << 21), rb = 2u * (unsigned)__double2hiint(xb) - (1u << 21);
+  if (max(ha, hb) >= 2042u << 20 || max(ra, rb) >= 2046u << 21) {
+    xa = div_nr(va, ma);
+    xb = div_nr(vb, mb);
+  }
+}
 }  // namespace pkde
 
 // Entry-point wrapper: converts exceptions into status codes + the thread's last error
