@@ -45,11 +45,12 @@ extern __shared__ double2 smc[];
 //   Src: at(l): offset of line l; load(offset); STEP(): bytes from element to element
 //   Dst: at(l): offset (ok(offset): the line exists); store(offset, v); step()
 // Lines through every stage, tiles a and b (byte addresses) in turn.  SCALED: element k of line
-// l is multiplied by f[k] c, (f, c) = src.factor(l).  Every thread calls; the caller
+// l is multiplied by f[k] c, (f, c) = src.factor(l).  tw: the plain twiddle table in shared
+// memory (copy_table), 0 where the line has none.  Every thread calls; the caller
 // synchronises before the tiles are reused.
 template <int T, bool SCALED, class Src, class Dst>
 __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const ChunkTile &t, unsigned a, unsigned b,
-                                                const Src &src, const Dst &dst) {
+                                                unsigned tw, const Src &src, const Dst &dst) {
   const int R = ax.R, L = t.L, Lr = t.Lr, total = ax.nst + (R > 1 ? 1 : 0);
   const unsigned PB = t.P * 16u;
   const FastDiv dLr = t.dLr;
@@ -167,16 +168,26 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
       case 2: stage(std::integral_constant<int, 2>{}); break;
       case 3: stage(std::integral_constant<int, 3>{}); break;
       case 5: stage(std::integral_constant<int, 5>{}); break;
-      default:
-        line_stage_generic<T>(s, ax.n, Lr, dLr, smc + (in - smem_of(smc)) / 16, t.P, [&](int l, int pos, double2 v) {
+      default: {
+        const unsigned base = in;
+        auto ld = [base](unsigned p) { return lds(base + p); };
+        auto put1 = [&](int l, int pos, double2 v) {
           if (last) {
             const unsigned o = dst.at(l);
             if (dst.ok(o)) dst.store(o + pos * dst.step(), v);
           } else {
             sts(out + pos * PB + l * 16u, v);
           }
-        });
+        };
+        if (tw) {
+          line_stage_generic<T>(s, ax.n, L, t.H, t.dH, PB, [tw](unsigned o) { return lds(tw + o); }, ld, put1);
+        } else {
+          const char *g = reinterpret_cast<const char *>(s.tw);
+          line_stage_generic<T>(s, ax.n, L, t.H, t.dH, PB,
+                                [g](unsigned o) { return __ldg(reinterpret_cast<const double2 *>(g + o)); }, ld, put1);
+        }
         break;
+      }
     }
     if (!last) __syncthreads();
     const unsigned x = in;
@@ -203,6 +214,20 @@ __device__ __forceinline__ void chunk_transform(const ChunkAxis &ax, const Chunk
     if (R == 3) combine(std::integral_constant<int, 3>{});
     else combine(std::integral_constant<int, 5>{});
   }
+}
+
+// A line with a stage of another radix reads n factors all the time, which the L1 left beside the
+// tiles does not hold for long: up to kTableLen points they go to shared memory (beyond, they would
+// cost a resident CTA).
+constexpr int kTableLen = 512;
+__host__ __device__ __forceinline__ int table_points(const ChunkAxis &ax) {
+  return ax.plain && ax.n <= kTableLen ? ax.n : 0;
+}
+template <int T>
+__device__ __forceinline__ unsigned copy_table(const ChunkAxis &ax, double2 *to) {
+  if (!table_points(ax)) return 0;
+  for (int i = threadIdx.x; i < ax.n; i += T) to[i] = __ldg(ax.plain + i);
+  return smem_of(to);
 }
 
 // Inverse FFT along one axis >= 2 of A arrays in each of C steps.  Tile = L consecutive lines of
@@ -245,7 +270,9 @@ __device__ __forceinline__ void axis_body(const AxisJob &job, unsigned block) {
   const ChunkAxis &ax = job.ax;
   const ChunkTile &t = job.t;
   const ChunkRun &run = job.run;
-  const double **sf = reinterpret_cast<const double **>(smc + axis_tiles_held(ax) * t.size);
+  double2 *table = smc + axis_tiles_held(ax) * t.size;
+  const unsigned tw = copy_table<kCT>(ax, table);
+  const double **sf = reinterpret_cast<const double **>(table + table_points(ax));
   double *sc = reinterpret_cast<double *>(sf + t.L);
   unsigned *off = reinterpret_cast<unsigned *>(sc + t.L);
   const unsigned G = run.G, lines = ax.lines, inner = ax.inner;
@@ -278,7 +305,7 @@ __device__ __forceinline__ void axis_body(const AxisJob &job, unsigned block) {
       reinterpret_cast<const char *>(job.in + (SPECTRA ? (int64_t)(run.a0 + arr0) * G : base)), inner * 16u, off, sf, sc};
   const AxisDst dst{reinterpret_cast<char *>(job.out + base), inner * 16u, off, valid};
   const unsigned a = smem_of(smc);
-  chunk_transform<kCT, SPECTRA>(ax, t, a, a + t.size * 16u, src, dst);
+  chunk_transform<kCT, SPECTRA>(ax, t, a, a + t.size * 16u, tw, src, dst);
 }
 
 template <bool SPECTRA>
@@ -356,6 +383,7 @@ __device__ __forceinline__ void rows_body(const RowsJob &job, unsigned block) {
   const int total = ax.nst + (ax.R > 1 ? 1 : 0) + ax.generic_first;
   unsigned cur = tile0;  // the tile (of two) that holds the inputs
   const unsigned both = 2 * tile0 + tsize;
+  const unsigned tw = copy_table<kRT>(ax, smc + 2 * t.size);
   load(cur);
   const int pairs = VMR ? job.pairs : 1;
   for (int p = 0; p < pairs; ++p) {
@@ -363,7 +391,7 @@ __device__ __forceinline__ void rows_body(const RowsJob &job, unsigned block) {
     __syncthreads();
     // each stage reads one tile and writes the other
     const unsigned res = (total & 1) ? both - cur : cur;
-    chunk_transform<kRT, false>(ax, t, both - cur, cur, RowsTile{cur, PB}, RowsTile{res, PB});
+    chunk_transform<kRT, false>(ax, t, both - cur, cur, tw, RowsTile{cur, PB}, RowsTile{res, PB});
     __syncthreads();
     cur = both - res;
     z += 2 * (int64_t)G;
@@ -459,16 +487,39 @@ __global__ void __launch_bounds__(kCT) chunk_converge_kernel(int64_t G, int C, i
   cs.mu_last[i] = m;
 }
 
-// Lines per tile: as many as 2048 points hold, balanced over the tiles.
-ChunkTile make_tile(int n, int R, int64_t lines, int most, bool odd) {
-  const int64_t tiles = (lines + most - 1) / most;
+// Lines per tile, at most `most` (as many as its points hold) of `per` sub-tiles each (the rows
+// kernel's z and w): the number that leaves the fewest butterfly slots of T threads empty over
+// all tiles.  An item of a radix other than 2, 3, 4, 5, 8 is four outputs of R terms, so an idle
+// third of a pass of threads costs as much as the other stages together (41 points, 256 threads: 49
+// lines are 539 items in three passes, 46 are 506 in two: 150 x 77, 100 bootstraps, 250 steps 8.3 -> 7.9 ms).
+int balanced_lines(const ChunkAxis &ax, int64_t lines, int most, int per, int T) {
+  int best = 1;
+  double best_cost = 1e300;
+  for (int L = (int)std::min<int64_t>(most, lines); L >= 1 && 2 * L >= std::min<int64_t>(most, lines); --L) {
+    double cost = 0.0;
+    auto add = [&](int64_t items, double work) { cost += (double)((items + T - 1) / T) * work; };
+    for (int i = 0; i < ax.nst; ++i) {
+      const int R = ax.st[i].R, nb = ax.st[i].nb * ax.R;
+      if (R <= 5 || R == 8) add((int64_t)nb * L * per, 12.0 * R);
+      else add((int64_t)((R + 3) / 4) * nb * ((L * per + 1) / 2), 60.0 * R);
+    }
+    if (ax.R > 1) add((int64_t)ax.M * L * per, 12.0 * ax.R);
+    cost *= (double)((lines + L - 1) / L);
+    if (cost < best_cost) best_cost = cost, best = L;
+  }
+  return best;
+}
+
+ChunkTile make_tile(int n, int R, int L, bool odd) {
   ChunkTile t;
-  t.L = (int)((lines + tiles - 1) / tiles);
+  t.L = L;
   t.Lr = t.L * R;
   t.P = odd ? t.Lr | 1 : t.Lr;
   t.PN = odd ? t.L | 1 : t.L;
   t.size = std::max(n * t.PN, n / R * t.P);
+  t.H = (t.L + 1) / 2;
   t.dL = make_fastdiv((uint32_t)t.L);
+  t.dH = make_fastdiv((uint32_t)t.H);
   t.dLr = make_fastdiv((uint32_t)t.Lr);
   return t;
 }
@@ -624,6 +675,8 @@ ChunkPlan plan_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch) {
     a.twc = k.R > 1 ? combine_twiddles_device(ctx, k.R, a.M) : nullptr;
     a.nst = make_stages(ctx, a.M, a.st);
     a.fixed = chunk_len_known(a.n, a.R);
+    for (int i = 0; i < a.nst; ++i)
+      if (a.st[i].R > 5 && a.st[i].R != 8) a.plain = a.st[i].tw;
     a.generic_first = a.st[0].R > 5 && a.st[0].R != 8;
     inner *= a.n;
   }
@@ -656,11 +709,10 @@ void add_axes(ChunkLaunches &L, const ChunkArgs &A, const ChunkPlan &P, int64_t 
     J.run.a0 = a0;
     J.run.A = arrays;
     const int64_t lines = (int64_t)arrays * J.ax.lines;
-    const int most = kTilePts / J.ax.n;
-    J.t = make_tile(J.ax.n, J.ax.R, lines, most, false);
+    J.t = make_tile(J.ax.n, J.ax.R, balanced_lines(J.ax, lines, kTilePts / J.ax.n, 1, kCT), false);
     J.in = j == N - 1 ? A.spectra : P.mid;
     J.out = P.mid;
-    const size_t smem = sizeof(double2) * (size_t)axis_tiles_held(J.ax) * J.t.size + 20 * (size_t)J.t.L;
+    const size_t smem = sizeof(double2) * (size_t)(axis_tiles_held(J.ax) * J.t.size + table_points(J.ax)) + 20 * (size_t)J.t.L;
     L.axis[N - 1 - j].add(J, (unsigned)((lines + J.t.L - 1) / J.t.L * C), smem, alone);
   }
 }
@@ -670,8 +722,8 @@ void add_rows(Launch<RowsJob> (&Ls)[2], const ChunkArgs &A, const ChunkPlan &P, 
   RowsJob J{};
   J.ax = P.ax[0];
   const int per = vmr ? 2 : 1, T = row_threads(J.ax.n), most = T * kRowPts / J.ax.n;
-  J.rt = make_tile(J.ax.n, 1, J.ax.lines, most, false).L;
-  J.t = make_tile(J.ax.n, J.ax.R, per * J.rt, per * J.rt, true);
+  J.rt = balanced_lines(J.ax, J.ax.lines, most, per, T);
+  J.t = make_tile(J.ax.n, J.ax.R, per * J.rt, true);
   J.G = P.run.G;
   J.A = arrays;
   J.arr0 = arr0;
@@ -686,7 +738,7 @@ void add_rows(Launch<RowsJob> (&Ls)[2], const ChunkArgs &A, const ChunkPlan &P, 
   J.out = out;
   J.tiles = (J.ax.lines + J.rt - 1) / J.rt;
   J.C = C;
-  Ls[T == 128 ? 0 : 1].add(J, (unsigned)J.tiles * C, sizeof(double2) * 2 * (size_t)J.t.size, alone);
+  Ls[T == 128 ? 0 : 1].add(J, (unsigned)J.tiles * C, sizeof(double2) * (size_t)(2 * J.t.size + table_points(J.ax)), alone);
 }
 
 size_t al256c(size_t x) { return (x + 255) & ~size_t(255); }

@@ -16,13 +16,14 @@ struct ChunkAxis {
   int fused;           // the first stage's sums fuse the scaling of one operand (power-of-two register tiles)
   int fixed;           // a length with passes of its own (pkde_chunk_len.cuh)
   const double2 *twc;  // combine twiddles [n1 - 1][k2]
+  const double2 *plain;  // (cos, sin)(2 pi m / n) of a line with a stage of another radix, else nullptr
   Stage1 st[kStages1];
 };
 // Lines of a tile: L (pitch PN where a tile holds lines), Lr = L R sub-lines (pitch P); size: units
-// of one tile.
+// of one tile; H: half the lines, rounded up (stages of other radices, R = 1).
 struct ChunkTile {
-  int L, Lr, P, PN, size;
-  FastDiv dL, dLr;
+  int L, Lr, P, PN, size, H;
+  FastDiv dL, dLr, dH;
 };
 
 struct ChunkRun {

@@ -134,41 +134,55 @@ __device__ __forceinline__ void line_stage(const Stage1 &s, int L, FastDiv dL, b
   }
 }
 
-// Any other radix: an item is QB outputs of one butterfly, every input is read once an
-// item.  src: the tile (pitch P); st(l, pos, v): output pos of line l.
-template <int T, class St>
-__device__ __forceinline__ void line_stage_generic(const Stage1 &s, int n, int L, FastDiv dL, const double2 *src, int P,
-                                                   St st) {
+// Any other radix: an item is four outputs of one butterfly of two lines, l and l + H (2 H lines
+// of which L exist).  tw(o): the factor at byte o of the plain table; ld(p): the element at p,
+// input r of butterfly j of line l at p = (j + r nb) PB + 16 l; st(l, pos, v): output pos of line l.
+// Six FP64 operations a term, two issue slots each; the two lines share the loads of the
+// factors and their index steps, which else fill the rest of the slots and the load pipe.  The 41
+// points of 50 x 41 x 36, 32 bootstraps, 100 steps: 8.5 ms from the L1 with an item a line, 7.1 with the
+// factors in shared memory, 6.5 here (67 % of the FP64 pipe); the 77 of 150 x 77: 5.3, 5.1, 4.4.
+template <int T, class Tw, class Ld, class St>
+__device__ __forceinline__ void line_stage_generic(const Stage1 &s, int n, int L, int H, FastDiv dH, unsigned PB, Tw tw,
+                                                   Ld ld, St st) {
   constexpr int QB = 4;
   const int R = s.R, nb = s.nb, Ns = s.Ns;
-  const int nblk = (R + QB - 1) / QB, per = nb * L;
+  const int nblk = (R + QB - 1) / QB, per = nb * H;
+  const unsigned end = n * 16u, d = nb * PB;
   for (int i = threadIdx.x; i < nblk * per; i += T) {
     const int qb = i / per, e = i - qb * per;
-    const int j = (int)fdiv((uint32_t)e, dL), l = e - j * L;
+    const int j = (int)fdiv((uint32_t)e, dH), l = e - j * H;
     const int jq = (int)fdiv((uint32_t)j, s.dns), k = j - jq * Ns;
     const int q0 = qb * QB, nq = min(QB, R - q0);
-    double2 v[QB];
-    int m[QB], inc[QB];
+    const bool two = l + H < L;
+    double2 v[QB], w[QB];
+    unsigned m[QB], inc[QB];
 #pragma unroll
     for (int q = 0; q < QB; ++q) {
       m[q] = 0;
-      inc[q] = q < nq ? k * s.tstep + (q0 + q) * nb : 0;
-      v[q] = make_double2(0.0, 0.0);
+      inc[q] = q < nq ? (unsigned)(k * s.tstep + (q0 + q) * nb) * 16u : 0;
+      v[q] = w[q] = make_double2(0.0, 0.0);
     }
-    const double2 *p = src + j * P + l;
-    for (int r = 0; r < R; ++r, p += nb * P) {
-      const double2 x = *p;
+    unsigned p = j * PB + l * 16u;
+    const unsigned next = two ? H * 16u : 0;
+#pragma unroll 1
+    for (int r = 0; r < R; ++r, p += d) {
+      const double2 x = ld(p), y = ld(p + next);
 #pragma unroll
       for (int q = 0; q < QB; ++q) {
-        v[q] = cadd(v[q], cmul1(x, __ldg(s.tw + m[q])));
-        m[q] += inc[q];
-        if (m[q] >= n) m[q] -= n;
+        const double2 f = tw(m[q]);
+        v[q] = cadd(v[q], cmul1(x, f));
+        w[q] = cadd(w[q], cmul1(y, f));
+        const unsigned t = m[q] + inc[q];
+        m[q] = min(t, t - end);
       }
     }
     const int o = j + jq * Ns * (R - 1) + q0 * Ns;
 #pragma unroll
     for (int q = 0; q < QB; ++q)
-      if (q < nq) st(l, o + q * Ns, v[q]);
+      if (q < nq) {
+        st(l, o + q * Ns, v[q]);
+        if (two) st(l + H, o + q * Ns, w[q]);
+      }
   }
 }
 

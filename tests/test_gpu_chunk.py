@@ -18,6 +18,9 @@ pytestmark = pytest.mark.gpu
     ((1024, 3), 3000, 3, 5),          # longest line of the row tiles: one row of z and w
     ((3, 1024), 3000, 3, 5),          # longest line of the column tiles
     ((1009, 4), 3000, 2, 4),          # a prime axis
+    ((511, 5), 3000, 3, 5),           # other radices' factors in shared memory, up to 512 points
+    ((514, 22), 3000, 3, 5),          # and from the L1; an odd number of lines in pairs
+    ((13, 26, 11), 3000, 4, 6),       # one butterfly a line; two lines an item, three axes
     ((33, 33), 3000, 37, 40),         # several steps a chunk, an odd number of bootstraps
     ((96, 100), 5000, 6, 8),          # mixed-radix rows, Stockham columns
     ((100, 40, 16), 5000, 4, 5),      # mixed-radix columns that read the spectra
