@@ -12,11 +12,13 @@ import subprocess
 import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SRC = ["pkde_ctx.cu", "pkde_binning.cu", "pkde_resample.cu", "pkde_fft.cu", "pkde_step.cu", "pkde_steps1d.cu", "pkde_chunk.cu", "pkde_chunk_pow2.cu",
+SRC = ["pkde_ctx.cu", "pkde_binning.cu", "pkde_resample.cu", "pkde_fft.cu", "pkde_step.cu", "pkde_steps1d.cu",
+       "pkde_steps1d_len0.cu", "pkde_steps1d_len1.cu", "pkde_steps1d_len2.cu", "pkde_steps1d_len3.cu", "pkde_steps1d_len4.cu",
+       "pkde_chunk.cu", "pkde_chunk_pow2.cu",
        "pkde_chunk_len0.cu", "pkde_chunk_len1.cu", "pkde_chunk_len2.cu", "pkde_chunk_len3.cu",
        "pkde_engine.cu", "pkde_gradepro.cu",
        "pkde_serve.cu", "pkde_grid.cu"]
-HDR = ["pkde_internal.cuh", "pkde_regfft.cuh", "pkde_step.cuh", "pkde_lines.cuh", "pkde_chunk.cuh", "pkde_chunk_len.cuh", "pkde_tile.cuh", "pkde_jobs.cuh",
+HDR = ["pkde_internal.cuh", "pkde_regfft.cuh", "pkde_step.cuh", "pkde_lines.cuh", "pkde_chunk.cuh", "pkde_chunk_len.cuh", "pkde_len.cuh", "pkde_steps1d.cuh", "pkde_steps1d_len.cuh", "pkde_tile.cuh", "pkde_jobs.cuh",
        os.path.join("..", "..", "include", "pkde_b200.h")]
 OUT = os.path.join(HERE, "lib", "libpkde_b200.so")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

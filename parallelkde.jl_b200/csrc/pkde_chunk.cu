@@ -405,7 +405,7 @@ __device__ __forceinline__ void rows_body(const RowsJob &job, unsigned block) {
         if (threadIdx.x + q * kRT < count) {
           const double2 zv = lds(res + at[q]), wv = lds(res + at[q] + rt * 16u);
           double xa, xb;
-          chunk_vmr2(zv, wv, job.inv_n, xa, xb);
+          chunk_vmr2(zv, wv, job.inv_n, st[q].x, xa, xb);
           chunk_welford(xa, ra, st[q]);
           if (has_b) chunk_welford(xb, rb, st[q]);
         }

@@ -61,10 +61,12 @@ __device__ __forceinline__ double recip_of(const double *table, int i) {
   return i < kChunkRecip ? __ldg(table + i) : 1.0 / (double)i;
 }
 
-// VMR of the two bootstraps of a pair at one point (DirectSpace.jl:550-552), 1 / n as a product.
-__device__ __forceinline__ void chunk_vmr2(double2 z, double2 w, double inv_n, double &xa, double &xb) {
+// VMR of the two bootstraps of a pair at one point (DirectSpace.jl:550-552), 1 / n as a product; mean: of
+// the bootstraps before.
+__device__ __forceinline__ void chunk_vmr2(double2 z, double2 w, double inv_n, double mean, double &xa, double &xb) {
   const double ma = __dmul_rn(fabs(z.x), inv_n), mb = __dmul_rn(fabs(z.y), inv_n);
-  div_nr2(__fma_rn(-ma, ma, __dmul_rn(fabs(w.x), inv_n)), ma, __fma_rn(-mb, mb, __dmul_rn(fabs(w.y), inv_n)), mb, xa, xb);
+  div_nr2(__fma_rn(-ma, ma, __dmul_rn(fabs(w.x), inv_n)), ma, __fma_rn(-mb, mb, __dmul_rn(fabs(w.y), inv_n)), mb, mean,
+          xa, xb);
 }
 
 __device__ __forceinline__ void chunk_welford(double x, double inv, double2 &st) {

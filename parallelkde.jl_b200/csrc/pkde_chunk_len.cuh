@@ -7,24 +7,9 @@
 #include <algorithm>
 
 #include "pkde_chunk.cuh"
-#include "pkde_tile.cuh"
+#include "pkde_len.cuh"
 
 namespace pkde {
-
-// The stages of make_plan for a 5-smooth length.
-struct LenStages {
-  int nst = 0, rad[10] = {};
-};
-__host__ __device__ constexpr LenStages len_stages(int m) {
-  LenStages s;
-  const int pref[5] = {8, 4, 2, 3, 5};
-  for (int i = 0; i < 5; ++i)
-    while (m % pref[i] == 0) {
-      s.rad[s.nst++] = pref[i];
-      m /= pref[i];
-    }
-  return s;
-}
 
 // Lines of a tile: about 800 points in multiples of eight lines (128 bytes of an element's
 // lines side by side, eight lanes of a butterfly position in different banks), four lines from 257
@@ -36,46 +21,10 @@ __host__ __device__ constexpr int len_warps(int threads) {
   return threads > 256 ? 256 : (threads + 31) / 32 * 32;
 }
 
-template <int n, int R>
-struct Len {
-  static constexpr int M = n / R;
-  static constexpr LenStages S = len_stages(M);
-  __host__ __device__ static constexpr int ns(int i) {
-    int v = 1;
-    for (int q = 0; q < i; ++q) v *= S.rad[q];
-    return v;
-  }
-};
-
 // Twiddle tables of the stages ([k][r - 1]) and of the combine, by value of a kernel parameter.
 struct LenTw {
   const double2 *st[10], *comb;
 };
-
-// One stage.  ld(l, j, v): inputs; st(l, pos, v) as line_stage.
-template <int T, int M, int Q, int Ns, int Lr, class Ld, class St>
-__device__ __forceinline__ void len_stage(const double2 *tw, Ld ld, St st) {
-  constexpr int nb = M / Q, items = nb * Lr, IT = (items + T - 1) / T;
-#pragma unroll
-  for (int it = 0; it < IT; ++it) {
-    const int e = (int)threadIdx.x + it * T;
-    if ((it + 1) * T <= items || e < items) {
-      const int j = e / Lr, l = e - j * Lr, jq = j / Ns;
-      double2 v[Q];
-      ld(l, j, v);
-      if constexpr (Ns > 1) {
-        const int k = j - jq * Ns;
-        if (k > 0) {
-          const double2 *w = tw + k * (Q - 1);
-#pragma unroll
-          for (int r = 1; r < Q; ++r) v[r] = cmul1(v[r], __ldg(w + r - 1));
-        }
-      }
-      dft_r<Q>(v);
-      st(l, j + jq * (Ns * (Q - 1)), v);
-    }
-  }
-}
 
 // All stages of L lines of n points through the tiles at byte addresses a and b in turn.
 // first(l, n1, j, step, v): the inputs of butterfly j of sub-line (l, n1), elements n1 + R (j + r step);
@@ -380,7 +329,7 @@ __global__ void __launch_bounds__(RowsLen<n, R>::T, RowsLen<n, R>::ctas)
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
         double xa, xb;
-        chunk_vmr2(zv[q], wv[q], job.inv_n, xa, xb);
+        chunk_vmr2(zv[q], wv[q], job.inv_n, st[it][q].x, xa, xb);
         chunk_welford(xa, ra, st[it][q]);
         if (has_b) chunk_welford(xb, rb, st[it][q]);
       }

@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kT, 2)
       const double2 o = other[i * P::NB8 + t];
       const double2 z = h ? o : v[i], w = h ? v[i + 4] : o;
       double xa, xb;
-      chunk_vmr2(z, w, job.inv_n, xa, xb);
+      chunk_vmr2(z, w, job.inv_n, st[i].x, xa, xb);
       chunk_welford(xa, ra, st[i]);
       if (has_b) chunk_welford(xb, rb, st[i]);
     }

@@ -186,9 +186,13 @@ size_t steps1d_job_bytes();
 size_t steps1d_state_bytes(int n1, int npairs, int64_t S);
 // Descriptors (count x steps1d_job_bytes()) and launches of several estimations.
 struct Steps1dPlan {
-  static constexpr int kClasses = 5;  // kernels
+  static constexpr int kClasses = 6;  // kernels
   int first[kClasses + 1], S[kClasses];
   size_t smem[kClasses];
+  struct Len {
+    int n, first, count, S;
+  };
+  std::vector<Len> len;  // the jobs of the last class by length
 };
 void steps1d_describe(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs, Steps1dPlan &plan);
 void steps1d_run(pkde_ctx *ctx, const Steps1dPlan &plan, const void *dev_jobs, cudaStream_t st);

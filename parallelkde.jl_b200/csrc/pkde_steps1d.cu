@@ -12,26 +12,10 @@
 
 #include "pkde_lines.cuh"
 #include "pkde_regfft.cuh"
-#include "pkde_step.cuh"
+#include "pkde_steps1d.cuh"
 
 namespace pkde {
 namespace {
-
-// One estimation (device-resident descriptor).  A tile holds the L = 2 a arrays (z, w) of
-// a bootstrap pairs; index 0 / 1 / 2: full tile, last tile, means (L = 1).
-struct Job1 {
-  int n, npairs, nboot, S, a, P, nst;
-  int fused;  // 1: the arithmetic of the step engine's power-of-two tiles, 0: every operation rounded by itself
-  int L[3];
-  FastDiv dL[3];
-  int64_t tab_stride;
-  const double2 *spectra;
-  const double *fz, *fw, *cw, *vscale;
-  double invG, ns, inv_ns;
-  double *f_out, *mu_out;
-  double2 *state;  // S x n running (mean, m2), lines too long for shared memory
-  Stage1 st[kStages1];
-};
 
 extern __shared__ double2 sm1[];
 
@@ -175,46 +159,6 @@ __device__ __forceinline__ int transform1(const Job1 &J, int a, int b, const dou
   return dst;
 }
 
-// x / d correctly rounded for an integer 1 <= d < 2^31 and rd = 1 / d rounded: the residual
-// x - q d of the first quotient is exact (an integer multiple of ulp(q) below 2^33 of
-// them), and x / d is either representable or at least ulp / (2 d) away from a rounding
-// midpoint, far more than the error of the correction.  For x whose exponent field is in
-// [100, 2000], where nothing underflows or overflows.
-__device__ __forceinline__ double div_int(double x, double d, double rd) {
-  const double q = __dmul_rn(x, rd);
-  return __fma_rn(__fma_rn(-q, d, x), rd, q);
-}
-__device__ __forceinline__ bool div_int_range(double x) {
-  return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 100u <= 1900u;
-}
-
-// VMR of one bootstrap at one point and its Welford update (DirectSpace.jl:550-552,
-// 572-577), i its number and inv_i = 1 / i.
-template <bool FUSED>
-__device__ __forceinline__ void vmr_update(double Mv, double Vv, double ns, double inv_ns, double i, double inv_i,
-                                           double2 &st) {
-  if constexpr (FUSED) {
-    const double m = __dmul_rn(fabs(Mv), inv_ns);
-    const double v = __fma_rn(-m, m, __dmul_rn(fabs(Vv), inv_ns));
-    const double x = div_nr(v, m);
-    const double delta = __dsub_rn(x, st.x);
-    st.x = __fma_rn(delta, inv_i, st.x);
-    st.y = __fma_rn(delta, __dsub_rn(x, st.x), st.y);
-  } else {
-    double m = div_int(fabs(Mv), ns, inv_ns), a = div_int(fabs(Vv), ns, inv_ns);
-    if (!(div_int_range(Mv) && div_int_range(Vv))) {
-      m = __ddiv_rn(fabs(Mv), ns);
-      a = __ddiv_rn(fabs(Vv), ns);
-    }
-    const double x = __ddiv_rn(__dsub_rn(a, __dmul_rn(m, m)), m);
-    const double delta = __dsub_rn(x, st.x);
-    double c = div_int(delta, i, inv_i);
-    if (!div_int_range(delta)) c = __ddiv_rn(delta, i);
-    st.x = __dadd_rn(st.x, c);
-    st.y = __dadd_rn(st.y, __dmul_rn(delta, __dsub_rn(x, st.x)));
-  }
-}
-
 // The tile's bootstraps b0 .. b0 + 2 np - 1 (the last one may not exist) at every point.
 template <int T, bool FUSED>
 __device__ __forceinline__ void vmr_points(int n, int np, int zt, int wt, int P, int b0, int nboot, double ns,
@@ -225,8 +169,7 @@ __device__ __forceinline__ void vmr_points(int n, int np, int zt, int wt, int P,
     for (int q = 0; q < np; ++q) {
       const double2 zv = z[2 * q], wv = w[2 * q];
       const int b = b0 + 2 * q;
-      vmr_update<FUSED>(zv.x, wv.x, ns, inv_ns, (double)(b + 1), recip[2 * q], st);
-      if (b + 1 < nboot) vmr_update<FUSED>(zv.y, wv.y, ns, inv_ns, (double)(b + 2), recip[2 * q + 1], st);
+      vmr_update2<FUSED>(zv, wv, ns, inv_ns, (double)(b + 1), recip[2 * q], recip[2 * q + 1], b + 1 < nboot, st);
     }
     state[x] = st;
   }
@@ -287,8 +230,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 4, LOGN == 10 ? 2 : 1)
       const double2 o = swap[((1 - h) * 4 + i) * P::NB8 + t];
       const double2 z = h ? o : v[i], w = h ? v[i + 4] : o;
       double2 st = make_double2(mean[i], m2[i]);
-      vmr_update<true>(z.x, w.x, 0.0, inv_ns, 0.0, inv_a, st);
-      if (has_b) vmr_update<true>(z.y, w.y, 0.0, inv_ns, 0.0, inv_b, st);
+      vmr_update2<true>(z, w, 0.0, inv_ns, 0.0, inv_a, inv_b, has_b, st);
       mean[i] = st.x;
       m2[i] = st.y;
     }
@@ -493,9 +435,11 @@ size_t steps1d_job_bytes() { return sizeof(Job1); }
 void steps1d_describe(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs, Steps1dPlan &plan) {
   plan = Steps1dPlan{};
   Job1 *hj = reinterpret_cast<Job1 *>(host_jobs);
-  // classes: the general kernel's three forms, then the power-of-two lengths 1024 and 2048
-  constexpr int NC = 5;
+  // classes: the general kernel's three forms, the power-of-two lengths 1024 and 2048, the lengths
+  // with a kernel of their own
+  constexpr int NC = 6;
   auto class_of = [](int n, const Shape1 &sh) {
+    if (steps1d_len_known(n)) return 5;
     if (n == 1024 || n == 2048) return n == 1024 ? 3 : 4;
     return sh.seq ? 2 : (sh.T == 512 ? 0 : 1);
   };
@@ -503,8 +447,11 @@ void steps1d_describe(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *h
   int(&first)[NC + 1] = plan.first, (&S)[NC] = plan.S;
   size_t(&smem)[NC] = plan.smem;
   int k = 0;
+  std::vector<int> order(count);
+  for (int e = 0; e < count; ++e) order[e] = e;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return args[x].n1 < args[y].n1; });
   for (int c = 0; c < NC; ++c) {  // the jobs of one kernel lie together
-    for (int e = 0; e < count; ++e) {
+    for (int e : order) {
       const Steps1dArgs &A = args[e];
       const Shape1 sh = shape1(A.n1, A.npairs);
       if (class_of(A.n1, sh) != c) continue;
@@ -537,6 +484,12 @@ void steps1d_describe(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *h
       J.f_out = A.f_out;
       J.mu_out = A.mu_out;
       J.nst = make_stages(ctx, A.n1, J.st);
+      if (c == NC - 1) {
+        if (plan.len.empty() || plan.len.back().n != A.n1) plan.len.push_back({A.n1, k, 0, 0});
+        auto &g = plan.len.back();
+        ++g.count;
+        g.S = std::max(g.S, A.S);
+      }
       hj[k++] = J;
     }
     first[c + 1] = k;
@@ -567,10 +520,18 @@ void steps1d_run(pkde_ctx *ctx, const Steps1dPlan &plan, const void *dev_jobs, c
   PKDE_P2(3, 10)
   PKDE_P2(4, 11)
 #undef PKDE_P2
+  for (const auto &g : plan.len) {
+    {
+      Trace tr(ctx, PKDE_PHASE_STEP_VMR, st);
+      steps1d_len_run(ctx, g.n, static_cast<const Job1 *>(dev_jobs) + g.first, g.count, g.S, st);
+    }
+    PKDE_CHECK_LAUNCH();
+  }
 }
 
 // Device bytes of the running state kept in global memory (0: in shared memory).
 size_t steps1d_state_bytes(int n1, int npairs, int64_t S) {
+  if (steps1d_len_known(n1)) return 0;
   return shape1(n1, npairs).seq ? sizeof(double2) * (size_t)n1 * (size_t)S : 0;
 }
 
