@@ -51,14 +51,14 @@ def workload(name, dims=None, samples=200_000):
 
 
 def measured_traffic(workload):
-    """DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one full-workload
-    engine launch, from the committed ncu summary of that kernel (profiles/); None if
+    """DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of all bandwidth steps of
+    the workload, from the committed ncu summary of the step kernels (profiles/); None if
     there is no capture for this workload."""
     import re
-    p = os.path.join(REPO, "profiles", f"engine_kernel_{workload}_ncu.md")
+    p = os.path.join(REPO, "profiles", f"chunk_kernels_{workload}_ncu.md")
     if not os.path.exists(p):
         return None
-    m = re.search(rf"dram_bytes_per_launch_full_{workload}:\s*([0-9.eE+]+)", open(p).read())
+    m = re.search(rf"dram_bytes_all_steps_{workload}:\s*([0-9.eE+]+)", open(p).read())
     return float(m.group(1)) if m else None
 
 
@@ -506,7 +506,7 @@ def main():
                      "frac": (achieved / peak) if achieved else None,
                      "traffic": measured_traffic(args.workload) if not small else None,
                      "algorithmic_bytes": alg_bytes,
-                     "kernel": "engine_kernel (persistent step engine: all bandwidth steps, one launch)",
+                     "kernel": "step kernels (inverse FFT passes, variance-to-mean rows, means and convergence of all bandwidth steps)",
                      "peak_source": peak_kind, "step_ms_per_estimation": step_ms,
                      "launches_per_estimation": step_launches},
         "phase_ms_per_estimation": dict(pstats["phase_ms"]),
@@ -607,7 +607,7 @@ def run_batched(args, world, rank, local, dist, record=False):
     lat_ms = sorted(a.elapsed_time(b) for a, b in lat)
     value = units * args.steps * world / (t_max / 1000.0)
     est_per_s = len(jobs) * args.steps * world / (t_max / 1000.0)
-    eng_ms = stats["phase_ms"]["step_vmr"] / args.steps
+    eng_ms = sum(stats["phase_ms"][q] for q in ("step_fft", "step_vmr", "step_means")) / args.steps
     achieved = alg_bytes / (eng_ms / 1000.0) / 1e9 if eng_ms > 0 else None
     peak, peak_kind = peaks()
 
@@ -682,7 +682,7 @@ def run_batched(args, world, rank, local, dist, record=False):
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None, "traffic": None,
-                     "kernel": "engine_kernel (all N-D estimations of the batch in one launch)",
+                     "kernel": "step kernels of all estimations of the batch",
                      "peak_source": peak_kind},
         "phase_ms_per_step": dict(pstats["phase_ms"]),
         "gpu_launches": stats["launches"],

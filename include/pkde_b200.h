@@ -229,10 +229,11 @@ int pkde_identify_convergence(pkde_ctx *ctx, int64_t G, double *density, const d
                               void *stream);
 
 /* How the bandwidth steps of an estimation are executed (a context setting).
- *   PKDE_STEPS_AUTO          : the persistent step engine for N-D grids with axes of
- *                              2..2048 points, one CTA per bandwidth step for 1-D
- *                              power-of-two grids of 256..4096 points, else per-step
- *                              kernel launches;
+ *   PKDE_STEPS_AUTO          : one CTA per bandwidth step for 1-D grids of up to 4096
+ *                              points, one launch per FFT pass and chunk of steps for
+ *                              N-D grids with axes of up to 1024 points, the persistent
+ *                              step engine for axes of up to 2048, else per-step kernel
+ *                              launches;
  *   PKDE_STEPS_PER_STEP_LAUNCH: every estimation on the plain form -- per bandwidth step
  *                              and pair group, one kernel launch per FFT axis, then the
  *                              VMR and the means/convergence launches, estimations one
@@ -246,13 +247,14 @@ int pkde_identify_convergence(pkde_ctx *ctx, int64_t G, double *density, const d
 int pkde_set_step_path(pkde_ctx *ctx, int path);
 
 /* Autotuning of the step engine's schedule per shape (grid dimensions and bootstrap
- * pairs): the first estimation of a new shape times trial runs over its first 16
+ * pairs) where the engine runs it: the first estimation of a new shape times trial runs over its first 16
  * bandwidth steps for ring-slot sizes 8..64 MB, slots holding half or all of the
  * bootstrap pairs where those are larger (while the ring stays within an eighth of the
  * free device memory; the context keeps the largest ring it tried), 1..8 tiles per
  * work item and pipeline delays 2..4, and keeps the fastest for the context (and, when
  * the environment variable PKDE_TUNE_CACHE names a file, appends it there and reads it
- * back in later processes).  A batch whose tuned rings together would not fit in half
+ * back in later processes; shapes whose steps run in chunks are recorded as 0 0 0, and a
+ * schedule that the file holds for a shape puts that shape into the engine).  A batch whose tuned rings together would not fit in half
  * of the free memory runs with slots of at most 64 MB.  The schedule never changes
  * results, only time.  On by default; 0 uses the fixed defaults (32 MB, 2 or 8 tiles,
  * delay 2).  No counterpart in the reference. */
@@ -262,7 +264,8 @@ int pkde_set_autotune(pkde_ctx *ctx, int enable);
  * step engine (a work item waiting for the items it reads from) polls a counter at most
  * `polls` times (about 0.1 us each) before it gives up: it then sets the launch's error
  * flag, every CTA leaves, and the call returns PKDE_ECUDA ("step engine: a dependency
- * wait timed out").  The context stays usable.  Default 20,000,000 (about 1-2 s);
+ * wait timed out").  The context stays usable.  Default 20,000,000 (about 1-2 s); with
+ * any other limit the engine runs every N-D estimation it can, so that the limit applies;
  * polls >= 0 (0: give up at the first check that finds the dependency not ready).
  * No counterpart in the reference, which has no waits that can time out (its
  * failures are ArgumentErrors, DirectSpace.jl:479-512). */

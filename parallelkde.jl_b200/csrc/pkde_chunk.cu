@@ -12,7 +12,8 @@
 // The steps are independent given the spectra, so a chunk has no ordering inside it: the
 // launches need no dependency counters, and every axis length fills its tiles (2048
 // points, as many lines as fit, lines of different arrays and steps side by side).
-// The persistent engine (pkde_engine.cu) keeps the shapes whose tiles it fills itself.
+// These kernels take any length; powers of two (pkde_chunk_pow2.cu) and other 2^a 3^b 5^c lengths
+// (pkde_chunk_len.cuh) have their own.  The persistent engine (pkde_engine.cu) keeps longer axes.
 #include <algorithm>
 #include <cstring>
 
@@ -555,12 +556,12 @@ ChunkShape chunk_shape(int64_t G, int npairs, int S, int level) {
 
 }  // namespace
 
-// Grids this path takes.  Against the persistent engine (step times): its shared-memory tiles hold
-// few lines of a length that is not 2^m, 3 2^m or 5 2^m (100 x 100, 100 bootstraps, 250 steps: 66
-// ms, here 4.3; 50 x 41 x 36, 32, 100: 148 and 11.7); its mixed-radix tiles leave a quarter of the
-// threads idle (96^3, 32, 100: 97 and 69); on a small grid a step has too few tiles for its order
-// of items (64 x 64, 33, 40: 2.0 and 0.4); on large powers of two it waits for dependencies and
-// spills (512 x 512, 64, 200: 52.7 and 43.4; 128^3, 32, 150: 199 and 182).  It keeps axes of
+// Grids this path takes.  Against the persistent engine (whole calls, then here): its shared-memory
+// tiles hold few lines of a length that is not 2^m, 3 2^m or 5 2^m (100 x 100, 100 bootstraps, 250
+// steps: 67 ms, 3.6; 50 x 41 x 36, 32, 100: 149 and 8.7); its mixed-radix tiles leave a quarter of the
+// threads idle (96^3, 32, 100: 100 and 51); on a small grid a step has too few tiles for its order
+// of items (64 x 64, 33, 40: 1.8 and 0.33); on large powers of two it waits for dependencies and
+// spills (512 x 512, 64, 200: 57.5 and 37.2; 128^3, 32, 150: 219 and 161).  It keeps axes of
 // 1025 to 2048 points, and runs where a schedule file or a wait limit of its own asks for it.
 bool chunk_ok(const pkde_grid *g) {
   if (g->ndim < 2) return false;

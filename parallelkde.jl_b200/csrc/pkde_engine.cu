@@ -1,5 +1,5 @@
-// Persistent dataflow engine for the per-bandwidth-step work of an N-D (N >= 2)
-// estimation on power-of-two axes of 16..2048 points.
+// Persistent dataflow engine for the per-bandwidth-step work of N-D (N >= 2) estimations: axes of
+// more than 1024 points, and shapes or contexts that ask for it (pkde_chunk.cu runs the others).
 //
 // Work: for every step s the inverse FFT of all bootstrap pairs (z, w arrays) and of the
 // full-sample means, then VMR + Welford over bootstraps, then the convergence update.

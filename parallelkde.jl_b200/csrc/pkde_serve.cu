@@ -55,7 +55,7 @@ struct Server {
 
 // Upper bound of the device memory one request needs inside a wave: samples, indices,
 // outputs, paired spectra, convergence state, factor tables, binning scratch, 1-D
-// per-step arrays and the step engine's ring slots and counters.
+// per-step arrays and the chunk scratch or the step engine's ring slots and counters.
 size_t footprint(const pkde_gradepro_params *p, int64_t n, bool has_idx) {
   const int N = p->grid.ndim;
   int64_t G = 1, axes = 0;

@@ -182,7 +182,8 @@ __device__ __forceinline__ void vmr_points(int n, int np, int zt, int wt, int P,
 // general kernel's threads would idle in its radix-8 stages.  Bound by the latency of
 // its shared-memory exchanges and dependent FP64 operations (40 % of the issue slots at 16 warps
 // an SM).  1,024 points, 250 steps, 100 bootstraps: 0.30 ms with z and w one after the other in
-// half the threads, 0.42 ms in the general kernel, 0.27 ms here.
+// half the threads, 0.42 ms in the general kernel, 0.27 ms here, 0.23 since a NaN mean skips the IEEE
+// division.
 template <int LOGN>
 __global__ void __launch_bounds__((1 << LOGN) / 4, LOGN == 10 ? 2 : 1)
     steps1d_pow2_kernel(const Job1 *jobs, const double2 *__restrict__ tw_g) {
@@ -261,7 +262,8 @@ constexpr int kPairs = 64;  // pairs per tile at most
 // stages; two tiles instead of one that is rewritten in place keep a thread's registers at one
 // butterfly, so 32 warps share an SM (in place, with 128 registers: 16 warps, 1.4x the time).
 // 250 steps, 100 bootstraps, against one launch per step and pass of a single CTA each (the
-// plain form, which has the same bits): 500 points 113 -> 0.32 ms, 2500 points 366 -> 1.65 ms.
+// plain form, which has the same bits): 3460 points (4 x 5 x 173) 2947 -> 22 ms.  Lengths without other
+// prime factors than 2, 3 and 5 have pkde_steps1d_len.cuh.
 // Shared memory: tiles a and b of n P units each; with SEQ a third one; the running
 // (mean, m2) of every point where it fits (J.state null), else in global memory.
 // SEQ: the z and the w line of a pair one after the other (lines too long for both).
