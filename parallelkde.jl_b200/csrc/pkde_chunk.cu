@@ -872,11 +872,13 @@ void run_chunk(pkde_ctx *ctx, const ChunkArgs *args, int count, char *const *scr
     }
     PKDE_CHECK_LAUNCH();
   }
+  std::vector<ConvergeJob> walks;
   for (int e = 0; e < count; ++e) {
     const ChunkArgs &A = args[e];
     if (plan[e].c.all_steps)
-      converge_steps(ctx, plan[e].run.G, A.S, plan[e].f, plan[e].mu, A.dlogt, A.eps, A.steps_low, A.steps_over, A.cs, st);
+      walks.push_back({plan[e].run.G, A.steps_low, A.steps_over, plan[e].f, plan[e].mu, A.dlogt, A.eps, A.S, A.cs});
   }
+  converge_steps(ctx, walks, st);
 }
 
 }  // namespace pkde

@@ -1063,13 +1063,15 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   // 1-D estimations: every bandwidth step of all of them in one launch, then the
   // convergence state machine over the stored per-step f_s and means
   steps1d_run(ctx, lplan, base + off_rjobs, st);
+  std::vector<ConvergeJob> walks;
   for (int e = 0; e < count; ++e) {
     Plan &P = plans[e];
     if (P.path != StepPath::Steps1D) continue;
     const int64_t S = P.L.S;
-    converge_steps(ctx, P.G, (int)S, P.per_step, P.per_step + S * P.G, P.d_scal + 2 * S, P.L.eps, P.L.steps_low,
-                   P.L.steps_over, P.cs, st);
+    walks.push_back({P.G, P.L.steps_low, P.L.steps_over, P.per_step, P.per_step + S * P.G, P.d_scal + 2 * S, P.L.eps,
+                     (int)S, P.cs});
   }
+  converge_steps(ctx, walks, st);
   // two persistent launches: estimations whose axes all take the register power-of-two
   // tiles run in the lean kernel instantiation, the others in the one with the
   // mixed-radix and shared-memory tiles (more registers spilled)

@@ -197,8 +197,14 @@ struct Steps1dPlan {
 void steps1d_describe(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs, Steps1dPlan &plan);
 void steps1d_run(pkde_ctx *ctx, const Steps1dPlan &plan, const void *dev_jobs, cudaStream_t st);
 // The convergence state machine over all steps (density and selected step of every point).
-void converge_steps(pkde_ctx *ctx, int64_t G, int S, const double *f_all, const double *mu_all, const double *dlogt,
-                    double eps, int64_t steps_low, int64_t steps_over, const StepState &cs, cudaStream_t st);
+struct ConvergeJob {
+  int64_t G, steps_low, steps_over;
+  const double *f, *mu, *dlogt;  // f and means of every step, S x G
+  double eps;
+  int S;
+  StepState cs;
+};
+void converge_steps(pkde_ctx *ctx, const std::vector<ConvergeJob> &jobs, cudaStream_t st);
 
 // power-of-two path (pkde_step.cu)
 bool pow2_path_ok(const pkde_grid *g);
