@@ -228,7 +228,11 @@ int pkde_identify_convergence(pkde_ctx *ctx, int64_t G, double *density, const d
                               uint16_t *counters_over, uint8_t *low_density_flags, uint32_t flags,
                               void *stream);
 
-/* How the bandwidth steps of an estimation are executed (a context setting).
+/* How the bandwidth steps of an estimation are executed (a context setting).  Chunks of steps hold up
+ * to 8 GB of intermediates and up to 8 GB of results of all steps, which the context keeps; less where
+ * that exceeds half of the free memory or the MB that the environment variable PKDE_RING_BUDGET_MB
+ * names (64 MB and 32 MB are always allowed), and 256 MB and 128 MB in serving lanes and in contexts whose
+ * autotuning is off.  The limits never change results.
  *   PKDE_STEPS_AUTO          : one CTA per bandwidth step for 1-D grids of up to 4096
  *                              points, one launch per FFT pass and chunk of steps for
  *                              N-D grids with axes of up to 1024 points, the persistent
@@ -278,9 +282,13 @@ int pkde_set_wait_limit(pkde_ctx *ctx, int64_t polls);
  *   of every estimation and the copy of its error flags have been queued, before the
  *   forward transforms -- the call fails with device work in flight and flags
  *   outstanding, which the context's next call must wait for and discard.
+ *   PKDE_FAULT_SCRATCH_ALLOC: in the same calls, the allocation of the chunked steps' scratch
+ *   reports that the device is out of memory (as when another user of it takes the memory
+ *   between the query and the allocation); the call goes on with smaller chunks.
  * No counterpart in the reference. */
 #define PKDE_FAULT_NONE 0
 #define PKDE_FAULT_AFTER_BINNING 1
+#define PKDE_FAULT_SCRATCH_ALLOC 2
 int pkde_set_fault(pkde_ctx *ctx, int32_t point);
 
 /* Diagnostic: out[i] = num[i] / den[i] with the quotient the step engine uses for the

@@ -103,7 +103,7 @@ int pkde_set_wait_limit(pkde_ctx *ctx, int64_t polls) {
 
 int pkde_set_fault(pkde_ctx *ctx, int32_t point) {
   if (!ctx) return PKDE_EINVAL;
-  if (point != PKDE_FAULT_NONE && point != PKDE_FAULT_AFTER_BINNING) {
+  if (point != PKDE_FAULT_NONE && point != PKDE_FAULT_AFTER_BINNING && point != PKDE_FAULT_SCRATCH_ALLOC) {
     pkde::thread_error(ctx) = "unknown fault point";
     return PKDE_EINVAL;
   }

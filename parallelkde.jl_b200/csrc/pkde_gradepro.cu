@@ -540,15 +540,19 @@ static void check_binning_flags(pkde_ctx *ctx) {
   }
 }
 
-// Scratch that the estimations of a batch call may hold together in buffer `id`: half of the
-// free memory, capped by PKDE_RING_BUDGET_MB (tests use it to force one launch per estimation).
+// PKDE_RING_BUDGET_MB: bytes that a process with other users of the device's memory allows for the
+// scratch of a call's bandwidth steps (tests use it to force one launch per estimation).
+static size_t budget_cap() {
+  const char *cap = getenv("PKDE_RING_BUDGET_MB");
+  return cap && *cap ? (size_t)std::max(0LL, atoll(cap)) << 20 : SIZE_MAX;
+}
+
+// Scratch that the estimations of a call may hold together in buffer `id`: half of the free
+// memory, at most the cap.
 static size_t shared_budget(pkde_ctx *ctx, BufId id) {
   size_t freeb = 0, totalb = 0;
   PKDE_CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
-  size_t budget = (freeb + ctx->buf[id].bytes) / 2;
-  if (const char *cap = getenv("PKDE_RING_BUDGET_MB"); cap && *cap)
-    budget = std::min(budget, (size_t)std::max(0LL, atoll(cap)) << 20);
-  return budget;
+  return std::min((freeb + ctx->buf[id].bytes) / 2, budget_cap());
 }
 
 // One estimation of a call (device pointers).
@@ -830,12 +834,11 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
   }
   char *base = (char *)ensure(ctx, BUF_BATCH, arena);
   // estimations in chunks of steps share launches as far as their scratch together fits the
-  // memory budget: chunk_group[i] = first of the i-th set
+  // memory budget: chunk_group[i] = first of the i-th set.  The level rises until the largest one's
+  // scratch fits the budget (the cap alone: to kCapLevel), and where an allocation fails.
   std::vector<size_t> chunk_group{0};
-  int chunk_level = ctx->tune_wide ? 0 : kServeLevel;
-  if (!chunk_e.empty()) {
-    // the device's free memory is asked for only where the kept scratch does not suffice
-    size_t budget = chunk_e.size() > 1 ? shared_budget(ctx, BUF_SCRATCH) : ctx->buf[BUF_SCRATCH].bytes;
+  int chunk_level = ctx->tune_wide && ctx->autotune ? 0 : kServeLevel;
+  auto group_chunks = [&] {
     auto largest = [&] {
       size_t most = 0;
       for (size_t i = 0; i < chunk_e.size(); ++i) {
@@ -845,15 +848,17 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
       }
       return most;
     };
-    size_t most = largest();
-    if (most > budget) {
-      size_t freeb = 0, totalb = 0;
-      PKDE_CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
-      while (chunk_level + 1 < kChunkLevels && most > (freeb + ctx->buf[BUF_SCRATCH].bytes) / 2) {
+    size_t most = largest(), budget = std::min(ctx->buf[BUF_SCRATCH].bytes, budget_cap());
+    // the device's free memory is asked for only where the kept scratch does not suffice
+    if (chunk_e.size() > 1 || most > budget) {
+      budget = shared_budget(ctx, BUF_SCRATCH);
+      while (chunk_level + 1 < kChunkLevels && most > budget && (chunk_level < kCapLevel || budget < budget_cap())) {
         ++chunk_level;
         most = largest();
       }
     }
+    chunk_group.assign(1, 0);
+    chunk_scr = 0;
     size_t need = 0;
     for (size_t i = 0; i < chunk_e.size(); ++i) {
       if (i > chunk_group.back() && need + chunk_bytes[i] > budget) {
@@ -864,11 +869,22 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
       chunk_scr = std::max(chunk_scr, need);
     }
     chunk_group.push_back(chunk_e.size());
+  };
+  if (!chunk_e.empty()) group_chunks();
+  while (generic_scr || chunk_scr) {  // sized once, so that no buffer grows while kernels are queued
+    try {
+      if (chunk_scr) fault_point(ctx, PKDE_FAULT_SCRATCH_ALLOC, PKDE_ENOMEM);
+      ensure(ctx, BUF_SCRATCH, std::max(generic_scr, chunk_scr));
+      break;
+    } catch (const Error &err) {
+      // the memory went to another user since it was asked for: smaller chunks need less
+      if (err.code != PKDE_ENOMEM || !chunk_scr || chunk_level + 1 == kChunkLevels) throw;
+      cudaGetLastError();
+      ++chunk_level;
+      group_chunks();
+    }
   }
-  if (generic_scr || chunk_scr) {  // sized once, so that no buffer grows while kernels are queued
-    ensure(ctx, BUF_SCRATCH, std::max(generic_scr, chunk_scr));
-    ensure(ctx, BUF_WELFORD, generic_wel);
-  }
+  if (generic_wel) ensure(ctx, BUF_WELFORD, generic_wel);
   std::vector<size_t> toffs(count);
   size_t toff = 0;
   for (int e = 0; e < count; ++e) {

@@ -635,10 +635,10 @@ struct DrainOnError {
 };
 
 // Host-side fault injection (pkde_set_fault): throws once at the armed point.
-inline void fault_point(pkde_ctx *ctx, int point) {
+inline void fault_point(pkde_ctx *ctx, int point, int code = PKDE_ECUDA) {
   if (ctx->fault_point == point) {
     ctx->fault_point = PKDE_FAULT_NONE;
-    throw Error{PKDE_ECUDA, "injected host fault (pkde_set_fault)"};
+    throw Error{code, "injected host fault (pkde_set_fault)"};
   }
 }
 

@@ -160,8 +160,11 @@ struct ChunkArgs {
 bool chunk_ok(const pkde_grid *g);
 // Whether an estimation that chunk_ok takes runs in chunks (a schedule file may say otherwise).
 bool chunk_schedule(pkde_ctx *ctx, const pkde_grid *g, int npairs);
-// Scratch at a memory level (0: the largest chunks .. kChunkLevels - 1).
-constexpr int kChunkLevels = 4, kServeLevel = 2;
+// Scratch at a memory level (0: the largest chunks .. kChunkLevels - 1).  Serving lanes, and contexts
+// that leave the choice of buffer sizes to fixed defaults (pkde_set_autotune), start at kServeLevel;
+// PKDE_RING_BUDGET_MB lowers to kCapLevel at most, whose scratch is always allowed, as ring slots of
+// kNarrowSlotMB are.
+constexpr int kChunkLevels = 6, kServeLevel = 3, kCapLevel = 4;
 size_t chunk_scratch_bytes(const pkde_grid *g, int npairs, int S, int level);
 // Whether density and selected step come out final (else the caller initialises the state
 // before and fills the points without a selected step after).

@@ -196,7 +196,7 @@ def set_wait_limit(polls, device=0):
     check(load().pkde_set_wait_limit(ctx, int(polls)), ctx)
 
 
-PKDE_FAULT_NONE, PKDE_FAULT_AFTER_BINNING = 0, 1
+PKDE_FAULT_NONE, PKDE_FAULT_AFTER_BINNING, PKDE_FAULT_SCRATCH_ALLOC = 0, 1, 2
 
 
 def set_fault(point, device=0):
