@@ -258,7 +258,8 @@ int pkde_set_step_path(pkde_ctx *ctx, int path);
  * work item and pipeline delays 2..4, and keeps the fastest for the context (and, when
  * the environment variable PKDE_TUNE_CACHE names a file, appends it there and reads it
  * back in later processes; shapes whose steps run in chunks are recorded as 0 0 0, and a
- * schedule that the file holds for a shape puts that shape into the engine).  A batch whose tuned rings together would not fit in half
+ * schedule that the file holds for such a shape is used only where the engine runs it,
+ * see pkde_set_wait_limit).  A batch whose tuned rings together would not fit in half
  * of the free memory runs with slots of at most 64 MB.  The schedule never changes
  * results, only time.  On by default; 0 uses the fixed defaults (32 MB, 2 or 8 tiles,
  * delay 2).  No counterpart in the reference. */

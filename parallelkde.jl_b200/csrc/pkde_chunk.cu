@@ -564,7 +564,7 @@ ChunkShape chunk_shape(int64_t G, int npairs, int S, int level) {
 // threads idle (96^3, 32, 100: 100 and 51); on a small grid a step has too few tiles for its order
 // of items (64 x 64, 33, 40: 1.8 and 0.33); on large powers of two it waits for dependencies and
 // spills (512 x 512, 64, 200: 57.5 and 37.2; 128^3, 32, 150: 219 and 161).  It keeps axes of
-// 1025 to 2048 points, and runs where a schedule file or a wait limit of its own asks for it.
+// 1025 to 2048 points, and the contexts with a wait limit of their own.
 bool chunk_ok(const pkde_grid *g) {
   if (g->ndim < 2) return false;
   const int64_t G = grid_size(g);

@@ -1386,7 +1386,10 @@ static void load_tune_file(pkde_ctx *ctx) {
   if (!f) return;
   char key[256];
   int a, b, c;
-  while (fscanf(f, "%255s %d %d %d", key, &a, &b, &c) == 4) ctx->tune[key] = {a, b, c};
+  while (fscanf(f, "%255s %d %d %d", key, &a, &b, &c) == 4) {
+    if (a) ctx->tune[key] = {a, b, c};
+    else ctx->chunk_recorded.insert(key);
+  }
   fclose(f);
 }
 
@@ -1399,18 +1402,15 @@ static void save_tune(pkde_ctx *ctx, const std::string &key, const std::array<in
   fclose(f);
 }
 
-// A shape's schedule may also be "in chunks of steps" (0 0 0), which the rule of chunk_ok
-// chooses without trials.  An engine schedule in the file for such a shape is kept.
-bool chunk_schedule(pkde_ctx *ctx, const pkde_grid *g, int npairs) {
+// A shape whose steps run in chunks is recorded as 0 0 0, once, where the file says nothing about it
+// (the record is for its reader: what the file holds never chooses between chunks and the
+// engine, whose own trials write to it too).
+void record_chunked(pkde_ctx *ctx, const pkde_grid *g, int npairs) {
+  if (!ctx->autotune) return;
   load_tune_file(ctx);
   const std::string key = tune_key(g, npairs);
-  auto it = ctx->tune.find(key);
-  if (it != ctx->tune.end()) return it->second[0] == 0 || !engine_ok(g);
-  if (ctx->autotune) {
-    ctx->tune[key] = {0, 0, 0};
-    save_tune(ctx, key, {0, 0, 0});
-  }
-  return true;
+  if (ctx->tune.count(key) || !ctx->chunk_recorded.insert(key).second) return;
+  save_tune(ctx, key, {0, 0, 0});
 }
 
 void autotune_engine(pkde_ctx *ctx, EngineArgs &A, cudaStream_t st) {

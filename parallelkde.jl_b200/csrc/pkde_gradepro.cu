@@ -785,9 +785,10 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
     // a wait limit of the caller's bounds the engine's waits: the steps stay where it applies
     const bool own_limit = ctx->wait_limit != kDefaultWaitLimit && engine_ok(P.g);
     if (steps1d_ok(P.g)) P.path = StepPath::Steps1D;
-    else if (chunk_ok(P.g) && !own_limit && chunk_schedule(ctx, P.g, (int)P.npairs)) P.path = StepPath::Chunk;
+    else if (chunk_ok(P.g) && !own_limit) P.path = StepPath::Chunk;
     else P.path = engine_ok(P.g) ? StepPath::Engine : StepPath::Generic;
     if (ctx->step_path == PKDE_STEPS_PER_STEP_LAUNCH) P.path = StepPath::Generic;
+    if (P.path == StepPath::Chunk) record_chunked(ctx, P.g, (int)P.npairs);
     tables_bytes += al256(sizeof(double) * 2 * P.L.S * P.tot);
   }
   std::vector<size_t> off_zero(count);

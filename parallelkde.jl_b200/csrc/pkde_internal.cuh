@@ -12,6 +12,7 @@
 #include <exception>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -126,6 +127,7 @@ struct pkde_ctx {
   bool recip_ready = false;  // the step engine's table of 1/i is in this device's constant memory
   pkde::DevBuf chunk_recip;  // the chunked steps' table of 1/i
   std::map<std::string, std::array<int, 3>> tune;
+  std::set<std::string> chunk_recorded;  // shapes that the schedule file names as run in chunks
   // polls a step-engine dependency wait makes before it gives up (pkde_set_wait_limit)
   int64_t wait_limit = pkde::kDefaultWaitLimit;
   // host-side fault injection for tests (pkde_set_fault): one-shot

@@ -158,8 +158,8 @@ struct ChunkArgs {
   StepState cs;
 };
 bool chunk_ok(const pkde_grid *g);
-// Whether an estimation that chunk_ok takes runs in chunks (a schedule file may say otherwise).
-bool chunk_schedule(pkde_ctx *ctx, const pkde_grid *g, int npairs);
+// Names an estimation's shape in the schedule file as one that runs in chunks.
+void record_chunked(pkde_ctx *ctx, const pkde_grid *g, int npairs);
 // Scratch at a memory level (0: the largest chunks .. kChunkLevels - 1).  Serving lanes, and contexts
 // that leave the choice of buffer sizes to fixed defaults (pkde_set_autotune), start at kServeLevel;
 // PKDE_RING_BUDGET_MB lowers to kCapLevel at most, whose scratch is always allowed, as ring slots of
