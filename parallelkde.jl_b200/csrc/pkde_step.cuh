@@ -189,7 +189,7 @@ size_t steps1d_job_bytes();
 size_t steps1d_state_bytes(int n1, int npairs, int64_t S);
 // Descriptors (count x steps1d_job_bytes()) and launches of several estimations.
 struct Steps1dPlan {
-  static constexpr int kClasses = 6;  // kernels
+  static constexpr int kClasses = 7;  // kernels
   int first[kClasses + 1], S[kClasses];
   size_t smem[kClasses];
   struct Len {

@@ -256,6 +256,57 @@ __global__ void __launch_bounds__((1 << LOGN) / 4, LOGN == 10 ? 2 : 1)
   }
 }
 
+// Power-of-two lines of which z and w do not fit side by side (4096 points: 74 KB each beside 65 KB of
+// twiddles): z, then w in register tiles of n / 8 threads, both transforms of a thread's eight points in
+// registers.  4096 points, 250 steps, 100 bootstraps, whole calls: 2.09 ms in the general kernel, whose running
+// variance is in memory there, 1.20 here.
+template <int LOGN>
+__global__ void __launch_bounds__((1 << LOGN) / 8, 1)
+    steps1d_line_kernel(const Job1 *jobs, const double2 *__restrict__ tw_g) {
+  using P = Pow2<LOGN, 1>;
+  double2 *tile = sm1, *sm_tw = sm1 + P::TILE;
+  const Job1 &J = jobs[blockIdx.y];
+  const int s = blockIdx.x, t = threadIdx.x;
+  if (s >= J.S) return;
+  for (int i = t; i < P::TWSIZE; i += P::THREADS) sm_tw[i] = tw_g[i];
+  const double *fz = J.fz + s * J.tab_stride, *fw = J.fw + s * J.tab_stride;
+  const double cz = J.invG, cw = J.invG * J.cw[s], inv_ns = J.inv_ns;
+  const int nboot = J.nboot, npairs = J.npairs;
+  double2 st[8];  // points out_pos(t, i)
+#pragma unroll
+  for (int i = 0; i < 8; ++i) st[i] = make_double2(0.0, 0.0);
+  auto transform = [&](int64_t line, const double *f, double c, double2(&v)[8]) {
+    const double2 *in = J.spectra + line * P::N;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const int k = in_pos<LOGN>(t, r);
+      v[r] = cscale(__ldg(in + k), c * __ldg(f + k));
+    }
+    tile_fft_reg<LOGN, 1, false, 1>(tile, v, sm_tw);
+  };
+  __syncthreads();
+  for (int p = 0; p < npairs; ++p) {
+    double2 z[8], w[8];
+    transform(2 * p, fz, cz, z);
+    transform(2 * p + 1, fw, cw, w);
+    const int b = 2 * p;
+    const double inv_a = 1.0 / (double)(b + 1), inv_b = 1.0 / (double)(b + 2);
+    const bool has_b = b + 1 < nboot;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) vmr_update2<true>(z[i], w[i], 0.0, inv_ns, 0.0, inv_a, inv_b, has_b, st[i]);
+  }
+  double2 v[8];
+  transform(2 * npairs, fz, cz, v);
+  const double vs = J.vscale[s], bm1 = (double)(nboot - 1);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int x = out_pos<LOGN>(t, i);
+    const double var = __ddiv_rn(__dmul_rn(vs, st[i].y), bm1);
+    J.f_out[(int64_t)s * P::N + x] = isfinite(var) ? log(var) : nan("");
+    J.mu_out[(int64_t)s * P::N + x] = sqrt(__fma_rn(v[i].x, v[i].x, __dmul_rn(v[i].y, v[i].y)));
+  }
+}
+
 constexpr int kPairs = 64;  // pairs per tile at most
 
 // Any length.  Bound by instruction issue (about a third FP64) and the barriers between the
@@ -448,12 +499,14 @@ size_t steps1d_job_bytes() { return sizeof(Job1); }
 void steps1d_describe(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs, Steps1dPlan &plan) {
   plan = Steps1dPlan{};
   Job1 *hj = reinterpret_cast<Job1 *>(host_jobs);
-  // classes: the general kernel's three forms, the power-of-two lengths 1024 and 2048, the lengths
-  // with a kernel of their own
-  constexpr int NC = 6;
+  // classes: the general kernel's three forms, the power-of-two lengths 1024, 2048 and 4096, the
+  // lengths with a kernel of their own.  Register tiles of 256 points lose to the general kernel where the
+  // steps do not fill the SMs (100 bootstraps, 50 steps: 0.092 ms and 0.072; 250: 0.095 and 0.101).  Of 512
+  // they take less time (250: 0.119 and 0.176), but the density's last bit is another one.
+  constexpr int NC = 7;
   auto class_of = [](int n, const Shape1 &sh) {
-    if (steps1d_len_known(n)) return 5;
-    if (n == 1024 || n == 2048) return n == 1024 ? 3 : 4;
+    if (steps1d_len_known(n)) return 6;
+    if (n == 1024 || n == 2048 || n == 4096) return n == 1024 ? 3 : n == 2048 ? 4 : 5;
     return sh.seq ? 2 : (sh.T == 512 ? 0 : 1);
   };
   static_assert(NC == Steps1dPlan::kClasses, "classes");
@@ -533,6 +586,8 @@ void steps1d_run(pkde_ctx *ctx, const Steps1dPlan &plan, const void *dev_jobs, c
   PKDE_P2(3, 10)
   PKDE_P2(4, 11)
 #undef PKDE_P2
+  launch(5, Pow2<12, 1>::THREADS, sizeof(double2) * (Pow2<12, 1>::TILE + Pow2<12, 1>::TWSIZE), steps1d_line_kernel<12>,
+         stage_twiddles_device(ctx, 12));
   for (const auto &g : plan.len) {
     {
       Trace tr(ctx, PKDE_PHASE_STEP_VMR, st);
@@ -544,7 +599,7 @@ void steps1d_run(pkde_ctx *ctx, const Steps1dPlan &plan, const void *dev_jobs, c
 
 // Device bytes of the running state kept in global memory (0: in shared memory).
 size_t steps1d_state_bytes(int n1, int npairs, int64_t S) {
-  if (steps1d_len_known(n1)) return 0;
+  if (steps1d_len_known(n1) || n1 == 4096) return 0;
   return shape1(n1, npairs).seq ? sizeof(double2) * (size_t)n1 * (size_t)S : 0;
 }
 
