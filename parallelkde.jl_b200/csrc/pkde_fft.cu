@@ -14,7 +14,7 @@
 namespace pkde {
 namespace {
 
-constexpr int kFftThreads = 256, kMostLines = 16;
+constexpr int kFftThreads = 256;
 
 template <int DIR>
 __global__ void __launch_bounds__(kFftThreads) fft_axis_kernel(const double2 *in, double2 *out,
@@ -31,10 +31,15 @@ __global__ void __launch_bounds__(kFftThreads) fft_axis_kernel(const double2 *in
   const int nl = (int)min((int64_t)tl, nlines - L0);
   const bool contiguous = ls.inner == 1;
   const int64_t per_array = ls.inner * ls.outer;
-  // the 64-bit divisions once a line, not an element (128^3, 33 arrays, three axes: 3.9 -> 3.2 ms)
-  __shared__ int64_t base[kMostLines];
-  if (threadIdx.x < nl) base[threadIdx.x] = ls.base(L0 + threadIdx.x);
-  __syncthreads();
+  // element k of line L at L + (L / inner) (n - 1) inner + k inner (axis_lines: arrays follow one another): one
+  // 64-bit division a tile (128^3, 33 arrays, three axes: 3.6 ms with those of LineSet::base an element, 2.9
+  // with its results a line in shared memory, which cost 24^4 5 % and 997 points 15 %, 2.5 here)
+  const int64_t o0 = L0 / ls.inner, skip = (int64_t)(n - 1) * ls.inner, base = L0 + o0 * skip;
+  const unsigned inner = (unsigned)ls.inner, i0 = (unsigned)(L0 - o0 * ls.inner);
+  auto at = [&](int l, int k) {
+    const unsigned o = contiguous ? l : (i0 + l) / inner;
+    return base + l + o * skip + (int64_t)k * ls.inner;
+  };
 
   for (int e = threadIdx.x; e < nl * n; e += kFftThreads) {
     int l, k;
@@ -45,10 +50,9 @@ __global__ void __launch_bounds__(kFftThreads) fft_axis_kernel(const double2 *in
       k = e / nl;
       l = e - k * nl;
     }
-    double2 v = in[base[l] + (int64_t)k * ls.inner];
+    double2 v = in[at(l, k)];
     if (nfac) {
-      const int64_t a = (L0 + l) / per_array;
-      const bool second = nfac == 2 && (a & 1);
+      const bool second = nfac == 2 && ((L0 + l) / per_array & 1);
       const double *f = second ? f1 : f0;
       const double sc = (second ? s1 : s0) * (f ? f[k] : 1.0);
       v = cscale(v, sc);
@@ -66,7 +70,7 @@ __global__ void __launch_bounds__(kFftThreads) fft_axis_kernel(const double2 *in
       k = e / nl;
       l = e - k * nl;
     }
-    out[base[l] + (int64_t)k * ls.inner] = res[l * pitch + k];
+    out[at(l, k)] = res[l * pitch + k];
   }
 }
 
@@ -85,7 +89,7 @@ const double2 *twiddles_device(pkde_ctx *ctx, int n) {
 // Lines per CTA: enough to fill ~2048 elements, capped by the shared-memory budget.
 int lines_per_cta(int n, int64_t nlines) {
   int tl = std::max(1, 2048 / n);
-  if (tl > kMostLines) tl = kMostLines;
+  if (tl > 16) tl = 16;
   if (tl > nlines) tl = (int)nlines;
   return std::max(tl, 1);
 }
