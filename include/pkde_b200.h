@@ -231,8 +231,8 @@ int pkde_identify_convergence(pkde_ctx *ctx, int64_t G, double *density, const d
 /* How the bandwidth steps of an estimation are executed (a context setting).  Chunks of steps hold up
  * to 8 GB of intermediates and up to 8 GB of results of all steps, which the context keeps; less where
  * that exceeds half of the free memory or the MB that the environment variable PKDE_RING_BUDGET_MB
- * names (64 MB and 32 MB are always allowed), and 256 MB and 128 MB in serving lanes and in contexts whose
- * autotuning is off.  The limits never change results.
+ * names (256 MB and 128 MB are always allowed), and those in serving lanes and in contexts whose autotuning
+ * is off.  The limits never change results.
  *   PKDE_STEPS_AUTO          : one CTA per bandwidth step for 1-D grids of up to 4096
  *                              points, one launch per FFT pass and chunk of steps for
  *                              N-D grids with axes of up to 1024 points, the persistent

@@ -534,12 +534,12 @@ struct ChunkShape {
 // larger the chunk the fewer launches drain the SMs, and the more steps share a reading of the
 // spectra; that its intermediates leave the L2 costs less (100 x 100, 100 bootstraps, 250 steps, with
 // 64 MB / 256 MB / 1 GB / 8 GB: 9.5 / 6.9 / 4.9 / 4.7 ms; 512 x 512, 64, 200, 1 / 2 / 4 / 8 GB: 45.2 / 41.3 /
-// 40.0 / 39.7; 128^3, 32, 150: 194 / 193 / 173 / 167).  Level kServeLevel for serving lanes, whose memory
+// 40.0 / 39.7; 128^3, 32, 150: 194 / 193 / 173 / 167; 256 MB: 53 and 202).  Level kServeLevel for serving lanes, whose memory
 // admission counts on it; a higher one where the device has no room or the caller's cap
 // leaves none.
 constexpr int64_t kMB = int64_t(1) << 20;
-constexpr int64_t kChunkBytes[kChunkLevels] = {8192 * kMB, 2048 * kMB, 1024 * kMB, 256 * kMB, 64 * kMB, 16 * kMB};
-constexpr int64_t kKeepBytes[kChunkLevels] = {8192 * kMB, 2048 * kMB, 512 * kMB, 128 * kMB, 32 * kMB, 4 * kMB};
+constexpr int64_t kChunkBytes[kChunkLevels] = {8192 * kMB, 2048 * kMB, 1024 * kMB, 256 * kMB, 16 * kMB};
+constexpr int64_t kKeepBytes[kChunkLevels] = {8192 * kMB, 2048 * kMB, 512 * kMB, 128 * kMB, 4 * kMB};
 ChunkShape chunk_shape(int64_t G, int npairs, int S, int level) {
   ChunkShape c;
   const int64_t step = (int64_t)sizeof(double2) * (2 * npairs + 1) * G;

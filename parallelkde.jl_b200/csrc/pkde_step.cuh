@@ -162,9 +162,10 @@ bool chunk_ok(const pkde_grid *g);
 void record_chunked(pkde_ctx *ctx, const pkde_grid *g, int npairs);
 // Scratch at a memory level (0: the largest chunks .. kChunkLevels - 1).  Serving lanes, and contexts
 // that leave the choice of buffer sizes to fixed defaults (pkde_set_autotune), start at kServeLevel;
-// PKDE_RING_BUDGET_MB lowers to kCapLevel at most, whose scratch is always allowed, as ring slots of
-// kNarrowSlotMB are.
-constexpr int kChunkLevels = 6, kServeLevel = 3, kCapLevel = 4;
+// PKDE_RING_BUDGET_MB lowers to kCapLevel at most, whose scratch is always allowed, as the engine's ring of
+// eight slots of kNarrowSlotMB is (512 x 512, 64 bootstraps, 200 steps: 53 ms within 256 MB, 62 within
+// 64 MB, 61 in the engine with those slots).
+constexpr int kChunkLevels = 5, kServeLevel = 3, kCapLevel = 3;
 size_t chunk_scratch_bytes(const pkde_grid *g, int npairs, int S, int level);
 // Whether density and selected step come out final (else the caller initialises the state
 // before and fills the points without a selected step after).

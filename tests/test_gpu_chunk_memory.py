@@ -53,15 +53,17 @@ def _launches(dims, B, S, chunk_mb, keep_mb):
 
 
 @pytest.mark.parametrize("dims,B,steps", [
-    ((257, 241), 67, 4),       # any length: pair groups, all steps kept
-    ((257, 241), 67, 40),      # and f and means of one step at a time
-    ((257, 241), 6, 40),       # several steps a chunk, f and means of one chunk at a time
-    ((257, 241), 6, 20),       # several chunks, all steps kept
-    ((240, 250), 71, 40),      # 2^a 3^b 5^c lengths; the last pair has no second half
-    ((192, 320), 72, 4),       # mixed radices
-    ((256, 256), 67, 40),      # powers of two
-    ((64, 32, 32), 68, 4),     # with a pass in place between
-    ((16, 16, 15, 16), 75, 36),
+    ((257, 241), 271, 4),      # any length: pair groups, all steps kept; the last pair has no second half
+    ((257, 241), 270, 139),    # and f and means of one step at a time
+    ((257, 241), 20, 139),     # several steps a chunk, f and means of one chunk at a time
+    ((257, 241), 20, 29),      # several chunks, all steps kept
+    ((240, 250), 279, 5),      # 2^a 3^b 5^c lengths
+    ((240, 250), 20, 140),
+    ((192, 320), 274, 4),      # mixed radices
+    ((256, 256), 261, 4),      # powers of two
+    ((256, 256), 20, 130),
+    ((64, 32, 32), 260, 4),    # with a pass in place between
+    ((16, 16, 15, 16), 280, 3),
 ])
 def test_small_chunks_keep_results(pk, monkeypatch, dims, B, steps):
     grid, x = _problem(pk, dims)
@@ -70,8 +72,8 @@ def test_small_chunks_keep_results(pk, monkeypatch, dims, B, steps):
         d0, s0, free = ctx.estimate(grid, x, B, steps)
         monkeypatch.setenv("PKDE_RING_BUDGET_MB", "1")
         d1, s1, capped = ctx.estimate(grid, x, B, steps)
-    vmr, means = _launches(dims, B, S, 64, 32)
-    assert vmr > 1 and (free["step_vmr"], free["step_means"]) == (1, 2)
+    vmr, means = _launches(dims, B, S, 256, 128)
+    assert (free["step_vmr"], free["step_means"]) == _launches(dims, B, S, 8192, 8192) and vmr > free["step_vmr"]
     assert (capped["step_vmr"], capped["step_means"]) == (vmr, means)
     assert np.array_equal(s0, s1)
     assert np.array_equal(d0, d1, equal_nan=True)
@@ -80,7 +82,7 @@ def test_small_chunks_keep_results(pk, monkeypatch, dims, B, steps):
 def test_batch_in_small_chunks_keeps_results(pk, monkeypatch):
     from pkde_b200 import raw
     jobs = []
-    for e, (dims, B, steps) in enumerate([((257, 241), 67, 5), ((240, 250), 20, 40), ((64, 64), 5, 10)]):
+    for e, (dims, B, steps) in enumerate([((257, 241), 271, 5), ((240, 250), 20, 140), ((64, 64), 5, 10)]):
         grid, x = _problem(pk, dims)
         G = int(np.prod(dims))
         jobs.append(dict(grid=grid, data=np.ascontiguousarray(x.T), density=np.empty(G),
