@@ -642,23 +642,25 @@ struct ChunkPlan {
   const double *recip;
 };
 
-const double *recip_table(pkde_ctx *ctx) {
+const double *recip_table(pkde_ctx *ctx, cudaStream_t st) {
   DevBuf &b = ctx->chunk_recip;
   if (!b.ptr) {
     std::vector<double> r(kChunkRecip, 0.0);
     for (int i = 1; i < kChunkRecip; ++i) r[i] = 1.0 / (double)i;
     b.ensure(sizeof(double) * kChunkRecip);
-    PKDE_CUDA_TRY(cudaMemcpy(b.ptr, r.data(), sizeof(double) * kChunkRecip, cudaMemcpyHostToDevice));
+    const cudaError_t e = cudaMemcpyAsync(b.ptr, r.data(), sizeof(double) * kChunkRecip, cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) b.release();
+    PKDE_CUDA_TRY(e);
   }
   return b.as<double>();
 }
 
-ChunkPlan plan_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch) {
+ChunkPlan plan_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch, cudaStream_t st) {
   ChunkPlan P{};
   const pkde_grid *g = A.grid;
   const int N = g->ndim, G = (int)grid_size(g);
   P.c = chunk_shape(G, A.npairs, A.S, A.level);
-  P.recip = recip_table(ctx);
+  P.recip = recip_table(ctx, st);
   size_t off[5];
   chunk_scratch(G, A.npairs, A.S, P.c, off);
   P.mid = (double2 *)(scratch + off[0]);
@@ -675,8 +677,8 @@ ChunkPlan plan_chunk(pkde_ctx *ctx, const ChunkArgs &A, char *scratch) {
     a.inner = inner;
     a.lines = G / a.n;
     a.fused = k.pow2;
-    a.twc = k.R > 1 ? combine_twiddles_device(ctx, k.R, a.M) : nullptr;
-    a.nst = make_stages(ctx, a.M, a.st);
+    a.twc = k.R > 1 ? combine_twiddles_device(ctx, k.R, a.M, st) : nullptr;
+    a.nst = make_stages(ctx, a.M, a.st, st);
     a.fixed = chunk_len_known(a.n, a.R);
     for (int i = 0; i < a.nst; ++i)
       if (a.st[i].R > 5 && a.st[i].R != 8) a.plain = a.st[i].tw;
@@ -754,7 +756,7 @@ void run_chunk(pkde_ctx *ctx, const ChunkArgs *args, int count, char *const *scr
   std::vector<ChunkPlan> plan;
   int chunks = 0;
   for (int e = 0; e < count; ++e) {
-    plan.push_back(plan_chunk(ctx, args[e], scratch[e]));
+    plan.push_back(plan_chunk(ctx, args[e], scratch[e], st));
     chunks = std::max(chunks, (args[e].S + plan[e].c.C - 1) / plan[e].c.C);
   }
   // every launch of the call; estimations whose steps are split by pair groups add launches of their own

@@ -9,7 +9,7 @@
 
 namespace pkde {
 
-const double2 *stage_twiddles_device(pkde_ctx *ctx, int logn);
+const double2 *stage_twiddles_device(pkde_ctx *ctx, int logn, cudaStream_t st);
 
 namespace {
 
@@ -315,7 +315,7 @@ void chunk_pow2_axis(pkde_ctx *ctx, const AxisJob &J, bool spectra, cudaStream_t
 #define PKDE_CALL(L)                                                                                         \
   {                                                                                                          \
     const int64_t tpa = J.ax.lines / PT<L>::NL;                                                              \
-    const double2 *tw = stage_twiddles_device(ctx, L);                                                       \
+    const double2 *tw = stage_twiddles_device(ctx, L, st);                                                   \
     Trace tr(ctx, PKDE_PHASE_STEP_FFT, st);                                                                  \
     if (spectra) {                                                                                           \
       const int per = per_cta(ctx, arrays * tpa * J.run.C, J.run.C);                                         \
@@ -341,7 +341,7 @@ void chunk_pow2_rows(pkde_ctx *ctx, const RowsJob &J, cudaStream_t st) {
     const unsigned blocks = (unsigned)(J.ax.lines / (PT<L>::NL / 2)) * J.C;                                       \
     allow_dynamic_smem(ctx, p2_rows_kernel<L>, p2_smem<L>());                                                     \
     Trace tr(ctx, PKDE_PHASE_STEP_VMR, st);                                                                       \
-    p2_rows_kernel<L><<<blocks, kT, p2_smem<L>(), st>>>(J, stage_twiddles_device(ctx, L));                        \
+    p2_rows_kernel<L><<<blocks, kT, p2_smem<L>(), st>>>(J, stage_twiddles_device(ctx, L, st));                    \
   }
   PKDE_P2_SWITCH(J.ax.n, PKDE_CALL)
 #undef PKDE_CALL
@@ -355,7 +355,7 @@ void chunk_pow2_means(pkde_ctx *ctx, const RowsJob &J, cudaStream_t st) {
     const int per = per_cta(ctx, tiles, tiles);                                                                     \
     allow_dynamic_smem(ctx, p2_means_kernel<L>, p2_smem<L>());                                                      \
     Trace tr(ctx, PKDE_PHASE_STEP_MEANS, st);                                                                       \
-    p2_means_kernel<L><<<(unsigned)((tiles + per - 1) / per), kT, p2_smem<L>(), st>>>(J, stage_twiddles_device(ctx, L), \
+    p2_means_kernel<L><<<(unsigned)((tiles + per - 1) / per), kT, p2_smem<L>(), st>>>(J, stage_twiddles_device(ctx, L, st), \
                                                                                      per, (unsigned)tiles);         \
   }
   PKDE_P2_SWITCH(J.ax.n, PKDE_CALL)

@@ -993,7 +993,7 @@ size_t tw_elems(int logn) {
 
 }  // namespace
 
-const double2 *stage_twiddles_device(pkde_ctx *ctx, int logn);
+const double2 *stage_twiddles_device(pkde_ctx *ctx, int logn, cudaStream_t st);
 
 // Engine schedule parameters; the environment overrides the defaults (tuning runs).
 int engine_env_int(const char *name, int dflt, int lo, int hi) {
@@ -1024,7 +1024,7 @@ static size_t mix_tile_elems(int R, int lm) {
 }
 
 // Combine twiddles of N = R * M: (cos, sin)(2 pi n1 k2 / N), n1 = 1..R-1, k2 < M.
-const double2 *combine_twiddles_device(pkde_ctx *ctx, int R, int M) {
+const double2 *combine_twiddles_device(pkde_ctx *ctx, int R, int M, cudaStream_t st) {
   const int N = R * M;
   const int key = -(1000000 + 10 * N + R);
   auto it = ctx->twiddles.find(key);
@@ -1036,10 +1036,7 @@ const double2 *combine_twiddles_device(pkde_ctx *ctx, int R, int M) {
       const long double a = two_pi * (long double)((n1 * k2) % N) / (long double)N;
       tw.push_back(make_double2((double)cosl(a), (double)sinl(a)));
     }
-  DevBuf &b = ctx->twiddles[key];
-  b.ensure(sizeof(double2) * tw.size());
-  PKDE_CUDA_TRY(cudaMemcpy(b.ptr, tw.data(), sizeof(double2) * tw.size(), cudaMemcpyHostToDevice));
-  return b.as<double2>();
+  return upload_table(ctx->twiddles, key, tw, st);
 }
 
 // Tile shape of grid axis j: the register radix-8 FFT where the axis is a power of two
@@ -1171,7 +1168,7 @@ void run_engine_batch(pkde_ctx *ctx, const EngineArgs *args, int count, cudaStre
   if (!ctx->recip_ready) {
     std::vector<double> r(kRecip, 0.0);
     for (int i = 1; i < kRecip; ++i) r[i] = 1.0 / (double)i;
-    PKDE_CUDA_TRY(cudaMemcpyToSymbol(c_recip, r.data(), sizeof(double) * kRecip));
+    PKDE_CUDA_TRY(cudaMemcpyToSymbolAsync(c_recip, r.data(), sizeof(double) * kRecip, 0, cudaMemcpyHostToDevice, st));
     ctx->recip_ready = true;
   }
   std::vector<EngineEst> est(count);
@@ -1185,17 +1182,17 @@ void run_engine_batch(pkde_ctx *ctx, const EngineArgs *args, int count, cudaStre
     E = describe(args[e]);
     for (int j = 0; j < E.ndim; ++j) {
       if (E.gen[j] == 2) {
-        R.tw[E.logn[j]] = stage_twiddles_device(ctx, E.logn[j]);
-        E.twc[j] = combine_twiddles_device(ctx, E.mixr[j], 1 << E.logn[j]);
+        R.tw[E.logn[j]] = stage_twiddles_device(ctx, E.logn[j], st);
+        E.twc[j] = combine_twiddles_device(ctx, E.mixr[j], 1 << E.logn[j], st);
         max_tile = std::max(max_tile, mix_tile_elems(E.mixr[j], E.logn[j]));
         max_tw = std::max(max_tw, tw_elems(E.logn[j]));
       } else if (E.gen[j]) {
-        E.twg[j] = twiddles_device(ctx, (int)E.dims[j]);
+        E.twg[j] = twiddles_device(ctx, (int)E.dims[j], st);
         plans[e][j] = make_plan((int)E.dims[j]);
         E.dlen[j] = make_fastdiv((uint32_t)E.dims[j]);
         max_tile = std::max(max_tile, (size_t)2 * E.tl[j] * (size_t)(E.dims[j] + 1));
       } else {
-        R.tw[E.logn[j]] = stage_twiddles_device(ctx, E.logn[j]);
+        R.tw[E.logn[j]] = stage_twiddles_device(ctx, E.logn[j], st);
         max_tile = std::max(max_tile, tile_elems(E.logn[j]));
         max_reg_tile = std::max(max_reg_tile, tile_elems(E.logn[j]));
         max_tw = std::max(max_tw, tw_elems(E.logn[j]));

@@ -76,14 +76,10 @@ __global__ void __launch_bounds__(kFftThreads) fft_axis_kernel(const double2 *in
 
 }  // namespace
 
-const double2 *twiddles_device(pkde_ctx *ctx, int n) {
+const double2 *twiddles_device(pkde_ctx *ctx, int n, cudaStream_t st) {
   auto it = ctx->twiddles.find(n);
   if (it != ctx->twiddles.end()) return it->second.as<double2>();
-  std::vector<double2> tw = make_twiddles(n);
-  DevBuf &b = ctx->twiddles[n];
-  b.ensure(sizeof(double2) * n);
-  PKDE_CUDA_TRY(cudaMemcpy(b.ptr, tw.data(), sizeof(double2) * n, cudaMemcpyHostToDevice));
-  return b.as<double2>();
+  return upload_table(ctx->twiddles, n, make_twiddles(n), st);
 }
 
 // Lines per CTA: enough to fill ~2048 elements, capped by the shared-memory budget.
@@ -107,7 +103,7 @@ void fft_axis(pkde_ctx *ctx, const LineSet &ls, const double2 *in, double2 *out,
   if (smem > ctx->smem_optin)
     throw Error{PKDE_EUNSUPPORTED, "grid axis too long for the shared-memory FFT"};
   FftPlan plan = make_plan(n);
-  const double2 *tw = twiddles_device(ctx, n);
+  const double2 *tw = twiddles_device(ctx, n, st);
   const int64_t blocks = (nlines + tl - 1) / tl;
   if (blocks > 0x7fffffff) throw Error{PKDE_EUNSUPPORTED, "too many FFT lines"};
   const double *f0 = factors ? factors[0] : nullptr;

@@ -639,7 +639,7 @@ static void run_generic(pkde_ctx *ctx, Plan &P, cudaStream_t st) {
   const size_t smem = sizeof(double2) * 2 * (size_t)tl * pitch;
   if (smem > ctx->smem_optin) throw Error{PKDE_EUNSUPPORTED, "grid axis 1 too long for the shared-memory FFT"};
   FftPlan plan1 = make_plan(n1);
-  const double2 *tw1 = twiddles_device(ctx, n1);
+  const double2 *tw1 = twiddles_device(ctx, n1, st);
   const unsigned fblocks = (unsigned)((rows + tl - 1) / tl);
   const double invG = 1.0 / (double)G;
   const double nsd = (double)E.n;
@@ -978,7 +978,7 @@ void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st)
       A.state = P.state1d;
       line.push_back(A);
     }
-    steps1d_describe(ctx, line.data(), (int)line.size(), hp + (off_rjobs - off_tjobs), lplan);
+    steps1d_describe(ctx, line.data(), (int)line.size(), hp + (off_rjobs - off_tjobs), lplan, st);
     PKDE_CUDA_TRY(cudaMemcpyAsync(base + off_tjobs, hp, desc_bytes, cudaMemcpyHostToDevice, st));
     {
       ::pkde::Trace _tr(ctx, PKDE_PHASE_OTHER, st);

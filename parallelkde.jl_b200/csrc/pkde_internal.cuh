@@ -80,6 +80,20 @@ struct DevBuf {
   }
 };
 
+// A table that the context keeps, uploaded on the stream of the call that first needs it: kernels queued there
+// after it find it complete, on a non-blocking stream too (a copy from pageable memory on the
+// legacy stream may return before its last part has arrived).  Kept under its key only once it is queued.
+template <class Map>
+inline const double2 *upload_table(Map &map, const typename Map::key_type &key, const std::vector<double2> &t,
+                                   cudaStream_t st) {
+  DevBuf b;
+  b.ensure(sizeof(double2) * t.size());
+  const cudaError_t e = cudaMemcpyAsync(b.ptr, t.data(), sizeof(double2) * t.size(), cudaMemcpyHostToDevice, st);
+  if (e != cudaSuccess) b.release();
+  PKDE_CUDA_TRY(e);
+  return (map[key] = b).template as<double2>();
+}
+
 enum BufId {
   BUF_DATA = 0,     // samples (device copy)
   BUF_IDX,          // bootstrap indices (device copy)
@@ -588,7 +602,7 @@ void binning_flags_check(const int *hmisc);
 void fft_nd(pkde_ctx *ctx, int ndim, const int64_t *dims, double2 *data, int64_t batch, int dir,
             cudaStream_t st, int phase);
 // Device twiddle table for size n (cached per context).
-const double2 *twiddles_device(pkde_ctx *ctx, int n);
+const double2 *twiddles_device(pkde_ctx *ctx, int n, cudaStream_t st);
 // Launch one axis pass: out[line] = FFT_dir(in[line] * factor), factor per element k of the
 // axis taken from factors[a % nfac][k] * scal[a % nfac] (factors may be null).
 void fft_axis(pkde_ctx *ctx, const LineSet &ls, const double2 *in, double2 *out, int dir,

@@ -189,6 +189,6 @@ __device__ __forceinline__ void line_stage_generic(const Stage1 &s, int n, int L
 // Host: the stages of an n-point line (radix sequence of make_plan, tables on the device);
 // returns their number.
 bool stages_ok(int n);
-int make_stages(pkde_ctx *ctx, int n, Stage1 *st);
+int make_stages(pkde_ctx *ctx, int n, Stage1 *stages, cudaStream_t st);
 
 }  // namespace pkde

@@ -168,16 +168,13 @@ __global__ void __launch_bounds__(Pow2<LOGN>::THREADS) means_pass_pow2_kernel(
 
 }  // namespace
 
-const double2 *stage_twiddles_device(pkde_ctx *ctx, int logn) {
+const double2 *stage_twiddles_device(pkde_ctx *ctx, int logn, cudaStream_t st) {
   const int key = -logn;  // negative keys: per-stage tables (positive: plain tables)
   auto it = ctx->twiddles.find(key);
   if (it != ctx->twiddles.end()) return it->second.as<double2>();
   std::vector<double2> tw = make_stage_twiddles(logn);
   if (tw.empty()) tw.push_back(make_double2(1.0, 0.0));
-  DevBuf &b = ctx->twiddles[key];
-  b.ensure(sizeof(double2) * tw.size());
-  PKDE_CUDA_TRY(cudaMemcpy(b.ptr, tw.data(), sizeof(double2) * tw.size(), cudaMemcpyHostToDevice));
-  return b.as<double2>();
+  return upload_table(ctx->twiddles, key, tw, st);
 }
 
 namespace {
@@ -188,7 +185,7 @@ void launch_axis(pkde_ctx *ctx, const LineSet &ls, const double2 *in, double2 *o
   using P = Pow2<LOGN>;
   const size_t smem = tile_smem_bytes<LOGN>();
   allow_dynamic_smem(ctx, axis_pass_pow2_kernel<LOGN>, smem);
-  const double2 *tw = stage_twiddles_device(ctx, LOGN);
+  const double2 *tw = stage_twiddles_device(ctx, LOGN, st);
   const int64_t blocks = ls.nlines() / P::NL;
   {
     Trace tr(ctx, PKDE_PHASE_STEP_FFT, st);
@@ -206,7 +203,7 @@ void launch_vmr(pkde_ctx *ctx, const double2 *in, int npairs, int b0, int nboot,
   using P = Pow2<LOGN>;
   const size_t smem = tile_smem_bytes<LOGN>() + sizeof(double2) * 8 * P::THREADS;
   allow_dynamic_smem(ctx, vmr_pass_pow2_kernel<LOGN>, smem);
-  const double2 *tw = stage_twiddles_device(ctx, LOGN);
+  const double2 *tw = stage_twiddles_device(ctx, LOGN, st);
   {
     Trace tr(ctx, PKDE_PHASE_STEP_VMR, st);
     vmr_pass_pow2_kernel<LOGN><<<(unsigned)(rows / P::NL), P::THREADS, smem, st>>>(in, npairs, b0, nboot, tw, fz, fw,
@@ -222,7 +219,7 @@ void launch_means(pkde_ctx *ctx, const double2 *in, int64_t rows, const double *
   using P = Pow2<LOGN>;
   const size_t smem = tile_smem_bytes<LOGN>();
   allow_dynamic_smem(ctx, means_pass_pow2_kernel<LOGN>, smem);
-  const double2 *tw = stage_twiddles_device(ctx, LOGN);
+  const double2 *tw = stage_twiddles_device(ctx, LOGN, st);
   {
     Trace tr(ctx, PKDE_PHASE_STEP_MEANS, st);
     means_pass_pow2_kernel<LOGN><<<(unsigned)(rows / P::NL), P::THREADS, smem, st>>>(

@@ -141,7 +141,7 @@ struct EngineAxis {
 };
 EngineAxis engine_axis(const pkde_grid *g, int j);
 // Combine twiddles of N = R M: (cos, sin)(2 pi n1 k2 / N) as [n1 - 1][k2].
-const double2 *combine_twiddles_device(pkde_ctx *ctx, int R, int M);
+const double2 *combine_twiddles_device(pkde_ctx *ctx, int R, int M, cudaStream_t st);
 
 // Bandwidth steps of N-D estimations in chunks of steps (pkde_chunk.cu).
 struct ChunkArgs {
@@ -198,7 +198,8 @@ struct Steps1dPlan {
   };
   std::vector<Len> len;  // the jobs of the last class by length
 };
-void steps1d_describe(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs, Steps1dPlan &plan);
+void steps1d_describe(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs, Steps1dPlan &plan,
+                      cudaStream_t st);
 void steps1d_run(pkde_ctx *ctx, const Steps1dPlan &plan, const void *dev_jobs, cudaStream_t st);
 // The convergence state machine over all steps (density and selected step of every point).
 struct ConvergeJob {

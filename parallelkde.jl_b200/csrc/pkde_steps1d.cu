@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(kConvThreads) converge_steps_kernel(const __gr
 }  // namespace
 
 // Twiddles of a radix-2/3/4/5/8 stage, [k][r - 1].
-static const double2 *stage1_twiddles(pkde_ctx *ctx, int n, int R, int Ns) {
+static const double2 *stage1_twiddles(pkde_ctx *ctx, int n, int R, int Ns, cudaStream_t st) {
   const std::array<int, 3> k3{n, R, Ns};
   auto it = ctx->stage_tw.find(k3);
   if (it != ctx->stage_tw.end()) return it->second.as<double2>();
@@ -468,21 +468,18 @@ static const double2 *stage1_twiddles(pkde_ctx *ctx, int n, int R, int Ns) {
   const int tstep = n / (Ns * R);
   for (int k = 0; k < Ns; ++k)
     for (int r = 1; r < R; ++r) tw.push_back(w[(size_t)r * k * tstep]);
-  DevBuf &b = ctx->stage_tw[k3];
-  b.ensure(sizeof(double2) * tw.size());
-  PKDE_CUDA_TRY(cudaMemcpy(b.ptr, tw.data(), sizeof(double2) * tw.size(), cudaMemcpyHostToDevice));
-  return b.as<double2>();
+  return upload_table(ctx->stage_tw, k3, tw, st);
 }
 
 bool stages_ok(int n) { return make_plan(n).nstages <= kStages1; }
 
-int make_stages(pkde_ctx *ctx, int n, Stage1 *st) {
+int make_stages(pkde_ctx *ctx, int n, Stage1 *stages, cudaStream_t st) {
   const FftPlan p = make_plan(n);
   int ns = 1;
   for (int q = 0; q < p.nstages; ++q) {
     const int R = p.radix[q];
-    st[q] = Stage1{R, n / R, ns, n / (ns * R), p.div_ns[q],
-                   R <= 5 || R == 8 ? stage1_twiddles(ctx, n, R, ns) : twiddles_device(ctx, n)};
+    stages[q] = Stage1{R, n / R, ns, n / (ns * R), p.div_ns[q],
+                       R <= 5 || R == 8 ? stage1_twiddles(ctx, n, R, ns, st) : twiddles_device(ctx, n, st)};
     ns *= R;
   }
   return p.nstages;
@@ -492,11 +489,12 @@ bool steps1d_ok(const pkde_grid *g) {
   return g->ndim == 1 && g->dims[0] <= 4096 && stages_ok((int)g->dims[0]);
 }
 
-const double2 *stage_twiddles_device(pkde_ctx *ctx, int logn);
+const double2 *stage_twiddles_device(pkde_ctx *ctx, int logn, cudaStream_t st);
 
 size_t steps1d_job_bytes() { return sizeof(Job1); }
 
-void steps1d_describe(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs, Steps1dPlan &plan) {
+void steps1d_describe(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *host_jobs, Steps1dPlan &plan,
+                      cudaStream_t st) {
   plan = Steps1dPlan{};
   Job1 *hj = reinterpret_cast<Job1 *>(host_jobs);
   // classes: the general kernel's three forms, the power-of-two lengths 1024, 2048 and 4096, the
@@ -549,7 +547,7 @@ void steps1d_describe(pkde_ctx *ctx, const Steps1dArgs *args, int count, void *h
       J.inv_ns = 1.0 / (double)A.n;
       J.f_out = A.f_out;
       J.mu_out = A.mu_out;
-      J.nst = make_stages(ctx, A.n1, J.st);
+      J.nst = make_stages(ctx, A.n1, J.st, st);
       if (c == NC - 1) {
         if (plan.len.empty() || plan.len.back().n != A.n1) plan.len.push_back({A.n1, k, 0, 0});
         auto &g = plan.len.back();
@@ -582,12 +580,12 @@ void steps1d_run(pkde_ctx *ctx, const Steps1dPlan &plan, const void *dev_jobs, c
   launch(2, 1024, smem[2], steps1d_kernel<1024, true>);
 #define PKDE_P2(C, L)                                                                                          \
   launch(C, Pow2<L, 2>::THREADS, sizeof(double2) * (Pow2<L, 2>::TILE + Pow2<L, 2>::N + Pow2<L, 2>::TWSIZE),     \
-         steps1d_pow2_kernel<L>, stage_twiddles_device(ctx, L));
+         steps1d_pow2_kernel<L>, stage_twiddles_device(ctx, L, st));
   PKDE_P2(3, 10)
   PKDE_P2(4, 11)
 #undef PKDE_P2
   launch(5, Pow2<12, 1>::THREADS, sizeof(double2) * (Pow2<12, 1>::TILE + Pow2<12, 1>::TWSIZE), steps1d_line_kernel<12>,
-         stage_twiddles_device(ctx, 12));
+         stage_twiddles_device(ctx, 12, st));
   for (const auto &g : plan.len) {
     {
       Trace tr(ctx, PKDE_PHASE_STEP_VMR, st);
