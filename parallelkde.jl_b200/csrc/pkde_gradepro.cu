@@ -1153,7 +1153,10 @@ void validate_gradepro_params(const pkde_gradepro_params *p, int64_t n) {
 // (FourierSpace.jl:242-262 split per axis), inverse FFT scaled by 1/G (:203-230), |.|
 // (copy_density!, :233-265).
 namespace {
-__global__ void abs_kernel(int64_t G, const double2 *__restrict__ z, double *__restrict__ out) {
+// Invalid data (errors set by the binning) leaves the caller's density as it was.
+__global__ void abs_kernel(int64_t G, const double2 *__restrict__ z, const int *__restrict__ errors,
+                           double *__restrict__ out) {
+  if (*errors) return;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < G; i += (int64_t)gridDim.x * blockDim.x) {
     const double2 v = z[i];
     out[i] = sqrt(v.x * v.x + v.y * v.y);
@@ -1217,7 +1220,7 @@ void run_rot(pkde_ctx *ctx, const pkde_grid *g, int rule, const double *d_data, 
   }
   {
     ::pkde::Trace _tr(ctx, PKDE_PHASE_STEP_MEANS, st);
-    abs_kernel<<<blocks_for(ctx, G), kThreads, 0, st>>>(G, spec, d_density);
+    abs_kernel<<<blocks_for(ctx, G), kThreads, 0, st>>>(G, spec, j.misc, d_density);
   }
   PKDE_CHECK_LAUNCH();
 }
@@ -1336,10 +1339,13 @@ int pkde_rot_estimate(pkde_ctx *ctx, const pkde_grid *grid, int32_t rule, const 
     }
     double *dens = dout ? density_out : (double *)ensure(ctx, BUF_OUT, sizeof(double) * G);
     run_rot(ctx, grid, rule, d_data, n, dens, st);
-    if (!dout) copy_out(density_out, dens, sizeof(double) * G, false, st);
     PKDE_CUDA_TRY(cudaStreamSynchronize(st));
     collect_trace(ctx);
     check_binning_flags(ctx);
+    if (!dout) {
+      copy_out(density_out, dens, sizeof(double) * G, false, st);
+      PKDE_CUDA_TRY(cudaStreamSynchronize(st));
+    }
   });
 }
 
