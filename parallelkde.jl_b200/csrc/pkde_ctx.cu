@@ -5,7 +5,7 @@
 #include <map>
 #include <memory>
 
-#include "pkde_internal.cuh"
+#include "pkde_steps1d.cuh"
 
 namespace pkde {
 
@@ -47,6 +47,13 @@ void copy_out(void *dst, const void *src, size_t bytes, bool dst_on_device, cuda
 __global__ void divide_kernel(const double *num, const double *den, double *out, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     out[i] = div_nr(num[i], den[i]);
+}
+
+__global__ void vmr_update_kernel(const double2 *z, const double2 *w, double2 *state, int64_t n, double ns, double i0,
+                                  bool has_b) {
+  const double inv_ns = 1.0 / ns, inv_a = 1.0 / i0, inv_b = 1.0 / (i0 + 1.0);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    vmr_update2<false>(z[i], w[i], ns, inv_ns, i0, inv_a, inv_b, has_b, state[i]);
 }
 
 }  // namespace pkde
@@ -138,6 +145,33 @@ int pkde_diag_divide(pkde_ctx *ctx, const double *num, const double *den, double
     divide_kernel<<<blocks, 256, 0, st>>>(dn, dd, dq, n);
     PKDE_CHECK_LAUNCH();
     if (!dev) copy_out(out, dq, bytes, false, st);
+    PKDE_CUDA_TRY(cudaStreamSynchronize(st));
+  });
+}
+
+int pkde_diag_vmr_update(pkde_ctx *ctx, const double *means, const double *squares, double *state, int64_t n,
+                         double n_samples, double first, int32_t both, void *stream) {
+  return pkde_guard(ctx, [&] {
+    using namespace pkde;
+    if (!ctx) throw invalid("context is NULL");
+    if (n < 0 || (n > 0 && (!means || !squares || !state))) throw invalid("means, squares and state are required");
+    if (!(n_samples >= 1.0 && n_samples < 2147483648.0 && first >= 1.0 && first < 2147483647.0) ||
+        n_samples != std::floor(n_samples) || first != std::floor(first))
+      throw invalid("n_samples and first must be whole numbers in 1..2^31 - 2");
+    PKDE_CUDA_TRY(cudaSetDevice(ctx->device));
+    settle_pending(ctx);
+    cudaStream_t st = (cudaStream_t)stream;
+    DrainOnError drain{ctx, st};
+    if (n == 0) return;
+    const size_t bytes = sizeof(double2) * (size_t)n;
+    double2 *b = (double2 *)ensure(ctx, BUF_MISC, 3 * bytes);
+    copy_in(b, means, bytes, false, st);
+    copy_in(b + n, squares, bytes, false, st);
+    copy_in(b + 2 * n, state, bytes, false, st);
+    const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)ctx->sm_count * 8);
+    vmr_update_kernel<<<blocks, 256, 0, st>>>(b, b + n, b + 2 * n, n, n_samples, first, both != 0);
+    PKDE_CHECK_LAUNCH();
+    copy_out(state, b + 2 * n, bytes, false, st);
     PKDE_CUDA_TRY(cudaStreamSynchronize(st));
   });
 }
