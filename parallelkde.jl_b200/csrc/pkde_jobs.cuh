@@ -30,11 +30,7 @@ __device__ __forceinline__ void find_job(const J *jobs, const unsigned *block0, 
   __syncthreads();
 }
 
-// Body::run(job, block) in T threads: one job as the kernel's parameter, or several.
-template <class Body, class J, int T>
-__global__ void __launch_bounds__(T) one_job_kernel(const __grid_constant__ J job) {
-  Body::run(job, blockIdx.x);
-}
+// Body::run(job, block) in T threads for each job.
 template <class Body, class J, int T>
 __global__ void __launch_bounds__(T) many_jobs_kernel(const J *jobs, const unsigned *block0, int count) {
   __shared__ J job;

@@ -32,7 +32,8 @@ struct Len {
   }
 };
 
-// One stage.  ld(l, j, v): inputs; st(l, pos, v) as line_stage.
+// One stage.  ld(l, j, v): the inputs of butterfly j of line l; st(l, pos, v): element pos + q Ns of line l
+// is v[q].
 template <int T, int M, int Q, int Ns, int Lr, class Ld, class St>
 __device__ __forceinline__ void len_stage(const double2 *tw, Ld ld, St st) {
   constexpr int nb = M / Q, items = nb * Lr, IT = (items + T - 1) / T;

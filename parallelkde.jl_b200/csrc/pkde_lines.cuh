@@ -104,36 +104,6 @@ __device__ __forceinline__ void dft_r(double2 *v) {
   }
 }
 
-// One stage of radix R over L lines in T threads.  ld(j, l, v): the R inputs of butterfly j
-// of line l (elements j + r nb); returns true when it has applied the butterfly itself (a
-// first stage that scales its inputs).  st(l, pos, v): element pos + q Ns of line l is v[q].
-template <int T, int R, class Ld, class St>
-__device__ __forceinline__ void line_stage(const Stage1 &s, int L, FastDiv dL, bool first, Ld ld, St st) {
-  const int items = s.nb * L, Ns = s.Ns;
-  const double2 *tw = s.tw;
-  const FastDiv dns = s.dns;
-  for (int e = threadIdx.x; e < items; e += T) {
-    const int j = (int)fdiv((uint32_t)e, dL), l = e - j * L;
-    double2 v[R];
-    if (!ld(j, l, v)) {
-      int jq = j;
-      if (!first) {
-        jq = (int)fdiv((uint32_t)j, dns);
-        const int k = j - jq * Ns;
-        if (k > 0) {
-          const double2 *w = tw + k * (R - 1) - 1;
-#pragma unroll
-          for (int r = 1; r < R; ++r) v[r] = cmul1(v[r], __ldg(w + r));
-        }
-      }
-      dft_r<R>(v);
-      st(l, j + jq * Ns * (R - 1), v);
-    } else {
-      st(l, j * R, v);
-    }
-  }
-}
-
 // Any other radix: an item is four outputs of one butterfly of two lines, l and l + H (2 H lines
 // of which L exist).  tw(o): the factor at byte o of the plain table; ld(p): the element at p,
 // input r of butterfly j of line l at p = (j + r nb) PB + 16 l; st(l, pos, v): output pos of line l.
