@@ -54,8 +54,8 @@ struct Server {
 };
 
 // Upper bound of the device memory one request needs inside a wave: samples, indices,
-// outputs, paired spectra, convergence state, factor tables, binning scratch, 1-D
-// per-step arrays and the chunk scratch or the step engine's ring slots and counters.
+// outputs, convergence state, factor tables, binning and spectra, 1-D per-step arrays and the
+// chunk scratch or the step engine's ring slots and counters.
 size_t footprint(const pkde_gradepro_params *p, int64_t n, bool has_idx) {
   const int N = p->grid.ndim;
   int64_t G = 1, axes = 0;
@@ -65,15 +65,11 @@ size_t footprint(const pkde_gradepro_params *p, int64_t n, bool has_idx) {
   }
   const int64_t B = p->n_bootstraps, P = (B + 1) / 2;
   const int64_t S = p->n_steps > 0 ? (int64_t)p->n_steps + 1 : 1001;  // bw_step ladders: a generous bound
-  const int64_t nc = int64_t(1) << N;
   size_t b = 0;
   b += sizeof(double) * N * n + (has_idx ? sizeof(int32_t) * n * B : 0) + 12 * (size_t)G;  // in/out
-  b += sizeof(double2) * (2 * P + 1) * G;                                                 // spectra
   b += 64 * (size_t)G;                                                                    // state
   b += sizeof(double) * 2 * S * axes;                                                     // tables
-  b += 4 * n + 8 * N * n + 32 * nc * n + 4 * (B + 1) * G;                                 // binning
-  b += sizeof(double2) * (2 * P + 1) * G;  // low parts of the fixed-point sums
-  b += 4 * B * n + 8 * n + 8 * (size_t)G;  // draws per sample, cell order, cell starts
+  b += dirac_zero_bytes(&p->grid, n, B) + dirac_job_scratch(&p->grid, n);                 // binning, spectra
   if (N == 1) b += sizeof(double) * 4 * S * G;                                            // 1-D steps
   const size_t slot = std::max<size_t>(32u << 20, sizeof(double2) * 2 * (size_t)G);
   const size_t engine = 8 * slot + 32 * (size_t)G + sizeof(int) * (size_t)S * (P + 1) * (N + G / 16 + 1);
