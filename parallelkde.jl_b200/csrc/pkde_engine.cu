@@ -1,5 +1,6 @@
 // Persistent dataflow engine for the per-bandwidth-step work of N-D (N >= 2) estimations: axes of
-// more than 1024 points, and shapes or contexts that ask for it (pkde_chunk.cu runs the others).
+// more than 1024 points, grids of more than 2^26, and contexts with a wait limit of their own
+// (pkde_chunk.cu runs the others).
 //
 // Work: for every step s the inverse FFT of all bootstrap pairs (z, w arrays) and of the
 // full-sample means, then VMR + Welford over bootstraps, then the convergence update.

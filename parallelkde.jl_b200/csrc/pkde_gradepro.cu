@@ -483,7 +483,6 @@ static void factor_tables(const pkde_grid *g, const Ladder &L, std::vector<doubl
   }
 }
 
-// The same tables written straight into fz/fw (S x tot each), steps [s0, s1).
 // Propagation factor tables of one estimation, computed on the device: for step s and
 // grid axis j, fz = exp(-(k t)^2 / 2) and fw = sqrt(fz) over the axis's frequencies k =
 // 2 pi fftfreq(n, h) (FourierSpace.jl:228-234 per axis; the full propagator is their
@@ -732,9 +731,9 @@ static void run_generic(pkde_ctx *ctx, Plan &P, cudaStream_t st) {
 
 
 // The :gradepro estimation of `count` independent sample sets on one stream: each phase
-// runs for every estimation before the next phase starts, so the whole call has one
-// host synchronisation per phase (Silverman moments, binning read-back), and the
-// bandwidth steps of all N-D power-of-two estimations run in one persistent launch.
+// runs for every estimation before the next phase starts, so the whole call has two
+// host synchronisations (Silverman's moments, the end); the steps of 1-D estimations share a launch per kernel,
+// those of N-D ones the launches of their chunks (pkde_chunk.cu) or one persistent launch of the engine.
 // An estimation gets the same result alone and in a batch: every kernel partitions its
 // work by the estimation's own sizes only.
 void run_many(pkde_ctx *ctx, const Estimation *ests, int count, cudaStream_t st) {
