@@ -302,11 +302,12 @@ int pkde_diag_divide(pkde_ctx *ctx, const double *num, const double *den, double
 
 /* Diagnostic: the variance-to-mean ratios of two bootstraps (numbers first and first + 1; without
  * `both` the first one only) at n points and their update of the running (mean, sum of squares),
- * with the arithmetic of the 1-D steps, whose quotients come from products where that rounds as IEEE
- * division does.  Host arrays of n pairs: means and squares (DirectSpace.jl:550-552), state
+ * with the arithmetic of the 1-D steps: every operation rounded by itself, the quotients from products
+ * where that rounds as IEEE division does; with `fused` that of power-of-two lengths from 256 (1 / n as a
+ * product, sums and products fused, pkde_diag_divide's quotient).  Host arrays of n pairs: means and squares (DirectSpace.jl:550-552), state
  * (:572-577, updated in place).  n_samples and first: whole numbers in 1..2^31 - 2. */
 int pkde_diag_vmr_update(pkde_ctx *ctx, const double *means, const double *squares, double *state, int64_t n,
-                         double n_samples, double first, int32_t both, void *stream);
+                         double n_samples, double first, int32_t both, int32_t fused, void *stream);
 
 /* Launch accounting and per-phase device time, for tracing and the roofline report.
  * No counterpart in the reference, which has no tracing.

@@ -62,10 +62,11 @@ __device__ __forceinline__ double recip_of(const double *table, int i) {
 }
 
 // VMR of the two bootstraps of a pair at one point (DirectSpace.jl:550-552), 1 / n as a product; mean: of
-// the bootstraps before.
+// the bootstraps before.  |V| / n is the fused product, as in the engine's tiles: where all resamples are alike, the
+// variance over them is the rounding of the ratio itself.
 __device__ __forceinline__ void chunk_vmr2(double2 z, double2 w, double inv_n, double mean, double &xa, double &xb) {
   const double ma = __dmul_rn(fabs(z.x), inv_n), mb = __dmul_rn(fabs(z.y), inv_n);
-  div_nr2(__fma_rn(-ma, ma, __dmul_rn(fabs(w.x), inv_n)), ma, __fma_rn(-mb, mb, __dmul_rn(fabs(w.y), inv_n)), mb, mean,
+  div_nr2(__fma_rn(fabs(w.x), inv_n, -__dmul_rn(ma, ma)), ma, __fma_rn(fabs(w.y), inv_n, -__dmul_rn(mb, mb)), mb, mean,
           xa, xb);
 }
 

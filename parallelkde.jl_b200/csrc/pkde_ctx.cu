@@ -49,11 +49,12 @@ __global__ void divide_kernel(const double *num, const double *den, double *out,
     out[i] = div_nr(num[i], den[i]);
 }
 
+template <bool FUSED>
 __global__ void vmr_update_kernel(const double2 *z, const double2 *w, double2 *state, int64_t n, double ns, double i0,
                                   bool has_b) {
   const double inv_ns = 1.0 / ns, inv_a = 1.0 / i0, inv_b = 1.0 / (i0 + 1.0);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    vmr_update2<false>(z[i], w[i], ns, inv_ns, i0, inv_a, inv_b, has_b, state[i]);
+    vmr_update2<FUSED>(z[i], w[i], ns, inv_ns, i0, inv_a, inv_b, has_b, state[i]);
 }
 
 }  // namespace pkde
@@ -150,7 +151,7 @@ int pkde_diag_divide(pkde_ctx *ctx, const double *num, const double *den, double
 }
 
 int pkde_diag_vmr_update(pkde_ctx *ctx, const double *means, const double *squares, double *state, int64_t n,
-                         double n_samples, double first, int32_t both, void *stream) {
+                         double n_samples, double first, int32_t both, int32_t fused, void *stream) {
   return pkde_guard(ctx, [&] {
     using namespace pkde;
     if (!ctx) throw invalid("context is NULL");
@@ -169,7 +170,8 @@ int pkde_diag_vmr_update(pkde_ctx *ctx, const double *means, const double *squar
     copy_in(b + n, squares, bytes, false, st);
     copy_in(b + 2 * n, state, bytes, false, st);
     const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)ctx->sm_count * 8);
-    vmr_update_kernel<<<blocks, 256, 0, st>>>(b, b + n, b + 2 * n, n, n_samples, first, both != 0);
+    auto kern = fused ? vmr_update_kernel<true> : vmr_update_kernel<false>;
+    kern<<<blocks, 256, 0, st>>>(b, b + n, b + 2 * n, n, n_samples, first, both != 0);
     PKDE_CHECK_LAUNCH();
     copy_out(state, b + 2 * n, bytes, false, st);
     PKDE_CUDA_TRY(cudaStreamSynchronize(st));

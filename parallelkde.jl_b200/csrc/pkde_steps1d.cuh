@@ -72,7 +72,7 @@ __device__ __forceinline__ void vmr_update2(double2 z, double2 w, double ns, dou
   if constexpr (FUSED) {
     const double ma = __dmul_rn(fabs(z.x), inv_ns), mb = __dmul_rn(fabs(z.y), inv_ns);
     double xa, xb;
-    div_nr2(__fma_rn(-ma, ma, __dmul_rn(fabs(w.x), inv_ns)), ma, __fma_rn(-mb, mb, __dmul_rn(fabs(w.y), inv_ns)), mb,
+    div_nr2(__fma_rn(fabs(w.x), inv_ns, -__dmul_rn(ma, ma)), ma, __fma_rn(fabs(w.y), inv_ns, -__dmul_rn(mb, mb)), mb,
             st.x, xa, xb);
     auto add = [&st](double x, double inv) {
       const double delta = __dsub_rn(x, st.x);

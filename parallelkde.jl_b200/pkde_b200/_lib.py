@@ -98,7 +98,7 @@ def load():
     lib.pkde_set_wait_limit.argtypes = [vp, i64]
     lib.pkde_set_fault.argtypes = [vp, i32]
     lib.pkde_diag_divide.argtypes = [vp, vp, vp, vp, i64, u32, vp]
-    lib.pkde_diag_vmr_update.argtypes = [vp, vp, vp, vp, i64, dbl, dbl, i32, vp]
+    lib.pkde_diag_vmr_update.argtypes = [vp, vp, vp, vp, i64, dbl, dbl, i32, i32, vp]
     lib.pkde_boot_index.argtypes = [u64, i64, i64, i64]
     lib.pkde_boot_index.restype = i64
     for name in EXPORTED:
@@ -219,16 +219,16 @@ def diag_divide(num, den, device=0):
     return out
 
 
-def diag_vmr_update(means, squares, state, n_samples, first, both=True, device=0):
+def diag_vmr_update(means, squares, state, n_samples, first, both=True, fused=False, device=0):
     """The running (mean, sum of squares), an (n, 2) array, after two bootstraps' variance-to-mean ratios
-    with the arithmetic of the 1-D steps; means, squares: (n, 2) float64."""
+    with the arithmetic of the 1-D steps (fused: of power-of-two lengths from 256); means, squares: (n, 2) float64."""
     m, v = (np.ascontiguousarray(a, dtype=np.float64) for a in (means, squares))
     out = np.array(state, dtype=np.float64, order="C")
     if not m.shape == v.shape == out.shape or m.ndim != 2 or m.shape[1] != 2:
         raise ValueError("means, squares and state must be (n, 2)")
     ctx = context(device)
     check(load().pkde_diag_vmr_update(ctx, ptr(m), ptr(v), ptr(out), m.shape[0], float(n_samples), float(first),
-                                      int(bool(both)), None), ctx)
+                                      int(bool(both)), int(bool(fused)), None), ctx)
     return out
 
 

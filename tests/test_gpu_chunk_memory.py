@@ -24,10 +24,10 @@ class Context:
     def __exit__(self, *exc):
         self.lib.pkde_destroy(self.handle)
 
-    def estimate(self, grid, x, B, steps, seed=3):
+    def estimate(self, grid, x, B, steps, seed=3, **kw):
         """(density, selected, launches per phase)"""
         from pkde_b200 import _lib
-        p = _lib.make_params(_lib.make_grid_struct(grid.lo, grid.hi, grid.h, grid.dims), B, steps)
+        p = _lib.make_params(_lib.make_grid_struct(grid.lo, grid.hi, grid.h, grid.dims), B, steps, **kw)
         data, G = np.ascontiguousarray(x.T), int(np.prod(grid.dims))
         d, s, st = np.empty(G), np.empty(G, dtype=np.int32), _lib.PkdeStats()
         self.lib.pkde_get_stats(self.handle, ctypes.byref(st), 1)

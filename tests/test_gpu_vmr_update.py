@@ -89,3 +89,27 @@ def test_quotients_next_to_midpoints(pk, near):
     state[:, 0] = 0.125
     _check(B * 2.0 ** -700, A * 2.0 ** -700, state, 1, 1)
     _check(B * 2.0 ** -650, A * 2.0 ** -600, state, 1, 5)
+
+
+def test_fused_operations(pk):
+    """Power-of-two lengths: |V| / n fused into the difference, 1 / i as a factor, both updates fused."""
+    import ctypes
+    import ctypes.util
+    from pkde_b200 import _lib
+    libm = ctypes.CDLL(ctypes.util.find_library("m"))
+    libm.fma.restype, libm.fma.argtypes = ctypes.c_double, [ctypes.c_double] * 3
+    fma = np.vectorize(libm.fma, otypes=[float])
+    rng = np.random.default_rng(8)
+    n, ns, first = 20000, 1000, 3
+    means, squares = rng.lognormal(0.0, 2.0, (n, 2)), rng.lognormal(0.0, 2.0, (n, 2)) + 1.0
+    state = np.stack([rng.standard_normal(n), rng.lognormal(size=n)], axis=1)
+    got = _lib.diag_vmr_update(means, squares, state, ns, first, fused=True)
+    mean, m2 = state.T.copy()
+    for k in range(2):
+        inv_n, inv_i = 1.0 / ns, 1.0 / (first + k)
+        m = means[:, k] * inv_n
+        x = _lib.diag_divide(fma(squares[:, k], inv_n, -(m * m)), m)
+        delta = x - mean
+        mean = fma(delta, inv_i, mean)
+        m2 = fma(delta, x - mean, m2)
+    assert np.array_equal(got, np.stack([mean, m2], axis=1))
